@@ -44,6 +44,11 @@ namespace {
 constexpr int kDenseMax = 2048;  // DOFs of the coarsest (dense) level at most
 constexpr int kMaxLevels = 8;
 constexpr int kNormCtas = 512;  // CTAs of the power-iteration norm
+constexpr int kSweepTile = 32;  // pivots of a step of the dense level's inversion, rows and columns of its tiles
+
+// row lengths of the dense level's FP64 work matrix (whole tiles) and of its inverse
+inline int64_t dense_ld(int64_t nc) { return (nc + kSweepTile - 1) / kSweepTile * kSweepTile; }
+inline int64_t inverse_ld(int64_t nc) { return (nc + 3) / 4 * 4; }
 
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -301,10 +306,10 @@ struct AmrAmg {
     int NM = 6;
     std::vector<AmgLevel> L;
     int64_t nc = 0;             // DOFs of the dense coarsest level
-    double *Cd = nullptr;       // nc x 2nc FP64 work (Gauss-Jordan)
-    cudaGraphExec_t gj_exec = nullptr;  // the Gauss-Jordan steps, captured once
-    float *Cinv = nullptr;      // nc x nc inverse, FP32 cycle
-    double *Cinv64 = nullptr;   // nc x nc inverse, FP64 cycle
+    double *Cd = nullptr;       // FP64 work of the inversion: the padded matrix, then the panels of a sweep step
+    cudaGraphExec_t gj_exec = nullptr;  // the sweep steps, captured once
+    float *Cinv = nullptr;      // nc rows of the inverse, FP32 cycle
+    double *Cinv64 = nullptr;   // nc rows of the inverse, FP64 cycle
     double *scratch = nullptr;  // norms: [0] result, [1] the power iteration's estimate, [8..] per-CTA partials
     unsigned int *ticket = nullptr;
     int32_t *pstop = nullptr;   // the power iteration met a zero or non-finite norm: its remaining steps return
@@ -589,8 +594,11 @@ static void amg_build_structure(amr_model *m) {
         H.push_back(std::move(hc));
     }
     if (g->nc > 32768) throw AmrError(AMR_EUNSUPPORTED, "the multigrid's coarsest level is too large to invert densely");
-    amr_alloc(&g->Cd, (size_t)g->nc * 2 * g->nc);  // [A | I] for Gauss-Jordan
-    amr_alloc(&g->Cinv, (size_t)g->nc * g->nc);
+    {  // the padded matrix, two panels of a sweep step and two diagonal tiles
+        const size_t ld = (size_t)dense_ld(g->nc);
+        amr_alloc(&g->Cd, ld * ld + 2 * ld * kSweepTile + 2 * kSweepTile * kSweepTile);
+    }
+    amr_alloc(&g->Cinv, (size_t)g->nc * inverse_ld(g->nc));
     amr_alloc(&g->scratch, 8 + kNormCtas);
     amr_alloc(&g->ticket, 1);
     amr_alloc(&g->pstop, 1);
@@ -1352,60 +1360,277 @@ __global__ void k_prolong_sa16(int64_t n, const int64_t *prp, const int32_t *pcj
     }
 }
 
-// dense coarsest level: expand the BSR matrix, invert it (Gauss-Jordan, FP64), multiply
+// ---------------------------------------------------------------------------
+// Dense coarsest level: the BSR matrix expanded to FP64, inverted by a blocked symmetric sweep, multiplied.
+//
+// The inverse of an SPD matrix of nc rows takes nc^3 / 2 FP64 FMAs when only one triangle is formed, and on this GPU
+// the FP64 pipe (two FMAs a clock per SM) is what bounds it: 61 us of every step's 68 us at nc = 1 428, 3.4 ms in
+// all.  An elimination with one launch per pivot moved the whole augmented matrix through L2 for every pivot:
+// 33.5 ms there (23.5 us a pivot), 3.8 ms at nc = 558 (now 0.9 ms).  Here 32 pivots are taken at a time:
+//   D = A_kk^-1 (in shared memory), W_i = A_ik D (k_sweep_panel), A_ij -= W_i A_kj for the other tiles of the
+//   lower triangle (k_sweep_update), A_ik = W_i, A_kk = -D;
+// after the last block the triangle holds -A^-1.  A 32 x 32 tile per CTA gives n = 1 332 some 900 tiles a step, six
+// even waves, and every tile is read and written once per 32 pivots.  The CTA that updates the next diagonal tile
+// inverts it in the same launch, beside the other tiles, so a step costs two launches.
+//
+// A product with a zero factor is left out, and a tile pair without a nonzero is skipped: the level is block diagonal
+// over the parts of a batch, so a part's non-finite values stay in its own rows and columns, and the zero tiles
+// cost a read.
+// ---------------------------------------------------------------------------
+constexpr int kSw = kSweepTile;
+
+__device__ __forceinline__ bool nz(double x) { return (__double_as_longlong(x) << 1) != 0; }
+__device__ __forceinline__ bool finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+// CTA per coarse node row: the lower triangle of the expanded matrix (C is zero before), ld columns
 template <int NM, class V>
 __global__ void k_dense_expand(int64_t n, const int64_t *rp, const int32_t *cj, const V *A, int64_t nbs, double *C,
-                               int64_t nc) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int64_t k = rp[i]; k < rp[i + 1]; k++)
-        for (int c = 0; c < NM; c++)
-            for (int d = 0; d < NM; d++)
-                C[(i * NM + c) * 2 * nc + (int64_t)cj[k] * NM + d] = A[(int64_t)(c * NM + d) * nbs + k];
+                               int64_t ld) {
+    const int64_t i = blockIdx.x;
+    const int64_t k0 = rp[i];
+    const int total = (int)(rp[i + 1] - k0) * NM * NM;
+    for (int t = threadIdx.x; t < total; t += blockDim.x) {
+        const int64_t k = k0 + t / (NM * NM);
+        const int q = t % (NM * NM);
+        const int64_t r = i * NM + q / NM, c = (int64_t)cj[k] * NM + q % NM;
+        if (c <= r) C[r * ld + c] = A[(int64_t)q * nbs + k];
+    }
 }
-__global__ void k_dense_init(int64_t nc, double *C) {  // C is nc x 2nc: [A | I]
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nc * 2 * nc) return;
-    const int64_t r = t / (2 * nc), c = t % (2 * nc);
-    C[t] = (c >= nc && c - nc == r) ? 1.0 : 0.0;
+// unit diagonal of the rows that pad the matrix to whole tiles
+__global__ void k_dense_pad(int64_t nc, int64_t ld, double *C) {
+    const int64_t r = nc + threadIdx.x;
+    if (r < ld) C[r * ld + r] = 1.0;
 }
-// One Gauss-Jordan step on pivot p of an SPD matrix (no pivoting needed), one launch: a grid row per matrix
-// row r != p, with the factor f_r = C[r][p] / C[p][p] (rows with f_r = 0, every row outside the pivot's block
-// when the level is block diagonal as for the parts of a batch, are left as they are), then
-// C[r][c] -= f_r C[p][c] for the columns c > p.  Columns c <= p of the left half are not updated: the pivot
-// row is zero there once eliminated, and of them only the diagonal, which no later step changes, is read
-// afterwards.  Nothing a step writes (rows r != p, columns > p) is read by another CTA of the same step.
-__global__ void k_gj_step(int64_t nc, int64_t p, double *C) {
-    const int64_t r = blockIdx.y;
-    if (r == p) return;
-    const int64_t w = 2 * nc;
-    __shared__ double sf;  // the FP64 division once per CTA, not per thread: the FP64 pipe is narrow
-    if (threadIdx.x == 0) sf = C[r * w + p] / C[p * w + p];
+
+// 1 / d from the FP32 reciprocal and two Newton steps (24, 48, 53 bits): a shorter chain on the FP64 pipe than the
+// division, which is taken outside the float range
+__device__ __forceinline__ double reciprocal(double d) {
+    const float f = (float)d;
+    const float a = fabsf(f);
+    if (!(a > 1e-30f && a < 1e30f)) return 1.0 / d;
+    double x = (double)__frcp_rn(f);
+    x = fma(x, fma(-d, x, 1.0), x);
+    return fma(x, fma(-d, x, 1.0), x);
+}
+
+struct SweepTile {
+    double S[2][kSw][kSw + 1];  // the tile before and after a pivot, by turns
+    double col[2][kSw], fac[2][kSw], inv[2];
+};
+
+// T.S[0] (lower triangle) swept over its kSw pivots: -S^-1, in T.S[0]; 256 threads.  One barrier a pivot: while the
+// other warps update the triangle, warp 0 forms the next pivot's column, its reciprocal and its factors.
+__device__ void sweep_tile(SweepTile &T) {
+    const int lane = threadIdx.x & 31;
+    const bool lead = threadIdx.x < 32;
+    int r[3], c[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const int e = (int)threadIdx.x - 32 + 224 * q;
+        int rr = 0;
+        if (e >= 0 && e < kSw * (kSw + 1) / 2) {
+            rr = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
+            if ((rr + 1) * (rr + 2) / 2 <= e) rr++;
+            if (rr * (rr + 1) / 2 > e) rr--;
+            r[q] = rr;
+            c[q] = e - rr * (rr + 1) / 2;
+        } else {
+            r[q] = c[q] = -1;
+        }
+    }
+    auto column = [&](int to, int q, double v) {  // lane's entry v of pivot q's column
+        const double iv = reciprocal(__shfl_sync(0xffffffffu, v, q));
+        T.col[to][lane] = v;
+        T.fac[to][lane] = nz(v) ? v * iv : 0.0;
+        if (lane == 0) T.inv[to] = iv;
+    };
+    if (lead) column(0, 0, T.S[0][lane][0]);
     __syncthreads();
-    const double fr = sf;
-    if (fr == 0.0) return;
-    const int64_t c = p + 1 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= w) return;
-    C[r * w + c] -= fr * C[p * w + c];
+    for (int p = 0; p < kSw; p++) {
+        const int cur = p & 1, nxt = cur ^ 1;
+        auto entry = [&](int rr, int cc) {  // entry (rr, cc) after pivot p
+            if (cc == p) return rr == p ? -T.inv[cur] : T.fac[cur][rr];
+            if (rr == p) return T.fac[cur][cc];
+            const double x = T.S[cur][rr][cc], f = T.fac[cur][rr], g = T.col[cur][cc];
+            return nz(f) && nz(g) ? fma(-f, g, x) : x;
+        };
+        if (lead) {
+            if (p + 1 < kSw) column(nxt, p + 1, entry(max(lane, p + 1), min(lane, p + 1)));
+        } else {
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+                if (r[q] >= 0) T.S[nxt][r[q]][c[q]] = entry(r[q], c[q]);
+        }
+        __syncthreads();
+    }
 }
+// D = -S mirrored (the inverse of the diagonal tile, all kSw x kSw entries)
+__device__ void store_inverse(const SweepTile &T, double *D) {
+    for (int t = threadIdx.x; t < kSw * kSw; t += 256) {
+        const int r = t / kSw, c = t % kSw;
+        D[t] = -(r >= c ? T.S[0][r][c] : T.S[0][c][r]);
+    }
+}
+
+// the inverse of the first diagonal tile
+__global__ void __launch_bounds__(256) k_sweep_first(const double *C, int64_t ld, double *D) {
+    __shared__ SweepTile T;
+    for (int t = threadIdx.x; t < kSw * kSw; t += 256) T.S[0][t / kSw][t % kSw] = C[(t / kSw) * ld + t % kSw];
+    __syncthreads();
+    sweep_tile(T);
+    store_inverse(T, D);
+}
+
+// W_i = A_ik D for 8 rows of a tile row i != k per CTA (four CTAs a tile row), written over A_ik and to Wb, with the old
+// A_ik in Pb; the last CTA writes A_kk = -D.
+__global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *C, const double *D, double *Wb,
+                                                     double *Pb) {
+    constexpr int R = 8;
+    __shared__ double sA[R][kSw + 1], sD[kSw][kSw + 1];
+    if (blockIdx.x == gridDim.x - 1) {
+        for (int t = threadIdx.x; t < kSw * kSw; t += 256)
+            C[((int64_t)k * kSw + t / kSw) * ld + k * kSw + t % kSw] = -D[t];
+        return;
+    }
+    int i = blockIdx.x / (kSw / R);
+    if (i >= k) i++;
+    const int r0 = (blockIdx.x % (kSw / R)) * R;
+    const int r = threadIdx.x / kSw, q = threadIdx.x % kSw;    // row and column, columns fastest
+    const int rt = threadIdx.x % R, qt = threadIdx.x / R;      // rows fastest
+    bool fin = true;
+    double d[kSw * kSw / 256];
+#pragma unroll
+    for (int u = 0; u < kSw * kSw / 256; u++) d[u] = D[threadIdx.x + 256 * u];
+    double a;
+    if (i > k) {  // stored as the tile (i, k)
+        a = C[((int64_t)i * kSw + r0 + r) * ld + k * kSw + q];
+        sA[r][q] = a;
+    } else {  // stored as the transpose of the tile (k, i)
+        a = C[((int64_t)k * kSw + qt) * ld + i * kSw + r0 + rt];
+        sA[rt][qt] = a;
+    }
+    fin &= finite(a);
+#pragma unroll
+    for (int u = 0; u < kSw * kSw / 256; u++) {
+        sD[(threadIdx.x + 256 * u) / kSw][q] = d[u];
+        fin &= finite(d[u]);
+    }
+    const int any = __syncthreads_or(nz(a)), all_finite = __syncthreads_and(fin);
+    const int64_t row = (int64_t)i * kSw + r0 + r;
+    Pb[row * kSw + q] = sA[r][q];
+    if (!any) {  // W_i is zero as A_ik is
+        Wb[row * kSw + q] = 0.0;
+        return;
+    }
+    double w = 0.0;
+    if (all_finite) {
+#pragma unroll 8
+        for (int t = 0; t < kSw; t++) w = fma(sA[r][t], sD[t][q], w);
+    } else {
+        for (int t = 0; t < kSw; t++)
+            if (nz(sA[r][t]) && nz(sD[t][q])) w = fma(sA[r][t], sD[t][q], w);
+    }
+    Wb[row * kSw + q] = w;
+    if (i > k) {
+        C[row * ld + k * kSw + q] = w;
+    } else {  // the transpose, written along the rows of the tile (k, i)
+        __syncthreads();
+        sA[r][q] = w;
+        __syncthreads();
+        C[((int64_t)k * kSw + qt) * ld + i * kSw + r0 + rt] = sA[rt][qt];
+    }
+}
+
+// A_ij -= W_i A_kj for a tile (i, j) of the lower triangle per CTA, i, j != k, m = tile rows - 1; the next diagonal
+// tile is CTA 0's, which also inverts it.
+__global__ void __launch_bounds__(256) k_sweep_update(int64_t ld, int k, int m, double *C, const double *Wb,
+                                                      const double *Pb, double *Dnext) {
+    __shared__ SweepTile T;
+    double(*sW)[kSw + 1] = T.S[0], (*sP)[kSw + 1] = T.S[1];
+    // tile number t of the compressed triangle (block k left out); number 0 and the next diagonal tile change places
+    int t = blockIdx.x;
+    const bool has_next = k < m;
+    if (has_next) {
+        const int tn = k * (k + 1) / 2 + k;
+        if (t == 0) t = tn;
+        else if (t == tn) t = 0;
+    }
+    int i = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+    while ((i + 1) * (i + 2) / 2 <= t) i++;
+    while (i * (i + 1) / 2 > t) i--;
+    int j = t - i * (i + 1) / 2;
+    if (i >= k) i++;
+    if (j >= k) j++;
+    const bool next = has_next && i == k + 1 && j == k + 1;
+    const int ty = threadIdx.x / kSw, tx = threadIdx.x % kSw;
+    double *tile = C + ((int64_t)i * kSw) * ld + (int64_t)j * kSw;
+    double v[4], w[4], p[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        w[u] = Wb[(int64_t)i * kSw * kSw + threadIdx.x + 256 * u];
+        p[u] = Pb[(int64_t)j * kSw * kSw + threadIdx.x + 256 * u];
+        v[u] = tile[(ty + 8 * u) * ld + tx];
+    }
+    bool aw = false, ap = false, fin = true;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        sW[ty + 8 * u][tx] = w[u];
+        sP[ty + 8 * u][tx] = p[u];
+        aw |= nz(w[u]);
+        ap |= nz(p[u]);
+        fin &= finite(w[u]) && finite(p[u]);
+    }
+    const int any_w = __syncthreads_or(aw), any_p = __syncthreads_or(ap), all_finite = __syncthreads_and(fin);
+    const bool work = any_w && any_p;
+    if (!work && !next) return;
+    if (work) {
+        if (all_finite) {  // (a zero factor then adds a zero)
+#pragma unroll 4
+            for (int q = 0; q < kSw; q++) {
+                const double x = -sP[tx][q];
+#pragma unroll
+                for (int u = 0; u < 4; u++) v[u] = fma(sW[ty + 8 * u][q], x, v[u]);
+            }
+        } else {
+            for (int q = 0; q < kSw; q++) {
+                const double x = -sP[tx][q];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (nz(x) && nz(sW[ty + 8 * u][q])) v[u] = fma(sW[ty + 8 * u][q], x, v[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) tile[(ty + 8 * u) * ld + tx] = v[u];
+    }
+    if (!next) return;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; u++) sW[ty + 8 * u][tx] = v[u];
+    __syncthreads();
+    sweep_tile(T);
+    store_inverse(T, Dnext);
+}
+
+// the full inverse from the swept triangle, rows of ldc (padded with zeros)
 template <class V>
-__global__ void k_dense_extract(int64_t nc, const double *C, V *Cinv) {
+__global__ void k_dense_extract(int64_t nc, const double *C, int64_t ld, V *Cinv, int64_t ldc) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nc * nc) return;
-    const int64_t r = t / nc, c = t % nc;
-    Cinv[t] = (V)(C[r * 2 * nc + nc + c] / C[r * 2 * nc + r]);
+    if (t >= nc * ldc) return;
+    const int64_t r = t / ldc, c = t % ldc;
+    Cinv[t] = c >= nc ? V(0) : (V)(-(r >= c ? C[r * ld + c] : C[c * ld + r]));
 }
 // x = Cinv b, warp per row
 template <class V>
-__global__ void k_dense_mv(int64_t nc, const V *Cinv, const V *b, V *x, const int32_t *halt = nullptr) {
+__global__ void k_dense_mv(int64_t nc, const V *Cinv, int64_t ldc, const V *b, V *x, const int32_t *halt = nullptr) {
     const int lane = threadIdx.x & 31;
     const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (r >= nc || (halt && *halt)) return;
     V s = V(0);
     // zero entries skipped: the inverse of a block-diagonal level (the parts of a batch) is block
     // diagonal, and a part's non-finite values must not reach the others through 0 * inf
+#pragma unroll 8
     for (int64_t c = lane; c < nc; c += 32) {
-        const V a = Cinv[r * nc + c];
+        const V a = Cinv[r * ldc + c];
         if (a != V(0)) s = vfma(a, b[c], s);
     }
 #pragma unroll
@@ -1581,7 +1806,8 @@ struct Cycle {
         cudaStream_t s = m->stream;
         AmgLevel &L = g->L[l];
         if (l + 1 == g->L.size()) {
-            k_dense_mv<V><<<nblk(g->nc * 32, 256), 256, 0, s>>>(g->nc, coarse_inverse(g), b, x, g->halt);
+            k_dense_mv<V><<<nblk(g->nc * 32, 256), 256, 0, s>>>(g->nc, coarse_inverse(g), inverse_ld(g->nc), b, x,
+                                                                g->halt);
             AMR_COUNT(1);
             return;
         }
@@ -1756,16 +1982,24 @@ struct Cycle {
         }
         // dense coarsest level
         AmgLevel &D = g->L[nl - 1];
-        const int64_t nc = g->nc, w = 2 * nc;
-        k_dense_init<<<nblk(nc * w, 256), 256, 0, s>>>(nc, g->Cd);
-        k_dense_expand<NM, V><<<nblk(D.n, 128), 128, 0, s>>>(D.n, D.rp, D.cj, vals<V>(D).A, D.nbs, g->Cd, nc);
+        const int64_t nc = g->nc, ld = dense_ld(nc), ldc = inverse_ld(nc);
+        const int nt = (int)(ld / kSw);  // tile rows
+        double *Wb = g->Cd + ld * ld, *Pb = Wb + ld * kSw, *Db = Pb + ld * kSw;
+        AMR_CUDA(cudaMemsetAsync(g->Cd, 0, ld * ld * sizeof(double), s));
+        k_dense_expand<NM, V><<<(unsigned)D.n, 256, 0, s>>>(D.n, D.rp, D.cj, vals<V>(D).A, D.nbs, g->Cd, ld);
+        k_dense_pad<<<1, kSw, 0, s>>>(nc, ld, g->Cd);
         AMR_COUNT(2);
-        // the nc pivot steps as one CUDA graph, captured once per hierarchy (its buffers are fixed)
+        // the sweep steps as one CUDA graph, captured once per hierarchy (its buffers are fixed)
         if (!g->gj_exec) {
             cudaGraph_t gr = nullptr;
             AMR_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-            for (int64_t p = 0; p < nc; p++)
-                k_gj_step<<<dim3(nblk(w - p - 1, 256), (unsigned)nc), 256, 0, s>>>(nc, p, g->Cd);
+            k_sweep_first<<<1, 256, 0, s>>>(g->Cd, ld, Db);
+            for (int k = 0; k < nt; k++) {
+                double *Dk = Db + (k & 1) * kSw * kSw, *Dn = Db + ((k + 1) & 1) * kSw * kSw;
+                k_sweep_panel<<<(unsigned)(4 * (nt - 1) + 1), 256, 0, s>>>(ld, k, g->Cd, Dk, Wb, Pb);
+                const int64_t tiles = (int64_t)(nt - 1) * nt / 2;
+                if (tiles > 0) k_sweep_update<<<(unsigned)tiles, 256, 0, s>>>(ld, k, nt - 1, g->Cd, Wb, Pb, Dn);
+            }
             const cudaError_t ce = cudaStreamEndCapture(s, &gr);
             if (ce == cudaSuccess) {
                 const cudaError_t ie = cudaGraphInstantiate(&g->gj_exec, gr, 0);
@@ -1777,8 +2011,8 @@ struct Cycle {
             }
         }
         AMR_CUDA(cudaGraphLaunch(g->gj_exec, s));
-        AMR_COUNT(nc);
-        k_dense_extract<V><<<nblk(nc * nc, 256), 256, 0, s>>>(nc, g->Cd, coarse_inverse(g));
+        AMR_COUNT(1 + nt + (nt > 1 ? nt : 0));
+        k_dense_extract<V><<<nblk(nc * ldc, 256), 256, 0, s>>>(nc, g->Cd, ld, coarse_inverse(g), ldc);
         AMR_COUNT(1);
         AMR_CUDA(cudaGetLastError());
     }
@@ -1805,7 +2039,7 @@ void ensure_fp64(amr_model *m, AmrAmg *g) {
             amr_alloc(&v.Q, (size_t)std::max<int64_t>(L.nq, 1) * L.b * g->NM);
         }
     }
-    amr_alloc(&g->Cinv64, (size_t)g->nc * g->nc);
+    amr_alloc(&g->Cinv64, (size_t)g->nc * inverse_ld(g->nc));
 }
 
 void prepare_structure(amr_model *m) {
