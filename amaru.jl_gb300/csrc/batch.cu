@@ -40,12 +40,14 @@ namespace {
 constexpr int kPartThreads = 512;  // fixed: the reduction order of a part depends on it
 constexpr int kWarps = kPartThreads / 32;
 constexpr int kCluster = 8;                 // CTAs that solve one large part together
+// Shared memory a CTA's slice should stay within when the part is solved with its matrix in shared memory: all of it, as
+// one such CTA fills an SM's registers anyway and a batch wants few CTAs per part (200 QUAD8 models of 10 to 40 cells
+// a side: 66 ms against 110 ms with 100 KB).
+constexpr size_t kSliceBatch = 224 * 1024;
+constexpr size_t kMaxC2 = 5;  // streams the groups of such parts run on at most (cluster sizes 1 to 16)
 constexpr int64_t kClusterMinNodes = 2048;  // parts with this many nodes or more are large (fixed: results depend on it)
 
-struct PartStat {
-    int32_t iters, refreshes, status, pad;
-    double rel_residual, umax;
-};
+using PartStat = AmrPartStat;
 
 enum { PH_START = 0, PH_ITER = 1, PH_DONE = 2 };
 enum { ACT_NONE = 0, ACT_COMMIT = 1, ACT_RESTORE = 2 };
@@ -996,7 +998,7 @@ __global__ void __launch_bounds__(256) k_ba_finish(int64_t np, int B, const int6
 }  // namespace
 
 struct AmrBatch {
-    int64_t nparts = 0, nlarge = 0;
+    int64_t nparts = 0, nlarge = 0, nstream = 0;  // nstream: parts solved by k_part_pcg, the first of `order`
     std::vector<int64_t> h_ptr;
     int64_t *part_ptr = nullptr, *order = nullptr;
     int32_t *node_part = nullptr, *elem_part = nullptr, *ip_part = nullptr;
@@ -1006,6 +1008,18 @@ struct AmrBatch {
     int32_t *perr = nullptr;
     StepInfo *step = nullptr, *h_step = nullptr;
     unsigned long long *counter = nullptr;
+    // the parts a cluster solves with the matrix in shared memory (resident.cu), grouped by cluster size: a launch per
+    // group, its parts at order[first..first + count), the groups on streams of their own
+    struct Group {
+        AmrResidentShape shape;
+        int64_t first = 0, count = 0;
+    };
+    std::vector<Group> groups;
+    int64_t *slices = nullptr, *first = nullptr;  // their slice bounds, and where each part's begin
+    uint16_t *perm = nullptr;                     // their slices' row orders
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> joined;
+    cudaEvent_t fork = nullptr;
     float *x32 = nullptr, *r32 = nullptr, *z32 = nullptr, *p32 = nullptr, *q32 = nullptr;
     PartAmg *pamg = nullptr;         // per-part state of the multigrid solve
     uint8_t *gate = nullptr;         // its fine-level row gate (nodes of running parts)
@@ -1025,8 +1039,12 @@ void amr_batch_free(amr_model *m) {
     amr_free(b->step); amr_free(b->counter);
     amr_free(b->x32); amr_free(b->r32); amr_free(b->z32); amr_free(b->p32); amr_free(b->q32);
     amr_free(b->pamg); amr_free(b->bsum); amr_free(b->gate);
+    amr_free(b->slices); amr_free(b->first); amr_free(b->perm);
     amr_pinned_free(b->h_step);
     amr_pinned_free(b->h_bsum);
+    for (cudaStream_t s : b->side) cudaStreamDestroy(s);
+    for (cudaEvent_t e : b->joined) cudaEventDestroy(e);
+    if (b->fork) cudaEventDestroy(b->fork);
     delete b;
     m->batch = nullptr;
 }
@@ -1056,14 +1074,66 @@ void amr_batch_set(amr_model *m, int64_t nparts, const int64_t *ptr) {
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(),
                      [&](int64_t x, int64_t y) { return ptr[x + 1] - ptr[x] > ptr[y + 1] - ptr[y]; });
-    int64_t nlarge = 0;
-    while (nlarge < nparts && ptr[order[nlarge] + 1] - ptr[order[nlarge]] >= kClusterMinNodes) nlarge++;
     amr_batch_free(m);
     AmrBatch *b = new AmrBatch();
     m->batch = b;
     try {
+        // the parts that do not fit a cluster's shared memory first, then those that do, by cluster size and, while
+        // the largest slices of their blocks, rows and windows fit together, in one group
+        std::vector<AmrResidentShape> shape(nparts);
+        for (int64_t i = 0; i < nparts; i++) shape[i] = amr_resident_shape(m, ptr[i], ptr[i + 1], kSliceBatch);
+        std::stable_sort(order.begin(), order.end(), [&](int64_t x, int64_t y) {
+            const int cx = shape[x].ctas ? shape[x].ctas : INT32_MAX, cy = shape[y].ctas ? shape[y].ctas : INT32_MAX;
+            return cx > cy;
+        });
+        int64_t nstream = 0, nlarge = 0;
+        while (nstream < nparts && !shape[order[nstream]].ctas) nstream++;
+        while (nlarge < nstream && ptr[order[nlarge] + 1] - ptr[order[nlarge]] >= kClusterMinNodes) nlarge++;
+        for (int64_t i = nstream; i < nparts; i++) {
+            const AmrResidentShape &s = shape[order[i]];
+            if (!b->groups.empty() && b->groups.back().shape.ctas == s.ctas) {
+                AmrResidentShape u = b->groups.back().shape;
+                u.slots = std::max(u.slots, s.slots);
+                u.rows = std::max(u.rows, s.rows);
+                u.window = std::max(u.window, s.window);
+                u.bytes = amr_resident_bytes(m, u);
+                if (u.bytes <= amr_resident_max_bytes()) {
+                    b->groups.back().shape = u;
+                    b->groups.back().count++;
+                    continue;
+                }
+            }
+            b->groups.push_back({s, i, 1});
+        }
+        if (!b->groups.empty()) {
+            std::vector<int64_t> first(nparts, 0), slices;
+            std::vector<uint16_t> perm(m->nnodes, 0);
+            for (int64_t i = 0; i < nparts; i++) {
+                first[i] = (int64_t)slices.size();
+                slices.insert(slices.end(), shape[i].bounds.begin(), shape[i].bounds.end());
+                std::copy(shape[i].perm.begin(), shape[i].perm.end(), perm.begin() + ptr[i]);
+            }
+            amr_alloc(&b->perm, perm.size());
+            amr_h2d(m, b->perm, perm.data(), perm.size() * sizeof(uint16_t));
+            amr_alloc(&b->slices, slices.size());
+            amr_alloc(&b->first, nparts);
+            amr_h2d(m, b->slices, slices.data(), slices.size() * sizeof(int64_t));
+            amr_h2d(m, b->first, first.data(), nparts * sizeof(int64_t));
+        }
+        if (b->groups.size() > 1) {
+            AMR_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+            for (size_t g = 1; g < std::min<size_t>(b->groups.size(), kMaxC2); g++) {
+                cudaStream_t st = nullptr;
+                AMR_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+                b->side.push_back(st);
+                cudaEvent_t ev = nullptr;
+                AMR_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+                b->joined.push_back(ev);
+            }
+        }
         b->nparts = nparts;
         b->nlarge = nlarge;
+        b->nstream = nstream;
         b->ctas_per_sm = m->B == 2 ? part_min_blocks<2>() : part_min_blocks<3>();
         b->h_ptr.assign(ptr, ptr + nparts + 1);
         const int64_t n = m->nnodes * m->B;
@@ -1107,7 +1177,7 @@ PcgArgs pcg_args(amr_model *m, double *x, const double *b_, double *reac, const 
                  const uint8_t *active) {
     AmrBatch *b = m->batch;
     PcgArgs a;
-    a.nlarge = b->nlarge; a.nsmall = b->nparts - b->nlarge; a.part_ptr = b->part_ptr; a.order = b->order;
+    a.nlarge = b->nlarge; a.nsmall = b->nstream - b->nlarge; a.part_ptr = b->part_ptr; a.order = b->order;
     a.active = active;
     a.nb = m->bstride; a.rp = m->brow_ptr; a.cj = m->bcol; a.K32 = m->K32; a.K64 = m->K64; a.Minv = m->Minv32;
     a.fm = m->free_mask; a.b = b_; a.x = x; a.reac = reac;
@@ -1119,16 +1189,33 @@ PcgArgs pcg_args(amr_model *m, double *x, const double *b_, double *reac, const 
 
 void launch_pcg(amr_model *m, const PcgArgs &a, int ctas_per_sm) {
     AmrBatch *b = m->batch;
-    AMR_CUDA(cudaMemsetAsync(b->counter, 0, 2 * sizeof(unsigned long long), m->stream));
-    // whole clusters: as many CTAs as the parts can use (a cluster per large part, a CTA per small
-    // one), at most ctas_per_sm per SM
-    const int64_t need = b->nlarge * kCluster + (b->nparts - b->nlarge);
-    const int64_t ctas = std::min<int64_t>(std::max<int64_t>(need, kCluster), (int64_t)device_sms() * ctas_per_sm);
-    const unsigned grid = (unsigned)(std::max<int64_t>(1, ctas / kCluster) * kCluster);
-    if (m->B == 3) k_part_pcg<3><<<grid, kPartThreads, 0, m->stream>>>(a);
-    else k_part_pcg<2><<<grid, kPartThreads, 0, m->stream>>>(a);
-    AMR_COUNT(1);
-    AMR_CUDA(cudaGetLastError());
+    // the groups whose matrices stay in shared memory, largest clusters first, side by side
+    if (!b->side.empty()) AMR_CUDA(cudaEventRecord(b->fork, m->stream));
+    for (size_t g = 0; g < b->groups.size(); g++) {
+        const AmrBatch::Group &q = b->groups[g];
+        const size_t lane = b->side.empty() ? 0 : g % (b->side.size() + 1);  // 0: the handle's stream
+        cudaStream_t st = lane == 0 ? m->stream : b->side[lane - 1];
+        if (lane > 0 && g == lane) AMR_CUDA(cudaStreamWaitEvent(st, b->fork, 0));
+        amr_resident_launch(m, q.shape, q.count, b->slices, b->first, b->perm, b->order + q.first, a.active, a.b, a.x, a.reac, a.stat,
+                            a.step ? &a.step->t0 : nullptr, a.step ? &a.step->t1 : nullptr, a.tol2, a.max_iters,
+                            a.force_every, st);
+    }
+    if (b->nstream > 0) {
+        AMR_CUDA(cudaMemsetAsync(b->counter, 0, 2 * sizeof(unsigned long long), m->stream));
+        // whole clusters: as many CTAs as the parts can use (a cluster per large part, a CTA per small
+        // one), at most ctas_per_sm per SM
+        const int64_t need = b->nlarge * kCluster + (b->nstream - b->nlarge);
+        const int64_t ctas = std::min<int64_t>(std::max<int64_t>(need, kCluster), (int64_t)device_sms() * ctas_per_sm);
+        const unsigned grid = (unsigned)(std::max<int64_t>(1, ctas / kCluster) * kCluster);
+        if (m->B == 3) k_part_pcg<3><<<grid, kPartThreads, 0, m->stream>>>(a);
+        else k_part_pcg<2><<<grid, kPartThreads, 0, m->stream>>>(a);
+        AMR_COUNT(1);
+        AMR_CUDA(cudaGetLastError());
+    }
+    for (size_t i = 0; i < b->side.size(); i++) {
+        AMR_CUDA(cudaEventRecord(b->joined[i], b->side[i]));
+        AMR_CUDA(cudaStreamWaitEvent(m->stream, b->joined[i], 0));
+    }
 }
 
 struct GraphScope {

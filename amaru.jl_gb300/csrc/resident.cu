@@ -1,0 +1,700 @@
+// Block-Jacobi PCG of a small model, or of the parts of a batch, with the matrix kept in shared memory.
+//
+// A part (a contiguous range of nodes that no element leaves; a small model is one part) is solved by a cluster of
+// 1 to 16 CTAs in one launch: solve_system! (src/solver.jl:5-79) by the mixed-precision method of solver.cu, FP32 PCG
+// with FP64 true-residual refreshes.  CTA r owns a contiguous slice of the rows, of about equal numbers of blocks (so
+// that nodes no element uses change nothing).  Its blocks of K32, with 16-bit
+// column offsets, stay in its shared memory over all iterations, beside the direction p over the slice's column
+// window; x, r, q and the block inverses of its rows are in registers.
+//
+// The matrix product is bound by shared-memory wavefronts.  Its rows are sorted by their number of blocks and laid out
+// lane by lane (one thread per row, or 2 or 4 where the rows are few): 32 blocks then take 7 wavefronts in 2-D, 4 of
+// them the values, without conflicts or shuffles.  8 lanes per row over the rows' own layout took 4.9 times as long
+// (9 430 cycles for 586 rows and 8 568 blocks).
+//
+// What else bounds it is the chain of an iteration, two cluster-wide sums (p.q, then r.z and r.r).  So:
+//   * the direction needs no sum of its own: a CTA pushes the z of its rows into the windows of the CTAs that read them,
+//     and after the second sum each forms p = z + beta p over its whole window;
+//   * what a CTA sends, its partial sum and its z, goes by st.async into the others' shared memory and is counted by
+//     their mbarriers, so a sum is one CTA barrier and one way across the cluster, with no fence; every warp
+//     adds the cluster's partials itself.  As each CTA waits for all, a sum is a barrier of the cluster: the slots and
+//     windows are never written while they may be read;
+//   * nothing in an iteration takes the FP64 pipe (two lanes a clock per SM): the partials of the CTAs, FP32 as in
+//     solver.cu, are added as pairs hi + lo by two-sums (48 bits), and alpha and beta are quotients of such pairs.
+// Measured, three launches per iteration over all SMs before: 26 us an iteration, now 2.7 us (1 613 QUAD8 nodes, 8
+// CTAs); a batch of 64 QUAD8 models of 10 to 60 cells a side 230 ms, now 42 ms.
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+#include <type_traits>
+
+#include <cooperative_groups.h>
+
+#include "amr_internal.h"
+
+namespace cg = cooperative_groups;
+
+namespace {
+
+constexpr int kT = 512;             // threads of a CTA
+constexpr int kW = kT / 32;
+constexpr int kRowsPerThread = 2;   // rows a thread keeps in registers
+constexpr int kMaxC = 16;           // CTAs of a cluster at most (above 8 where the device allows it)
+constexpr size_t kMaxDyn = 224 * 1024;
+
+struct Args {
+    const int64_t *slices, *first;   // the parts' slice bounds, and where a part's begin (null: 0)
+    const uint16_t *perm;            // per node: at n0 + i the i-th row of its slice by descending length, as n - n0
+    const int64_t *list;             // the launch's parts, a cluster each (null: part 0)
+    const uint8_t *active;           // null: every part
+    int64_t nb;
+    const int64_t *rp;
+    const int32_t *cj;
+    const float *K32;
+    const double *K64;
+    const float *Minv;
+    const uint8_t *fm;
+    const double *b;
+    double *x, *reac;
+    AmrPartStat *stat;
+    unsigned long long *t0, *t1;     // null: no timing
+    double tol2;
+    int max_iters, force_every;
+    int kcap, wcap;                  // slots of blocks and window nodes of a slice at most
+};
+
+// a value hi + lo of two FP32 numbers
+struct Pair {
+    float h, l;
+};
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+    const float s = __fadd_rn(a.h, b.h);
+    const float t = __fsub_rn(s, a.h);
+    const float e = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, t)), __fsub_rn(b.h, t));
+    const float l = __fadd_rn(__fadd_rn(a.l, b.l), e);
+    const float h = __fadd_rn(s, l);
+    return Pair{h, __fsub_rn(l, __fsub_rn(h, s))};
+}
+// a / b rounded to FP32
+__device__ __forceinline__ float pair_div(Pair a, Pair b) {
+    const float q = __fdiv_rn(a.h, b.h);
+    const float r = __fadd_rn(__fmaf_rn(-q, b.h, a.h), __fmaf_rn(-q, b.l, a.l));
+    return __fadd_rn(q, __fdiv_rn(r, b.h));
+}
+
+template <int B>
+size_t slice_bytes(int64_t slots, int64_t rows, int64_t window) {
+    (void)rows;
+    return (size_t)slots * (B * B * 4 + 2) + (size_t)window * 2 * B * 4;
+}
+// threads per row of a part whose slices have at most `rows` rows with blocks
+__host__ __device__ inline int threads_per_row(int64_t rows) { return rows * 4 <= kT ? 4 : rows * 2 <= kT ? 2 : 1; }
+
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ uint32_t shared_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int r) {  // the same place in rank r's shared memory
+    uint32_t remote;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(r));
+    return remote;
+}
+// v to a place in a CTA's shared memory, counted by an mbarrier there
+__device__ __forceinline__ void store_async(uint32_t to, float v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(to), "f"(v), "r"(bar)
+                 : "memory");
+}
+// waits for the phase of an mbarrier to complete; false after a limit far above any wait here
+__device__ __forceinline__ bool wait_phase(uint32_t bar, unsigned parity) {
+    for (int i = 0; i < (1 << 20); i++) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                     "selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(done)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+template <int B>
+__device__ __forceinline__ void load_node(const float *p, float *v) {
+    if constexpr (B == 2) {
+        const float2 f = *reinterpret_cast<const float2 *>(p);
+        v[0] = f.x;
+        v[1] = f.y;
+    } else {
+#pragma unroll
+        for (int d = 0; d < B; d++) v[d] = p[d];
+    }
+}
+
+template <int B>
+__global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
+    constexpr int BB = B * B, G = 8, M = kRowsPerThread;
+    extern __shared__ float dyn[];
+    __shared__ float s_warp[2 * kW];
+    __shared__ int s_off[M * kW + 1];       // first slot of each 32 rows' (row parts') blocks
+    __shared__ float s_slot[2][2][kMaxC];   // the cluster's partials of the two sums
+    __shared__ double s_slotd[2][kMaxC], s_dwarp[2][kW], s_dtot[2], s_um[kMaxC];
+    __shared__ __align__(8) uint64_t s_bar[2];                      // the two sums' arrivals
+    __shared__ int s_w0, s_w1, s_win[kMaxC][2], s_bytes;
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const long long part = a.list ? a.list[blockIdx.x / C] : 0;
+    if (a.active && !a.active[part]) return;  // (uniform over the cluster)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (a.t0 && tid == 0) atomicMin(a.t0, global_ns());
+    auto barrier = [&]() {
+        if (C > 1) cl.sync();
+        else __syncthreads();
+    };
+
+    // ---- the slice: rows [n0, n1), their blocks and the window of their columns
+    const int64_t *bound = a.slices + (a.first ? a.first[part] : 0);
+    const int64_t n0 = bound[rank], n1 = bound[rank + 1];
+    const int R = (int)(n1 - n0);
+    const int64_t k0 = a.rp[n0];
+    const int nk = (int)(a.rp[n1] - k0);
+    float4 *val4 = reinterpret_cast<float4 *>(dyn);           // [BB / 4][kcap]: the blocks' first 4 or 8 values
+    float *val1 = dyn + (size_t)(BB / 4) * 4 * a.kcap;        // [kcap] the ninth (3-D)
+    float *pwin = val1 + (size_t)(BB % 4) * a.kcap;           // [window][B]
+    float *zwin = pwin + (size_t)B * a.wcap;                  // [window][B], own rows and what the others push
+    uint16_t *cols = (uint16_t *)(zwin + (size_t)B * a.wcap); // [kcap]
+    if (tid == 0) {
+        s_w0 = (int)n0;
+        s_w1 = (int)n1;
+        s_bytes = 0;
+        for (int i = 0; i < 2; i++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_addr(&s_bar[i])), "r"(1) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    {
+        int lo = (int)n0, hi = (int)n1;
+        for (int k = tid; k < nk; k += kT) {
+            const int j = a.cj[k0 + k];
+            lo = min(lo, j);
+            hi = max(hi, j + 1);
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane == 0) { atomicMin(&s_w0, lo); atomicMax(&s_w1, hi); }
+    }
+    __syncthreads();
+    const int w0 = s_w0, W = s_w1 - w0, own = (int)n0 - w0;
+    // the rows with blocks, sorted: thread tid has the parts sub of the rows at (tid + m kT) / S
+    int most = 0, Rn = 0;  // (over the part's slices, so that S belongs to the part)
+    for (int r = 0; r < C; r++) {
+        const int64_t b0 = bound[r], b1 = bound[r + 1];
+        int lo = 0, hi = (int)(b1 - b0);  // rows without blocks are sorted last
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            const int64_t n = b0 + a.perm[b0 + mid];
+            if (a.rp[n + 1] > a.rp[n]) lo = mid + 1;
+            else hi = mid;
+        }
+        most = max(most, lo);
+        if (r == rank) Rn = lo;
+    }
+    const int S = threads_per_row(most), sub = tid & (S - 1);
+    int row[M], width[M];  // row: -1 none
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        const int i = (tid + m * kT) / S;
+        row[m] = i < Rn ? (int)a.perm[n0 + i] : -1;
+        const int n = row[m] >= 0 ? (int)(a.rp[n0 + row[m] + 1] - a.rp[n0 + row[m]]) : 0;
+        width[m] = __reduce_max_sync(0xffffffffu, (n + S - 1) / S);
+        if (lane == 0) s_off[m * kW + warp + 1] = 32 * width[m];
+    }
+    __syncthreads();
+    if (tid == 0) {
+        s_off[0] = 0;
+        for (int i = 0; i < M * kW; i++) s_off[i + 1] += s_off[i];
+    }
+    __syncthreads();
+    int slot0[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        slot0[m] = s_off[m * kW + warp] + lane;
+        const int64_t ks = row[m] >= 0 ? a.rp[n0 + row[m]] : 0, ke = row[m] >= 0 ? a.rp[n0 + row[m] + 1] : 0;
+        for (int t = 0; t < width[m]; t++) {
+            const int64_t k = ks + t * S + sub;
+            const bool in = k < ke;
+            float v[BB];
+#pragma unroll
+            for (int q = 0; q < BB; q++) v[q] = in ? a.K32[(int64_t)q * a.nb + k] : 0.0f;
+            const int e = slot0[m] + 32 * t;
+            cols[e] = in ? (uint16_t)(a.cj[k] - w0) : (uint16_t)own;
+#pragma unroll
+            for (int q = 0; q < BB / 4; q++) val4[q * a.kcap + e] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            if (BB % 4) val1[e] = v[BB - 1];
+        }
+    }
+    // the bytes of z the others push here: their rows with blocks in this window
+    {
+        int got = 0;
+        for (int i = tid; i < W; i += kT) {
+            const int64_t n = w0 + i;
+            if ((n < n0 || n >= n1) && a.rp[n + 1] > a.rp[n]) got += B * 4;
+        }
+        got = __reduce_add_sync(0xffffffffu, got);
+        if (lane == 0) atomicAdd(&s_bytes, got);
+    }
+    for (int i = tid; i < W * B; i += kT) pwin[i] = zwin[i] = 0.0f;
+    if (sub != 0)  // from here on a row's first thread owns it
+#pragma unroll
+        for (int m = 0; m < M; m++) row[m] = -1;
+    float xr[M][B], rv[M][B], mi[M][BB];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+#pragma unroll
+        for (int c = 0; c < B; c++) xr[m][c] = rv[m][c] = 0.0f;
+#pragma unroll
+        for (int q = 0; q < BB; q++) mi[m][q] = row[m] >= 0 ? a.Minv[(n0 + row[m]) * BB + q] : 0.0f;
+    }
+
+    // every CTA's window; the ranks (bits) whose windows hold a row of this thread
+    if (tid < C) {
+        *cl.map_shared_rank(&s_win[rank][0], tid) = w0;
+        *cl.map_shared_rank(&s_win[rank][1], tid) = w0 + W;
+    }
+    barrier();  // (also: every CTA's mbarriers and zero window exist before a neighbour writes there)
+    const int bytes2 = s_bytes + 2 * C * 4;  // what arrives here in a second sum
+    unsigned to[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        to[m] = 0;
+        const int n = (int)n0 + row[m];
+        if (row[m] >= 0)
+            for (int r = 0; r < C; r++)
+                if (r != rank && n >= s_win[r][0] && n < s_win[r][1]) to[m] |= 1u << r;
+    }
+    // z of this thread's row m into its window and the others'; counted (st.async) by their second mbarrier, or plain
+    // stores that a barrier of the cluster follows
+    auto push_z = [&](auto counted, int m, const float *z) {
+        float *mine = zwin + (own + row[m]) * B;
+#pragma unroll
+        for (int c = 0; c < B; c++) mine[c] = z[c];
+        for (unsigned t = to[m]; t; t &= t - 1) {
+            const int r = __ffs(t) - 1;
+            const uint32_t z_to = cluster_addr(shared_addr(zwin + ((int)n0 + row[m] - s_win[r][0]) * B), r);
+            if constexpr (decltype(counted)::value) {
+                const uint32_t bar = cluster_addr(shared_addr(&s_bar[1]), r);
+#pragma unroll
+                for (int c = 0; c < B; c++) store_async(z_to + 4 * c, z[c], bar);
+            } else {
+#pragma unroll
+                for (int c = 0; c < B; c++)
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(z_to + 4 * c), "f"(z[c]) : "memory");
+            }
+        }
+    };
+    // where this CTA's partials go: lanes r and 16 + r push to rank r
+    const int half = lane >> 4, hl = lane & 15;
+    const uint32_t slot_to = cluster_addr(shared_addr(&s_slot[0][half][rank]), min(hl, C - 1)),
+                   bar_to = cluster_addr(shared_addr(&s_bar[0]), min(hl, C - 1));
+    unsigned parity = 0;  // bit i: the phase of s_bar[i] to wait for
+    bool timeout = false;
+    // the cluster's sums of v0 (and v1, with two), the same pairs in every thread; set: the slots used.  Two sums share
+    // their steps, one in each half of a warp.
+    auto cluster_sum = [&](auto two, int set, float v0, float v1, Pair &o0, Pair &o1) {
+        constexpr bool two_sums = decltype(two)::value;
+        float t;
+        if (two_sums) t = (half ? v1 : v0) + __shfl_xor_sync(0xffffffffu, half ? v0 : v1, 16);
+        else t = v0 + __shfl_xor_sync(0xffffffffu, v0, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (hl == 0) s_warp[half * kW + warp] = t;
+        __syncthreads();
+        if (warp == 0) {
+            t = s_warp[two_sums ? lane : hl];
+#pragma unroll
+            for (int o = kW / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (hl < C && (two_sums || half == 0)) store_async(slot_to + set * 2 * kMaxC * 4, t, bar_to + set * 8);
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(&s_bar[set])),
+                             "r"(two_sums ? bytes2 : C * 4) : "memory");
+        }
+        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u);
+        parity ^= 1u << set;
+        Pair p{hl < C ? s_slot[set][two_sums ? half : 0][hl] : 0.0f, 0.0f};
+#pragma unroll
+        for (int o = kMaxC / 2; o > 0; o >>= 1)
+            p = pair_add(p, Pair{__shfl_xor_sync(0xffffffffu, p.h, o), __shfl_xor_sync(0xffffffffu, p.l, o)});
+        if (two_sums) {
+            const Pair q{__shfl_xor_sync(0xffffffffu, p.h, 16), __shfl_xor_sync(0xffffffffu, p.l, 16)};
+            o0 = half ? q : p;
+            o1 = half ? p : q;
+        } else {
+            o0 = p;
+        }
+    };
+    // FP64 sums (a refresh only), valid in every thread
+    auto cluster_sum64 = [&](double v0, double v1, double &t0, double &t1) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v0 += __shfl_down_sync(0xffffffffu, v0, o);
+            v1 += __shfl_down_sync(0xffffffffu, v1, o);
+        }
+        if (lane == 0) { s_dwarp[0][warp] = v0; s_dwarp[1][warp] = v1; }
+        __syncthreads();
+        if (warp == 0) {
+            double u0 = lane < kW ? s_dwarp[0][lane] : 0.0, u1 = lane < kW ? s_dwarp[1][lane] : 0.0;
+#pragma unroll
+            for (int o = kW / 2; o > 0; o >>= 1) {
+                u0 += __shfl_xor_sync(0xffffffffu, u0, o);
+                u1 += __shfl_xor_sync(0xffffffffu, u1, o);
+            }
+            if (lane < C) {
+                *cl.map_shared_rank(&s_slotd[0][rank], lane) = u0;
+                *cl.map_shared_rank(&s_slotd[1][rank], lane) = u1;
+            }
+        }
+        barrier();
+        if (warp == 0) {
+            double u0 = lane < C ? s_slotd[0][lane] : 0.0, u1 = lane < C ? s_slotd[1][lane] : 0.0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                u0 += __shfl_xor_sync(0xffffffffu, u0, o);
+                u1 += __shfl_xor_sync(0xffffffffu, u1, o);
+            }
+            if (lane == 0) { s_dtot[0] = u0; s_dtot[1] = u1; }
+        }
+        __syncthreads();
+        t0 = s_dtot[0];
+        t1 = s_dtot[1];
+    };
+    auto split = [](double v) {
+        const float h = (float)v;
+        return Pair{h, (float)(v - (double)h)};
+    };
+    // the FP64 true residual of the slice from a.x (published by a barrier before): r, z = Minv r, r.z and |r|^2
+    auto residual64 = [&](double &rz, double &rr) {
+        const int gl = tid % G, grp = tid / G;
+        const unsigned gmask = 0xffu << (G * ((tid & 31) / G));
+        double srr = 0.0, srz = 0.0;
+        for (int i = grp; i < R; i += kT / G) {
+            const int64_t n = n0 + i;
+            double acc[B];
+#pragma unroll
+            for (int c = 0; c < B; c++) acc[c] = 0.0;
+            for (int64_t k = a.rp[n] + gl; k < a.rp[n + 1]; k += G) {
+                const int64_t j = a.cj[k];
+                double u[B];
+#pragma unroll
+                for (int d = 0; d < B; d++) u[d] = __ldcg(a.x + j * B + d);
+#pragma unroll
+                for (int c = 0; c < B; c++)
+#pragma unroll
+                    for (int d = 0; d < B; d++) acc[c] = fma(__ldg(a.K64 + (int64_t)(c * B + d) * a.nb + k), u[d], acc[c]);
+            }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int c = 0; c < B; c++) acc[c] += __shfl_down_sync(gmask, acc[c], o, G);
+            if (gl == 0)
+#pragma unroll
+                for (int c = 0; c < B; c++) {
+                    double res = 0.0;
+                    if (a.fm[n * B + c]) res = a.b[n * B + c] - acc[c];
+                    else if (a.reac) a.reac[n * B + c] = acc[c];
+                    zwin[(own + i) * B + c] = (float)res;
+                    srr = fma(res, res, srr);
+                }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            const int i = row[m];
+            if (i < 0) continue;
+#pragma unroll
+            for (int c = 0; c < B; c++) rv[m][c] = zwin[(own + i) * B + c];
+            float z[B];
+#pragma unroll
+            for (int c = 0; c < B; c++) {
+                z[c] = 0.0f;
+#pragma unroll
+                for (int d = 0; d < B; d++) z[c] = fmaf(mi[m][c * B + d], rv[m][d], z[c]);
+                srz = fma((double)rv[m][c], (double)z[c], srz);
+            }
+            push_z(std::false_type(), m, z);
+        }
+        cluster_sum64(srz, srr, rz, rr);
+    };
+
+    double rz64, rr_true;
+    residual64(rz64, rr_true);
+    const double bnorm2 = rr_true;
+    const float stop_rr = (float)(0.0625 * a.tol2 * bnorm2);
+    Pair gam = split(rz64);
+    float thr = fmaxf(stop_rr, (float)(1e-2 * rr_true)), beta = 0.0f;
+    int iters = 0, refreshes = 0, status = 0, since = 0;
+    bool done = !(bnorm2 > 0.0) || rr_true <= a.tol2 * bnorm2;
+    if (isnan(rr_true)) { status = AMR_ENOCONV; done = true; }
+    while (!done) {
+        if (iters >= a.max_iters) { status = AMR_ENOCONV; break; }
+        // p = z + beta p over the window
+#pragma unroll 4
+        for (int i = tid; i < W * B; i += kT) pwin[i] = fmaf(beta, pwin[i], zwin[i]);
+        __syncthreads();
+        // q = K32 p, p.q
+        float q[M][B], dot = 0.0f;
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+#pragma unroll
+            for (int c = 0; c < B; c++) q[m][c] = 0.0f;
+            int e = slot0[m];
+#pragma unroll 4
+            for (int t = 0; t < width[m]; t++, e += 32) {
+                const int j = (int)cols[e] * B;
+                float v[BB], pv[B];
+#pragma unroll
+                for (int u = 0; u < BB / 4; u++) {
+                    const float4 f = val4[u * a.kcap + e];
+                    v[4 * u] = f.x; v[4 * u + 1] = f.y; v[4 * u + 2] = f.z; v[4 * u + 3] = f.w;
+                }
+                if (BB % 4) v[BB - 1] = val1[e];
+                load_node<B>(pwin + j, pv);
+#pragma unroll
+                for (int c = 0; c < B; c++)
+#pragma unroll
+                    for (int d = 0; d < B; d++) q[m][c] = fmaf(v[c * B + d], pv[d], q[m][c]);
+            }
+            if (S > 1)  // (uniform)
+#pragma unroll
+                for (int c = 0; c < B; c++) {
+                    q[m][c] += __shfl_xor_sync(0xffffffffu, q[m][c], 1);
+                    if (S > 2) q[m][c] += __shfl_xor_sync(0xffffffffu, q[m][c], 2);
+                }
+            if (row[m] >= 0)
+#pragma unroll
+                for (int c = 0; c < B; c++) dot = fmaf(pwin[(own + row[m]) * B + c], q[m][c], dot);
+        }
+        Pair pq, t2[2];
+        cluster_sum(std::false_type(), 0, dot, 0.0f, pq, pq);
+        if (timeout) { status = AMR_ETIMEOUT; break; }
+        if (!(pq.h > 0.0f)) { status = AMR_ENOCONV; break; }
+        const float alpha = pair_div(gam, pq);
+        // x += alpha p ; r -= alpha q ; z = Minv r
+        float v0 = 0.0f, v1 = 0.0f;
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            const int i = row[m];
+            if (i < 0) continue;
+#pragma unroll
+            for (int c = 0; c < B; c++) {
+                xr[m][c] = fmaf(alpha, pwin[(own + i) * B + c], xr[m][c]);
+                rv[m][c] = fmaf(-alpha, q[m][c], rv[m][c]);
+            }
+            float z[B];
+#pragma unroll
+            for (int c = 0; c < B; c++) {
+                z[c] = 0.0f;
+#pragma unroll
+                for (int d = 0; d < B; d++) z[c] = fmaf(mi[m][c * B + d], rv[m][d], z[c]);
+                v0 = fmaf(rv[m][c], z[c], v0);
+                v1 = fmaf(rv[m][c], rv[m][c], v1);
+            }
+            push_z(std::true_type(), m, z);
+        }
+        cluster_sum(std::true_type(), 1, v0, v1, t2[0], t2[1]);
+        if (timeout) { status = AMR_ETIMEOUT; break; }
+        beta = pair_div(t2[0], gam);
+        gam = t2[0];
+        iters++;
+        since++;
+        if (!(t2[1].h > thr) || since >= a.force_every) {
+            // refresh: fold the FP32 correction into the FP64 solution and recompute the true residual
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                const int i = row[m];
+                if (i < 0) continue;
+#pragma unroll
+                for (int c = 0; c < B; c++) {
+                    const int64_t g = (n0 + i) * B + c;
+                    if (a.fm[g]) a.x[g] += (double)xr[m][c];
+                    xr[m][c] = 0.0f;
+                }
+            }
+            __threadfence();
+            barrier();
+            residual64(rz64, rr_true);
+            gam = split(rz64);
+            thr = fmaxf(stop_rr, (float)(1e-2 * rr_true));
+            refreshes++;
+            since = 0;
+            if (isnan(rr_true)) { status = AMR_ENOCONV; break; }
+            if (rr_true <= a.tol2 * bnorm2) done = true;
+        }
+    }
+    // the largest |x| at free slots (NaN as +inf), and the part's statistics
+    double um = 0.0;
+    for (int64_t i = n0 * B + tid; i < n1 * B; i += kT)
+        if (a.fm[i]) {
+            const double v = fabs(a.x[i]);
+            um = fmax(um, isnan(v) ? INFINITY : v);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) um = fmax(um, __shfl_down_sync(0xffffffffu, um, o));
+    __syncthreads();
+    if (lane == 0) s_dwarp[0][warp] = um;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kW; w++) um = fmax(um, s_dwarp[0][w]);
+        *cl.map_shared_rank(&s_um[rank], 0) = um;
+    }
+    barrier();  // (also: no CTA leaves while a neighbour may read its shared memory)
+    if (rank == 0 && tid == 0) {
+        for (int r = 0; r < C; r++) um = fmax(um, s_um[r]);
+        AmrPartStat s;
+        s.iters = iters;
+        s.refreshes = refreshes;
+        s.status = status;
+        s.pad = 0;
+        s.rel_residual = bnorm2 > 0.0 ? sqrt(rr_true / bnorm2) : 0.0;
+        s.umax = um;
+        a.stat[part] = s;
+    }
+    if (a.t1 && tid == 0) atomicMax(a.t1, global_ns());
+}
+
+// the kernels' attributes, once per device and process (a launch that changed them would race with others); the
+// largest cluster the device takes with the largest slice
+int device_cluster() {
+    static std::mutex mu;
+    static int found[64] = {0};
+    int dev = 0;
+    AMR_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lk(mu);
+    if (found[dev]) return found[dev] < 0 ? 0 : found[dev];
+    int best = -1;
+    const void *kernels[2] = {(const void *)k_resident_pcg<2>, (const void *)k_resident_pcg<3>};
+    bool ok = true, wide = true;
+    for (const void *k : kernels) {
+        ok &= cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn) == cudaSuccess;
+        wide &= cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    }
+    if (ok)
+        for (int c : {16, 8}) {
+            if (c > 8 && !wide) continue;
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = (unsigned)c;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.gridDim = dim3((unsigned)c);
+            cfg.blockDim = dim3(kT);
+            cfg.dynamicSmemBytes = kMaxDyn;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int n2 = 0, n3 = 0;
+            if (cudaOccupancyMaxActiveClusters(&n2, k_resident_pcg<2>, &cfg) == cudaSuccess &&
+                cudaOccupancyMaxActiveClusters(&n3, k_resident_pcg<3>, &cfg) == cudaSuccess && n2 > 0 && n3 > 0) {
+                best = c;
+                break;
+            }
+        }
+    cudaGetLastError();
+    found[dev] = best;
+    return best < 0 ? 0 : best;
+}
+
+}  // namespace
+
+// The cluster size that solves nodes [P0, P1), and the largest slice: the smallest whose slices stay within `prefer`
+// bytes of shared memory, else the largest the device takes if its slices fit at all; 0: none.
+AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer) {
+    AmrResidentShape best;
+    const int most = device_cluster();
+    const int64_t len = P1 - P0;
+    if (most == 0 || len <= 0 || len > (int64_t)most * 65535) return best;
+    const std::vector<int64_t> &rp = m->h_brow_ptr;
+    for (int C = 1; C <= most; C *= 2) {
+        AmrResidentShape s;
+        s.ctas = C;
+        s.bounds.resize(C + 1);
+        for (int r = 0; r <= C; r++)
+            s.bounds[r] = r == 0   ? P0
+                          : r == C ? P1
+                                   : std::lower_bound(rp.begin() + P0, rp.begin() + P1, rp[P0] + (rp[P1] - rp[P0]) * r / C) -
+                                         rp.begin();
+        s.perm.resize(len);
+        int64_t most_rows = 0;
+        for (int r = 0; r < C; r++) {
+            const int64_t n0 = s.bounds[r], n1 = s.bounds[r + 1];
+            if (n1 - n0 > 65535) { s.rows = n1 - n0; break; }
+            uint16_t *pm = s.perm.data() + (n0 - P0);
+            for (int64_t i = 0; i < n1 - n0; i++) pm[i] = (uint16_t)i;
+            std::stable_sort(pm, pm + (n1 - n0), [&](uint16_t x, uint16_t y) {
+                return rp[n0 + x + 1] - rp[n0 + x] > rp[n0 + y + 1] - rp[n0 + y];
+            });
+            int64_t used = 0;
+            while (used < n1 - n0 && rp[n0 + pm[used] + 1] > rp[n0 + pm[used]]) used++;
+            most_rows = std::max(most_rows, used);
+            s.rows = std::max(s.rows, n1 - n0);
+        }
+        if (s.rows > 65535 || most_rows > kT * kRowsPerThread) continue;
+        const int S = threads_per_row(most_rows);
+        bool fits = true;
+        for (int r = 0; r < C && fits; r++) {
+            const int64_t n0 = s.bounds[r], n1 = s.bounds[r + 1];
+            const uint16_t *pm = s.perm.data() + (n0 - P0);
+            int64_t lo = n0, hi = n1, slots = 0;
+            for (int64_t n = n0; n < n1; n++)
+                if (rp[n + 1] > rp[n]) {  // a row's columns ascend
+                    lo = std::min<int64_t>(lo, m->h_bcol[rp[n]]);
+                    hi = std::max<int64_t>(hi, m->h_bcol[rp[n + 1] - 1] + 1);
+                }
+            for (int64_t i = 0; i < n1 - n0; i += 32 / S) {  // the rows of a warp: the first is the longest
+                const int64_t n = n0 + pm[i];
+                slots += 32 * ((rp[n + 1] - rp[n] + S - 1) / S);
+            }
+            s.slots = std::max(s.slots, slots);
+            s.window = std::max(s.window, hi - lo);
+            fits = s.window < 65536;
+        }
+        if (!fits) continue;
+        s.bytes = amr_resident_bytes(m, s);
+        if (s.bytes > kMaxDyn) continue;
+        best = s;
+        if (s.bytes <= prefer) break;
+    }
+    return best;
+}
+
+size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s) {
+    return m->B == 3 ? slice_bytes<3>(s.slots, s.rows, s.window) : slice_bytes<2>(s.slots, s.rows, s.window);
+}
+size_t amr_resident_max_bytes() { return kMaxDyn; }
+
+void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
+                         const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active, const double *b, double *x, double *reac,
+                         AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1, double tol2, int max_iters,
+                         int force_every, cudaStream_t stream) {
+    if (nparts <= 0) return;
+    Args a;
+    a.slices = slices; a.first = first; a.perm = perm; a.list = list; a.active = active; a.nb = m->bstride; a.rp = m->brow_ptr; a.cj = m->bcol;
+    a.K32 = m->K32; a.K64 = m->K64; a.Minv = m->Minv32; a.fm = m->free_mask; a.b = b; a.x = x; a.reac = reac;
+    a.stat = stat; a.t0 = t0; a.t1 = t1; a.tol2 = tol2; a.max_iters = max_iters; a.force_every = force_every;
+    a.kcap = (int)shape.slots; a.wcap = (int)shape.window;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)shape.ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(shape.ctas * nparts));
+    cfg.blockDim = dim3(kT);
+    cfg.dynamicSmemBytes = shape.bytes;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (m->B == 3) AMR_CUDA(cudaLaunchKernelEx(&cfg, k_resident_pcg<3>, a));
+    else AMR_CUDA(cudaLaunchKernelEx(&cfg, k_resident_pcg<2>, a));
+    AMR_COUNT(1);
+}
