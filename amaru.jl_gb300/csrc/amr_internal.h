@@ -254,22 +254,23 @@ struct AmrPartStat {
 };
 struct AmrResidentShape {
     int ctas = 0;  // CTAs of the cluster, 0: the part is not solved this way
+    bool exact = false;                        // with solve_mixed's order of operations
     int64_t slots = 0, rows = 0, window = 0;   // the largest slice's
     size_t bytes = 0;                          // its shared memory
     std::vector<int64_t> bounds;               // the slices' node ranges, ctas + 1 bounds
     std::vector<uint16_t> perm;                // per node, slice by slice: its rows by descending length, stable
 };
-AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer);
+AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer, bool exact);
 size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s);  // of a slice of these sizes
 size_t amr_resident_max_bytes();
 // solves the parts list[0..nparts) (null: part 0) on `stream`: part p's slice bounds at slices[first[p]] (null: 0), the
 // slices' row orders in perm (per node of the model); x
-// (in: prescribed values, initial guess), b, reac node-major FP64; stat per part; t0 / t1 (may be null) the
+// (in: prescribed values, initial guess), b, reac node-major FP64; rows64: 2 x nnodes of scratch (exact shapes); stat per part; t0 / t1 (may be null) the
 // %globaltimer span
 void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
                          const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active, const double *b, double *x, double *reac,
-                         AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1, double tol2, int max_iters,
-                         int force_every, cudaStream_t stream);
+                         double *rows64, AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1,
+                         double tol2, int max_iters, int force_every, cudaStream_t stream);
 // vector helpers (solver.cu)
 double amr_norm_inf(amr_model *m, const double *v, const uint8_t *mask_or_null);
 void amr_eq_to_nm(amr_model *m, const double *d_eq, double *d_nm);  // scatter eq_id-ordered -> node-major (0 elsewhere)

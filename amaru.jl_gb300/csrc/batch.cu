@@ -1081,7 +1081,7 @@ void amr_batch_set(amr_model *m, int64_t nparts, const int64_t *ptr) {
         // the parts that do not fit a cluster's shared memory first, then those that do, by cluster size and, while
         // the largest slices of their blocks, rows and windows fit together, in one group
         std::vector<AmrResidentShape> shape(nparts);
-        for (int64_t i = 0; i < nparts; i++) shape[i] = amr_resident_shape(m, ptr[i], ptr[i + 1], kSliceBatch);
+        for (int64_t i = 0; i < nparts; i++) shape[i] = amr_resident_shape(m, ptr[i], ptr[i + 1], kSliceBatch, false);
         std::stable_sort(order.begin(), order.end(), [&](int64_t x, int64_t y) {
             const int cx = shape[x].ctas ? shape[x].ctas : INT32_MAX, cy = shape[y].ctas ? shape[y].ctas : INT32_MAX;
             return cx > cy;
@@ -1196,7 +1196,7 @@ void launch_pcg(amr_model *m, const PcgArgs &a, int ctas_per_sm) {
         const size_t lane = b->side.empty() ? 0 : g % (b->side.size() + 1);  // 0: the handle's stream
         cudaStream_t st = lane == 0 ? m->stream : b->side[lane - 1];
         if (lane > 0 && g == lane) AMR_CUDA(cudaStreamWaitEvent(st, b->fork, 0));
-        amr_resident_launch(m, q.shape, q.count, b->slices, b->first, b->perm, b->order + q.first, a.active, a.b, a.x, a.reac, a.stat,
+        amr_resident_launch(m, q.shape, q.count, b->slices, b->first, b->perm, b->order + q.first, a.active, a.b, a.x, a.reac, nullptr, a.stat,
                             a.step ? &a.step->t0 : nullptr, a.step ? &a.step->t1 : nullptr, a.tol2, a.max_iters,
                             a.force_every, st);
     }

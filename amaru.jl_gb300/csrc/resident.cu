@@ -12,6 +12,13 @@
 // them the values, without conflicts or shuffles.  8 lanes per row over the rows' own layout took 4.9 times as long
 // (9 430 cycles for 586 rows and 8 568 blocks).
 //
+// Two forms.  For a model alone (Exact) the operations are those of solve_mixed's launch-per-step kernels in solver.cu,
+// in the same order: the eight partial sums of a row and their tree, the rows' products by warps and CTAs of 32, 64
+// and 256 rows, the refresh's FP64 sums over CTAs.  Only an iteration's sums over CTAs are pairs of FP32 numbers
+// instead of FP64: they reach the iteration as alpha and beta rounded to FP32, which 48 bits give as 53 do but for one
+// in some ten million.  So which form a model's size selects shows in its time and hardly ever in a bit of its
+// result.  For a batch's parts, which other CTAs summed anyway, the order is free: one sum per row, one per thread.
+//
 // What else bounds it is the chain of an iteration, two cluster-wide sums (p.q, then r.z and r.r).  So:
 //   * the direction needs no sum of its own: a CTA pushes the z of its rows into the windows of the CTAs that read them,
 //     and after the second sum each forms p = z + beta p over its whole window;
@@ -21,8 +28,8 @@
 //     windows are never written while they may be read;
 //   * nothing in an iteration takes the FP64 pipe (two lanes a clock per SM): the partials of the CTAs, FP32 as in
 //     solver.cu, are added as pairs hi + lo by two-sums (48 bits), and alpha and beta are quotients of such pairs.
-// Measured, three launches per iteration over all SMs before: 26 us an iteration, now 2.7 us (1 613 QUAD8 nodes, 8
-// CTAs); a batch of 64 QUAD8 models of 10 to 60 cells a side 230 ms, now 42 ms.
+// Measured, three launches per iteration over all SMs before: 26 us an iteration, now 3.5 us with Exact and 2.7 us without
+// (1 613 QUAD8 nodes, 8 CTAs); a batch of 64 QUAD8 models of 10 to 60 cells a side 230 ms, now 44 ms.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -40,7 +47,8 @@ constexpr int kT = 512;             // threads of a CTA
 constexpr int kW = kT / 32;
 constexpr int kRowsPerThread = 2;   // rows a thread keeps in registers
 constexpr int kMaxC = 16;           // CTAs of a cluster at most (above 8 where the device allows it)
-constexpr size_t kMaxDyn = 224 * 1024;
+constexpr size_t kMaxDyn = 224 * 1024, kMaxDynExact = 206 * 1024;  // the latter leaves room for the rows' partials
+constexpr int kMaxGroups = kMaxC * kT * kRowsPerThread / 32;        // groups of 32 rows of a part
 
 struct Args {
     const int64_t *slices, *first;   // the parts' slice bounds, and where a part's begin (null: 0)
@@ -56,6 +64,8 @@ struct Args {
     const uint8_t *fm;
     const double *b;
     double *x, *reac;
+    double *rows64;                  // Exact: 2 x nnodes, r.r and r.z of each row at a refresh
+    int64_t nnodes;
     AmrPartStat *stat;
     unsigned long long *t0, *t1;     // null: no timing
     double tol2;
@@ -133,9 +143,81 @@ __device__ __forceinline__ void load_node(const float *p, float *v) {
     }
 }
 
-template <int B>
+// sum of n doubles as solver.cu's grid_sum adds its CTAs' partials: thread j of 256 has partials j, j + 256, .., a
+// shuffle tree per warp, then the warps'; levels and warps that would add zeros left out.  One warp; get(i): partial i.
+template <class F>
+__device__ __forceinline__ double tree_sum(int n, F get) {
+    const int lane = threadIdx.x & 31;
+    double w[8];
+    const int nw = min(8, (n + 31) / 32);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        w[q] = 0.0;
+        if (q < nw) {
+            double v = 0.0;
+            for (int i = 32 * q + lane; i < n; i += 256) v += get(i);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                if (o < n) v += __shfl_xor_sync(0xffffffffu, v, o);
+            w[q] = v;
+        }
+    }
+    return nw == 1 ? w[0] : ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+}
+// One row's product (or this thread's eighth-th of it): the thread's share of the eight sums of k_spmv32v's lanes, which take
+// four blocks each in turn, then the lanes' tree
+template <int B, int S>
+__device__ __forceinline__ void exact_row(const float4 *val4, const float *val1, const uint16_t *cols, int kcap, int e,
+                                          int chunks, const float *pwin, float *q) {
+    constexpr int BB = B * B, A = 8 / S;
+    float acc[A][B];
+#pragma unroll
+    for (int i = 0; i < A; i++)
+#pragma unroll
+        for (int c = 0; c < B; c++) acc[i][c] = 0.0f;
+    for (int t0 = 0; t0 < chunks; t0 += A)
+#pragma unroll
+        for (int i = 0; i < A; i++) {
+            if (t0 + i >= chunks) break;  // (uniform over the warp)
+#pragma unroll
+            for (int u = 0; u < 4; u++, e += 32) {
+                const int j = (int)cols[e] * B;
+                float v[BB], pv[B];
+#pragma unroll
+                for (int w = 0; w < BB / 4; w++) {
+                    const float4 f = val4[w * kcap + e];
+                    v[4 * w] = f.x; v[4 * w + 1] = f.y; v[4 * w + 2] = f.z; v[4 * w + 3] = f.w;
+                }
+                if (BB % 4) v[BB - 1] = val1[e];
+                load_node<B>(pwin + j, pv);
+#pragma unroll
+                for (int c = 0; c < B; c++)
+#pragma unroll
+                    for (int d = B - 1; d >= 0; d--) acc[i][c] = fmaf(v[c * B + d], pv[d], acc[i][c]);
+            }
+        }
+#pragma unroll
+    for (int c = 0; c < B; c++) {
+        if constexpr (S == 1) {
+            q[c] = ((acc[0][c] + acc[4][c]) + (acc[2][c] + acc[6][c])) + ((acc[1][c] + acc[5][c]) + (acc[3][c] + acc[7][c]));
+        } else if constexpr (S == 2) {
+            const float x = (acc[0][c] + acc[2][c]) + (acc[1][c] + acc[3][c]);
+            q[c] = x + __shfl_xor_sync(0xffffffffu, x, 1);
+        } else {
+            float x = acc[0][c] + acc[1][c];
+            x += __shfl_xor_sync(0xffffffffu, x, 2);
+            q[c] = x + __shfl_xor_sync(0xffffffffu, x, 1);
+        }
+    }
+}
+
+template <int B, bool Exact>
 __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
-    constexpr int BB = B * B, G = 8, M = kRowsPerThread;
+    constexpr int BB = B * B, M = kRowsPerThread;
+    constexpr int XR = Exact ? kT * kRowsPerThread : 1, XG = Exact ? kMaxGroups : 1;
+    __shared__ float s_row[2][XR];           // Exact: a value of each row of the slice
+    __shared__ float s_grp[3][XG];           //   the sums of 32 rows: p.q; r.z and r.r
+    __shared__ double s_grpd[2][XG / 2 + 1]; //   the sums of 64 rows at a refresh
     extern __shared__ float dyn[];
     __shared__ float s_warp[2 * kW];
     __shared__ int s_off[M * kW + 1];       // first slot of each 32 rows' (row parts') blocks
@@ -207,9 +289,10 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     for (int m = 0; m < M; m++) {
         const int i = (tid + m * kT) / S;
         row[m] = i < Rn ? (int)a.perm[n0 + i] : -1;
-        const int n = row[m] >= 0 ? (int)(a.rp[n0 + row[m] + 1] - a.rp[n0 + row[m]]) : 0;
+        int n = row[m] >= 0 ? (int)(a.rp[n0 + row[m] + 1] - a.rp[n0 + row[m]]) : 0;
+        if (Exact && n > 0) n = ((int)(a.rp[n0 + row[m]] & 3) + n + 3) / 4;  // runs of four from a multiple of four
         width[m] = __reduce_max_sync(0xffffffffu, (n + S - 1) / S);
-        if (lane == 0) s_off[m * kW + warp + 1] = 32 * width[m];
+        if (lane == 0) s_off[m * kW + warp + 1] = 32 * (Exact ? 4 : 1) * width[m];
     }
     __syncthreads();
     if (tid == 0) {
@@ -222,9 +305,9 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     for (int m = 0; m < M; m++) {
         slot0[m] = s_off[m * kW + warp] + lane;
         const int64_t ks = row[m] >= 0 ? a.rp[n0 + row[m]] : 0, ke = row[m] >= 0 ? a.rp[n0 + row[m] + 1] : 0;
-        for (int t = 0; t < width[m]; t++) {
-            const int64_t k = ks + t * S + sub;
-            const bool in = k < ke;
+        for (int t = 0; t < width[m] * (Exact ? 4 : 1); t++) {
+            const int64_t k = Exact ? (ks & ~int64_t(3)) + 4 * ((t >> 2) * S + sub) + (t & 3) : ks + t * S + sub;
+            const bool in = k >= ks && k < ke;
             float v[BB];
 #pragma unroll
             for (int q = 0; q < BB; q++) v[q] = in ? a.K32[(int64_t)q * a.nb + k] : 0.0f;
@@ -246,6 +329,8 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
         if (lane == 0) atomicAdd(&s_bytes, got);
     }
     for (int i = tid; i < W * B; i += kT) pwin[i] = zwin[i] = 0.0f;
+    if constexpr (Exact)  // (rows without blocks keep their zeros)
+        for (int i = tid; i < XR; i += kT) s_row[0][i] = s_row[1][i] = 0.0f;
     if (sub != 0)  // from here on a row's first thread owns it
 #pragma unroll
         for (int m = 0; m < M; m++) row[m] = -1;
@@ -334,6 +419,40 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             o0 = p;
         }
     };
+    // Exact: sums over 32 rows of the slice's values s_row[0] (s_row[1]), in the order `first` (p.q: lane bits 2, 1, then 16,
+    // 8, 4, as the warps of 4 rows and CTAs of 32 add them) or natural, pushed to every CTA
+    const int64_t P0 = bound[0];
+    const int groups = (int)((bound[C] - P0 + 31) / 32), g0 = (int)((n0 - P0) / 32);
+    auto push_groups = [&](auto two, int set) {
+        constexpr bool two_sums = decltype(two)::value;
+        __syncthreads();
+        for (int g = warp; g * 32 < R; g += kW) {
+            const int i = 32 * g + lane;
+            float t = i < R ? s_row[0][i] : 0.0f;
+            if (two_sums) {
+                const float v1 = i < R ? s_row[1][i] : 0.0f;
+                t = (half ? v1 : t) + __shfl_xor_sync(0xffffffffu, half ? t : v1, 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            } else {
+                t += __shfl_xor_sync(0xffffffffu, t, 2);
+                t += __shfl_xor_sync(0xffffffffu, t, 1);
+                t += __shfl_xor_sync(0xffffffffu, t, 16);
+                t += __shfl_xor_sync(0xffffffffu, t, 8);
+                t += __shfl_xor_sync(0xffffffffu, t, 4);
+            }
+            if (hl < C && (two_sums || half == 0))
+                store_async(cluster_addr(shared_addr(&s_grp[two_sums ? 1 + half : 0][g0 + g]), hl), t, bar_to + set * 8);
+        }
+        if (tid == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(&s_bar[set])),
+                         "r"(two_sums ? s_bytes + 8 * groups : 4 * groups) : "memory");
+        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u);
+        parity ^= 1u << set;
+    };
+    auto lane_pair = [&](Pair p, int o) {
+        return pair_add(p, Pair{__shfl_xor_sync(0xffffffffu, p.h, o), __shfl_xor_sync(0xffffffffu, p.l, o)});
+    };
     // FP64 sums (a refresh only), valid in every thread
     auto cluster_sum64 = [&](double v0, double v1, double &t0, double &t1) {
 #pragma unroll
@@ -375,8 +494,10 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     };
     // the FP64 true residual of the slice from a.x (published by a barrier before): r, z = Minv r, r.z and |r|^2
     auto residual64 = [&](double &rz, double &rr) {
+        constexpr int G = Exact ? 4 : 8;  // lanes per row
         const int gl = tid % G, grp = tid / G;
-        const unsigned gmask = 0xffu << (G * ((tid & 31) / G));
+        const unsigned gmask = ((1u << G) - 1u) << (G * ((tid & 31) / G));
+        if constexpr (Exact) __syncthreads();
         double srr = 0.0, srz = 0.0;
         for (int i = grp; i < R; i += kT / G) {
             const int64_t n = n0 + i;
@@ -396,16 +517,20 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
 #pragma unroll
             for (int o = G / 2; o > 0; o >>= 1)
 #pragma unroll
-                for (int c = 0; c < B; c++) acc[c] += __shfl_down_sync(gmask, acc[c], o, G);
-            if (gl == 0)
+                for (int c = 0; c < B; c++) acc[c] += __shfl_xor_sync(gmask, acc[c], o, G);
+            if (gl == 0) {
+                double row_rr = 0.0;
 #pragma unroll
                 for (int c = 0; c < B; c++) {
                     double res = 0.0;
                     if (a.fm[n * B + c]) res = a.b[n * B + c] - acc[c];
                     else if (a.reac) a.reac[n * B + c] = acc[c];
                     zwin[(own + i) * B + c] = (float)res;
-                    srr = fma(res, res, srr);
+                    row_rr = fma(res, res, row_rr);
                 }
+                if constexpr (Exact) a.rows64[n] = row_rr;
+                else srr += row_rr;
+            }
         }
         __syncthreads();
 #pragma unroll
@@ -415,16 +540,53 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
 #pragma unroll
             for (int c = 0; c < B; c++) rv[m][c] = zwin[(own + i) * B + c];
             float z[B];
+            double row_rz = 0.0;
 #pragma unroll
             for (int c = 0; c < B; c++) {
                 z[c] = 0.0f;
 #pragma unroll
                 for (int d = 0; d < B; d++) z[c] = fmaf(mi[m][c * B + d], rv[m][d], z[c]);
-                srz = fma((double)rv[m][c], (double)z[c], srz);
+                row_rz = fma((double)rv[m][c], (double)z[c], row_rz);
             }
+            if constexpr (Exact) a.rows64[a.nnodes + n0 + i] = row_rz;
+            else srz += row_rz;
             push_z(std::false_type(), m, z);
         }
-        cluster_sum64(srz, srr, rz, rr);
+        if constexpr (Exact) {
+            // sums over 64 rows (the slices are whole groups of 64): row bits 4, 2, 1, then 32, 16, 8
+            __syncthreads();
+            for (int g = warp; g * 64 < R; g += kW)
+#pragma unroll
+                for (int w = 0; w < 2; w++) {
+                    double h[2];
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int i = 64 * g + 32 * u + lane;
+                        // (a row without blocks has no owner, and no r)
+                        const bool in = i < R && a.rp[n0 + i + 1] > a.rp[n0 + i];
+                        h[u] = in ? __ldcg(a.rows64 + (w ? a.nnodes : 0) + n0 + i) : 0.0;
+                        h[u] += __shfl_xor_sync(0xffffffffu, h[u], 4);
+                        h[u] += __shfl_xor_sync(0xffffffffu, h[u], 2);
+                        h[u] += __shfl_xor_sync(0xffffffffu, h[u], 1);
+                    }
+                    double t = h[0] + h[1];
+                    t += __shfl_xor_sync(0xffffffffu, t, 16);
+                    t += __shfl_xor_sync(0xffffffffu, t, 8);
+                    if (lane < C) *cl.map_shared_rank(&s_grpd[w][(n0 - P0) / 64 + g], lane) = t;
+                }
+            barrier();
+            if (warp == 0) {
+                const int n = (groups + 1) / 2;
+                const double trr = tree_sum(n, [&](int i) { return s_grpd[0][i]; });
+                const double trz = tree_sum(n, [&](int i) { return s_grpd[1][i]; });
+                if (lane == 0) { s_dtot[0] = trz; s_dtot[1] = trr; }
+            }
+            __syncthreads();
+            rz = s_dtot[0];
+            rr = s_dtot[1];
+        } else {
+            cluster_sum64(srz, srr, rz, rr);
+        }
     };
 
     double rz64, rr_true;
@@ -432,7 +594,13 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     const double bnorm2 = rr_true;
     const float stop_rr = (float)(0.0625 * a.tol2 * bnorm2);
     Pair gam = split(rz64);
-    float thr = fmaxf(stop_rr, (float)(1e-2 * rr_true)), beta = 0.0f;
+    // the next refresh: after a 10x drop, or, where that would end within the tolerance, at a quarter of the
+    // tolerance (a refresh just inside it would return the solution with up to four times the residual; not with
+    // Exact, which refreshes where solve_mixed does)
+    auto threshold = [&]() {
+        return Exact || 1e-2 * rr_true > a.tol2 * bnorm2 ? fmaxf(stop_rr, (float)(1e-2 * rr_true)) : stop_rr;
+    };
+    float thr = threshold(), beta = 0.0f;
     int iters = 0, refreshes = 0, status = 0, since = 0;
     bool done = !(bnorm2 > 0.0) || rr_true <= a.tol2 * bnorm2;
     if (isnan(rr_true)) { status = AMR_ENOCONV; done = true; }
@@ -449,6 +617,17 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
 #pragma unroll
             for (int c = 0; c < B; c++) q[m][c] = 0.0f;
             int e = slot0[m];
+            if constexpr (Exact) {  // (S is uniform)
+                if (S == 1) exact_row<B, 1>(val4, val1, cols, a.kcap, e, width[m], pwin, q[m]);
+                else if (S == 2) exact_row<B, 2>(val4, val1, cols, a.kcap, e, width[m], pwin, q[m]);
+                else exact_row<B, 4>(val4, val1, cols, a.kcap, e, width[m], pwin, q[m]);
+                if (row[m] >= 0) {
+                    float d = 0.0f;
+#pragma unroll
+                    for (int c = 0; c < B; c++) d = fmaf(pwin[(own + row[m]) * B + c], q[m][c], d);
+                    s_row[0][row[m]] = d;
+                }
+            } else {
 #pragma unroll 4
             for (int t = 0; t < width[m]; t++, e += 32) {
                 const int j = (int)cols[e] * B;
@@ -474,9 +653,18 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             if (row[m] >= 0)
 #pragma unroll
                 for (int c = 0; c < B; c++) dot = fmaf(pwin[(own + row[m]) * B + c], q[m][c], dot);
+            }
         }
         Pair pq, t2[2];
-        cluster_sum(std::false_type(), 0, dot, 0.0f, pq, pq);
+        if constexpr (Exact) {
+            push_groups(std::false_type(), 0);
+            pq = Pair{0.0f, 0.0f};
+            for (int i = lane; i < groups; i += 32) pq = pair_add(pq, Pair{s_grp[0][i], 0.0f});
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) pq = lane_pair(pq, o);
+        } else {
+            cluster_sum(std::false_type(), 0, dot, 0.0f, pq, pq);
+        }
         if (timeout) { status = AMR_ETIMEOUT; break; }
         if (!(pq.h > 0.0f)) { status = AMR_ENOCONV; break; }
         const float alpha = pair_div(gam, pq);
@@ -492,6 +680,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
                 rv[m][c] = fmaf(-alpha, q[m][c], rv[m][c]);
             }
             float z[B];
+            if (Exact) v0 = v1 = 0.0f;
 #pragma unroll
             for (int c = 0; c < B; c++) {
                 z[c] = 0.0f;
@@ -501,13 +690,35 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
                 v1 = fmaf(rv[m][c], rv[m][c], v1);
             }
             push_z(std::true_type(), m, z);
+            if constexpr (Exact) {
+                s_row[0][i] = v0;
+                s_row[1][i] = v1;
+            }
         }
-        cluster_sum(std::true_type(), 1, v0, v1, t2[0], t2[1]);
+        if constexpr (Exact) {
+            push_groups(std::true_type(), 1);
+            // CTAs of 256 rows: eight warps' sums by bits 4, 2, 1; then over the CTAs
+            t2[0] = t2[1] = Pair{0.0f, 0.0f};
+            for (int i0 = 0; i0 < groups; i0 += 32)
+#pragma unroll
+                for (int w = 0; w < 2; w++) {
+                    float t = i0 + lane < groups ? s_grp[1 + w][i0 + lane] : 0.0f;
+                    t += __shfl_xor_sync(0xffffffffu, t, 4);
+                    t += __shfl_xor_sync(0xffffffffu, t, 2);
+                    t += __shfl_xor_sync(0xffffffffu, t, 1);
+                    t2[w] = pair_add(t2[w], Pair{t, 0.0f});
+                }
+#pragma unroll
+            for (int w = 0; w < 2; w++) t2[w] = lane_pair(lane_pair(t2[w], 16), 8);
+        } else {
+            cluster_sum(std::true_type(), 1, v0, v1, t2[0], t2[1]);
+        }
         if (timeout) { status = AMR_ETIMEOUT; break; }
         beta = pair_div(t2[0], gam);
         gam = t2[0];
         iters++;
         since++;
+        if (Exact && iters >= a.max_iters) { status = AMR_ENOCONV; break; }
         if (!(t2[1].h > thr) || since >= a.force_every) {
             // refresh: fold the FP32 correction into the FP64 solution and recompute the true residual
 #pragma unroll
@@ -525,7 +736,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             barrier();
             residual64(rz64, rr_true);
             gam = split(rz64);
-            thr = fmaxf(stop_rr, (float)(1e-2 * rr_true));
+            thr = threshold();
             refreshes++;
             since = 0;
             if (isnan(rr_true)) { status = AMR_ENOCONV; break; }
@@ -574,10 +785,12 @@ int device_cluster() {
     std::lock_guard<std::mutex> lk(mu);
     if (found[dev]) return found[dev] < 0 ? 0 : found[dev];
     int best = -1;
-    const void *kernels[2] = {(const void *)k_resident_pcg<2>, (const void *)k_resident_pcg<3>};
+    const void *kernels[4] = {(const void *)k_resident_pcg<2, false>, (const void *)k_resident_pcg<3, false>,
+                              (const void *)k_resident_pcg<2, true>, (const void *)k_resident_pcg<3, true>};
     bool ok = true, wide = true;
     for (const void *k : kernels) {
-        ok &= cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn) == cudaSuccess;
+        ok &= cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(k == kernels[2] || k == kernels[3] ? kMaxDynExact : kMaxDyn)) == cudaSuccess;
         wide &= cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     }
     if (ok)
@@ -590,12 +803,15 @@ int device_cluster() {
             at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
             cfg.gridDim = dim3((unsigned)c);
             cfg.blockDim = dim3(kT);
-            cfg.dynamicSmemBytes = kMaxDyn;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            int n2 = 0, n3 = 0;
-            if (cudaOccupancyMaxActiveClusters(&n2, k_resident_pcg<2>, &cfg) == cudaSuccess &&
-                cudaOccupancyMaxActiveClusters(&n3, k_resident_pcg<3>, &cfg) == cudaSuccess && n2 > 0 && n3 > 0) {
+            bool fits = true;
+            for (const void *k : kernels) {
+                int n = 0;
+                cfg.dynamicSmemBytes = k == kernels[2] || k == kernels[3] ? kMaxDynExact : kMaxDyn;
+                fits &= cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0;
+            }
+            if (fits) {
                 best = c;
                 break;
             }
@@ -609,7 +825,7 @@ int device_cluster() {
 
 // The cluster size that solves nodes [P0, P1), and the largest slice: the smallest whose slices stay within `prefer`
 // bytes of shared memory, else the largest the device takes if its slices fit at all; 0: none.
-AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer) {
+AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer, bool exact) {
     AmrResidentShape best;
     const int most = device_cluster();
     const int64_t len = P1 - P0;
@@ -624,7 +840,15 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
                           : r == C ? P1
                                    : std::lower_bound(rp.begin() + P0, rp.begin() + P1, rp[P0] + (rp[P1] - rp[P0]) * r / C) -
                                          rp.begin();
+        if (exact)  // whole groups of 64 rows
+            for (int r = 1; r < C; r++) s.bounds[r] = std::min(P1, P0 + (s.bounds[r] - P0 + 32) / 64 * 64);
+        s.exact = exact;
         s.perm.resize(len);
+        // a row's blocks, or with `exact` its runs of four blocks from a multiple of four
+        auto width = [&](int64_t n) {
+            const int64_t l = rp[n + 1] - rp[n];
+            return exact && l > 0 ? ((rp[n] & 3) + l + 3) / 4 : l;
+        };
         int64_t most_rows = 0;
         for (int r = 0; r < C; r++) {
             const int64_t n0 = s.bounds[r], n1 = s.bounds[r + 1];
@@ -632,14 +856,14 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
             uint16_t *pm = s.perm.data() + (n0 - P0);
             for (int64_t i = 0; i < n1 - n0; i++) pm[i] = (uint16_t)i;
             std::stable_sort(pm, pm + (n1 - n0), [&](uint16_t x, uint16_t y) {
-                return rp[n0 + x + 1] - rp[n0 + x] > rp[n0 + y + 1] - rp[n0 + y];
+                return width(n0 + x) > width(n0 + y);
             });
             int64_t used = 0;
             while (used < n1 - n0 && rp[n0 + pm[used] + 1] > rp[n0 + pm[used]]) used++;
             most_rows = std::max(most_rows, used);
             s.rows = std::max(s.rows, n1 - n0);
         }
-        if (s.rows > 65535 || most_rows > kT * kRowsPerThread) continue;
+        if (s.rows > (exact ? kT * kRowsPerThread : 65535) || most_rows > kT * kRowsPerThread) continue;
         const int S = threads_per_row(most_rows);
         bool fits = true;
         for (int r = 0; r < C && fits; r++) {
@@ -652,8 +876,7 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
                     hi = std::max<int64_t>(hi, m->h_bcol[rp[n + 1] - 1] + 1);
                 }
             for (int64_t i = 0; i < n1 - n0; i += 32 / S) {  // the rows of a warp: the first is the longest
-                const int64_t n = n0 + pm[i];
-                slots += 32 * ((rp[n + 1] - rp[n] + S - 1) / S);
+                slots += 32 * (exact ? 4 : 1) * ((width(n0 + pm[i]) + S - 1) / S);
             }
             s.slots = std::max(s.slots, slots);
             s.window = std::max(s.window, hi - lo);
@@ -661,7 +884,7 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
         }
         if (!fits) continue;
         s.bytes = amr_resident_bytes(m, s);
-        if (s.bytes > kMaxDyn) continue;
+        if (s.bytes > (exact ? kMaxDynExact : kMaxDyn)) continue;
         best = s;
         if (s.bytes <= prefer) break;
     }
@@ -675,13 +898,13 @@ size_t amr_resident_max_bytes() { return kMaxDyn; }
 
 void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
                          const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active, const double *b, double *x, double *reac,
-                         AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1, double tol2, int max_iters,
-                         int force_every, cudaStream_t stream) {
+                         double *rows64, AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1,
+                         double tol2, int max_iters, int force_every, cudaStream_t stream) {
     if (nparts <= 0) return;
     Args a;
     a.slices = slices; a.first = first; a.perm = perm; a.list = list; a.active = active; a.nb = m->bstride; a.rp = m->brow_ptr; a.cj = m->bcol;
     a.K32 = m->K32; a.K64 = m->K64; a.Minv = m->Minv32; a.fm = m->free_mask; a.b = b; a.x = x; a.reac = reac;
-    a.stat = stat; a.t0 = t0; a.t1 = t1; a.tol2 = tol2; a.max_iters = max_iters; a.force_every = force_every;
+    a.rows64 = rows64; a.nnodes = m->nnodes; a.stat = stat; a.t0 = t0; a.t1 = t1; a.tol2 = tol2; a.max_iters = max_iters; a.force_every = force_every;
     a.kcap = (int)shape.slots; a.wcap = (int)shape.window;
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[1];
@@ -694,7 +917,8 @@ void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t np
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (m->B == 3) AMR_CUDA(cudaLaunchKernelEx(&cfg, k_resident_pcg<3>, a));
-    else AMR_CUDA(cudaLaunchKernelEx(&cfg, k_resident_pcg<2>, a));
+    auto kernel = m->B == 3 ? (shape.exact ? k_resident_pcg<3, true> : k_resident_pcg<3, false>)
+                            : (shape.exact ? k_resident_pcg<2, true> : k_resident_pcg<2, false>);
+    AMR_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
     AMR_COUNT(1);
 }

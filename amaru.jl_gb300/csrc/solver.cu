@@ -672,6 +672,7 @@ struct AmrSolveWork {
     AmrResidentShape shape;
     int64_t *slices = nullptr;
     uint16_t *perm = nullptr;
+    double *rows64 = nullptr;
     AmrPartStat *stat = nullptr, *h_stat = nullptr;  // (h_stat pinned)
     // all-FP64 comparators: Krylov vectors (allocated on their first use)
     double *r64 = nullptr, *z64 = nullptr, *p64 = nullptr, *q64 = nullptr;
@@ -715,7 +716,7 @@ void amr_solver_free(amr_model *m) {
     amr_free(w->partials); amr_free(w->ctl);
     amr_pinned_free(w->h_ctl);
     amr_free(w->r64); amr_free(w->z64); amr_free(w->p64); amr_free(w->q64);
-    amr_free(w->slices); amr_free(w->perm); amr_free(w->stat);
+    amr_free(w->slices); amr_free(w->perm); amr_free(w->rows64); amr_free(w->stat);
     amr_pinned_free(w->h_stat);
     delete w;
     m->sw = nullptr;
@@ -747,21 +748,22 @@ static void launch_pupdate32(amr_model *m, AmrSolveWork *w) {
 
 // Shared memory a CTA's slice should stay within when a cluster of fewer CTAs would also do, for a model alone: fewer
 // CTAs mean shorter sums, smaller slices a shorter product.  An elastoplastic stage of 1 613 QUAD8 nodes (14 000
-// iterations) took 38.6 ms with 100 KB and 42.8 ms with 48 KB, a stage of 525 HEX8 nodes 2.6 and 2.8 ms, one of 112
-// nodes 2.1 and 2.0 ms; with all of the shared memory the first took twice as long.
+// iterations) took 51.0 ms with 100 KB, 54.5 ms with 48 KB and 57.9 ms with all 206 KB; a stage of 525 HEX8 nodes 3.0 ms
+// with 24 to 100 KB and 3.2 ms with 206 KB.
 constexpr size_t kSliceSingle = 100 * 1024;
 
 // solve_mixed in one launch, where the model's matrix fits the shared memory of a cluster; false: it does not
 static bool solve_resident(amr_model *m, AmrSolveWork *w, double *x, const double *b, double *reac,
                            const amr_solve_opts &o, AmrSolveResult &res) {
     if (!w->shape_known) {
-        w->shape = amr_resident_shape(m, 0, m->nnodes, kSliceSingle);
+        w->shape = amr_resident_shape(m, 0, m->nnodes, kSliceSingle, true);
         w->shape_known = true;
         if (w->shape.ctas) {
             const std::vector<int64_t> &bounds = w->shape.bounds;
             amr_alloc(&w->slices, bounds.size());
             amr_alloc(&w->perm, w->shape.perm.size());
             amr_h2d(m, w->perm, w->shape.perm.data(), w->shape.perm.size() * sizeof(uint16_t));
+            amr_alloc(&w->rows64, 2 * m->nnodes);
             amr_alloc(&w->stat, 1);
             w->h_stat = (AmrPartStat *)amr_pinned_alloc(sizeof(AmrPartStat));
             amr_h2d(m, w->slices, bounds.data(), bounds.size() * sizeof(int64_t));
@@ -771,8 +773,8 @@ static bool solve_resident(amr_model *m, AmrSolveWork *w, double *x, const doubl
     const int every = o.refine_every > 0 ? o.refine_every : 32;
     cudaStream_t s = m->stream;
     AMR_CUDA(cudaEventRecord(m->ev0, s));
-    amr_resident_launch(m, w->shape, 1, w->slices, nullptr, w->perm, nullptr, nullptr, b, x, reac, w->stat, nullptr, nullptr,
-                        o.rtol * o.rtol, o.max_iters, 16 * every, s);
+    amr_resident_launch(m, w->shape, 1, w->slices, nullptr, w->perm, nullptr, nullptr, b, x, reac, w->rows64, w->stat, nullptr,
+                        nullptr, o.rtol * o.rtol, o.max_iters, 16 * every, s);
     AMR_CUDA(cudaEventRecord(m->ev1, s));
     AMR_CUDA(cudaMemcpyAsync(w->h_stat, w->stat, sizeof(AmrPartStat), cudaMemcpyDeviceToHost, s));
     AMR_CUDA(cudaStreamSynchronize(s));
