@@ -230,6 +230,9 @@ void amr_stiffness(amr_model *m);                       // Kel + gather into K64
 void amr_stiffness_elements(amr_model *m);              // Kel only (element kernels)
 void amr_combine_K(amr_model *m, double a1, const double *Ks, double a2);  // K64 = a1 Ks + a2 K64, K32, Minv
 void amr_mass(amr_model *m);                            // mount_M: element masses gathered into M64 / Mkeep
+// K or M as CSC over the equation numbers: the entries that keep marks, rows ascending (csc.cu); colptr null: nnz only
+void amr_export_csc(amr_model *m, int64_t *nnz, int64_t *colptr, int64_t *rowval, double *nzval, const uint16_t *keep,
+                    const double *vals);
 // K64 = Ks + s1 M + s2 (alpha M + beta Ks) (Ks may be null: K = 0), then K32, Minv
 void amr_dyn_combine(amr_model *m, const double *Ks, double s1, double s2, double alpha, double beta);
 void amr_update_elements(amr_model *m, const double *dU_nm, double *dFin_nm);  // node-major device vectors

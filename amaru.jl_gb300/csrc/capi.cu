@@ -552,72 +552,10 @@ int amr_assemble_K(amr_model *m) {
     });
 }
 
-// Host export of K in the reference layout (CSC over eq_id order, eps drop rule)
-// CSC of the block matrix vals (SoA, K's pattern) with the scalar entries its keep bits mark
-static void export_csc(amr_model *m, int64_t *nnz_out, int64_t *colptr, int64_t *rowval, double *nzval,
-                       const uint16_t *d_keep, const double *d_vals) {
-    int B = m->B, BB = m->BB;
-    std::vector<uint16_t> keep(m->nblocks);
-    amr_d2h(m, keep.data(), d_keep, m->nblocks * sizeof(uint16_t));
-    std::vector<double> K;
-    if (nzval) {
-        K.resize((size_t)m->bstride * BB);
-        amr_d2h(m, K.data(), d_vals, K.size() * sizeof(double));
-    }
-    const std::vector<int64_t> &eq = m->h_eq_id;
-    // count per column (= per row of the symmetric pattern walk)
-    std::vector<int64_t> cnt(m->ndofs + 1, 0);
-    for (int64_t n = 0; n < m->nnodes; n++)
-        for (int64_t k = m->h_brow_ptr[n]; k < m->h_brow_ptr[n + 1]; k++) {
-            int64_t j = m->h_bcol[k];
-            for (int c = 0; c < B; c++) {
-                int64_t r = eq[3 * n + c];
-                if (r < 0) continue;
-                for (int d = 0; d < B; d++) {
-                    int64_t col = eq[3 * j + d];
-                    if (col < 0 || !(keep[k] >> (c * B + d) & 1)) continue;
-                    cnt[col + 1]++;
-                }
-            }
-        }
-    for (int64_t i = 0; i < m->ndofs; i++) cnt[i + 1] += cnt[i];
-    *nnz_out = cnt[m->ndofs];
-    if (!colptr) return;
-    std::vector<int64_t> pos(cnt.begin(), cnt.end() - 1);
-    for (int64_t n = 0; n < m->nnodes; n++)
-        for (int64_t k = m->h_brow_ptr[n]; k < m->h_brow_ptr[n + 1]; k++) {
-            int64_t j = m->h_bcol[k];
-            for (int c = 0; c < B; c++) {
-                int64_t r = eq[3 * n + c];
-                if (r < 0) continue;
-                for (int d = 0; d < B; d++) {
-                    int64_t col = eq[3 * j + d];
-                    if (col < 0 || !(keep[k] >> (c * B + d) & 1)) continue;
-                    int64_t p = pos[col]++;
-                    rowval[p] = r;
-                    if (nzval) nzval[p] = K[(size_t)(c * B + d) * m->bstride + k];
-                }
-            }
-        }
-    for (int64_t i = 0; i <= m->ndofs; i++) colptr[i] = cnt[i];
-    // sort rows within each column
-    std::vector<std::pair<int64_t, double>> tmp;
-    for (int64_t col = 0; col < m->ndofs; col++) {
-        int64_t a = cnt[col], b = cnt[col + 1];
-        tmp.resize(b - a);
-        for (int64_t p = a; p < b; p++) tmp[p - a] = {rowval[p], nzval ? nzval[p] : 0.0};
-        std::sort(tmp.begin(), tmp.end(), [](const auto &x, const auto &y) { return x.first < y.first; });
-        for (int64_t p = a; p < b; p++) {
-            rowval[p] = tmp[p - a].first;
-            if (nzval) nzval[p] = tmp[p - a].second;
-        }
-    }
-}
-
 int amr_get_K_nnz(amr_model *m, int64_t *nnz) {
     return guarded(m, [&] {
         if (!m->K_valid) throw AmrError(AMR_EINVAL, "K has not been assembled");
-        export_csc(m, nnz, nullptr, nullptr, nullptr, m->keep, m->K64);
+        amr_export_csc(m, nnz, nullptr, nullptr, nullptr, m->keep, m->K64);
         return AMR_OK;
     });
 }
@@ -626,7 +564,7 @@ int amr_get_K_csc(amr_model *m, int64_t *colptr, int64_t *rowval, double *nzval)
     return guarded(m, [&] {
         int64_t nnz = 0;
         if (!m->K_valid) throw AmrError(AMR_EINVAL, "K has not been assembled");
-        export_csc(m, &nnz, colptr, rowval, nzval, m->keep, m->K64);
+        amr_export_csc(m, &nnz, colptr, rowval, nzval, m->keep, m->K64);
         return AMR_OK;
     });
 }
@@ -661,7 +599,7 @@ int amr_get_M_csc(amr_model *m, int64_t *nnz, int64_t *colptr, int64_t *rowval, 
     return guarded(m, [&] {
         if (!nnz) throw AmrError(AMR_EINVAL, "null argument");
         if (!m->M64) throw AmrError(AMR_EINVAL, "M has not been assembled");
-        export_csc(m, nnz, colptr, rowval, nzval, m->Mkeep, m->M64);
+        amr_export_csc(m, nnz, colptr, rowval, nzval, m->Mkeep, m->M64);
         return AMR_OK;
     });
 }

@@ -23,6 +23,8 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <mutex>
+#include <set>
 #include <type_traits>
 #include <vector>
 
@@ -765,37 +767,50 @@ __global__ void __launch_bounds__(256, stiff_min_blocks<DIM, NEN>()) stiffness_k
 #define RSUB __dsub_rn
 #define RDIV __ddiv_rn
 
-// B[l][(b,d)] of setB (mech-solid.jl:82-121) from g = dN/dX of node b; hb = N_b / r, the hoop row of an
-// axisymmetric analysis (0 otherwise)
+// The nonzero rows of column (b, d) of B (setB, mech-solid.jl:82-121), ascending: kRefTerms of them, row(q) and value(q).
+// g = dN/dX of node b, gs = g / sqrt(2) of the shear rows, hb = N_b / r, the hoop row of an axisymmetric analysis.
+// Where a sum of the reference runs over all six rows, the products with B's zeros are left out: they add +-0 to
+// sums that start at +0, which changes no bit of them.
+constexpr int kRefTerms = 3;
 template <int DIM>
-__device__ __forceinline__ double ref_B(int l, int d, const double *g, double hb) {
-    if (DIM == 3) {
-        switch (l) {
-        case 0: return d == 0 ? g[0] : 0.0;
-        case 1: return d == 1 ? g[1] : 0.0;
-        case 2: return d == 2 ? g[2] : 0.0;
-        case 3: return d == 1 ? RDIV(g[2], SQ2) : (d == 2 ? RDIV(g[1], SQ2) : 0.0);
-        case 4: return d == 0 ? RDIV(g[2], SQ2) : (d == 2 ? RDIV(g[0], SQ2) : 0.0);
-        default: return d == 0 ? RDIV(g[1], SQ2) : (d == 1 ? RDIV(g[0], SQ2) : 0.0);
-        }
-    }
-    switch (l) {
-    case 0: return d == 0 ? g[0] : 0.0;
-    case 1: return d == 1 ? g[1] : 0.0;
-    case 2: return d == 0 ? hb : 0.0;
-    case 5: return d == 0 ? RDIV(g[1], SQ2) : RDIV(g[0], SQ2);
-    default: return 0.0;
-    }
+__device__ __forceinline__ int ref_row(int q, int d) {
+    if (DIM == 3) return q == 0 ? d : q == 1 ? (d == 0 ? 4 : 3) : (d == 2 ? 4 : 5);
+    return q == 0 ? d : q == 1 ? 2 : 5;
+}
+template <int DIM>
+__device__ __forceinline__ double ref_value(int q, int d, const double *g, const double *gs, double hb) {
+    if (DIM == 3) return q == 0 ? g[d] : q == 1 ? gs[d == 2 ? 1 : 2] : gs[d == 0 ? 1 : 0];
+    return q == 0 ? g[d] : q == 1 ? (d == 0 ? hb : 0.0) : gs[d == 0 ? 1 : 0];
+}
+
+// One element per CTA.  The geometry of all integration points first, a thread per entry: Jacobians, inverses (a division
+// per thread), dN/dX and its shear form g / sqrt(2) (once, not at each use in a product), D; then D B for kRefChunk
+// points at a time and the sums of B' (D B).  The FP64 pipe bounds it: 7 operations per entry and point, 0.3 ms for
+// 4 901 HEX8 elements.  With a thread's serial geometry per point and B formed with its divisions inside the sums it
+// took 4.1 ms there; now the whole assembly, gather and synchronisation included, takes 0.52 ms.
+constexpr int kRefChunk = 8;
+template <int DIM, int NEN>
+__host__ __device__ constexpr int ref_doubles(int nip) {  // shared memory of the CTA, in doubles
+    return NEN * DIM + nip * (2 * NEN * DIM + 36 + 2 * DIM * DIM + 1 + NEN) + (nip < kRefChunk ? nip : kRefChunk) * 6 * NEN * DIM;
 }
 
 template <int DIM, int NEN>
 __global__ void __launch_bounds__(256) stiffness_ref_kernel(ModelArgs M, GroupArgs G, double *Kel, const double *st,
                                                             int32_t *status) {
-    constexpr int ND = NEN * DIM;
+    constexpr int ND = NEN * DIM, JJ = DIM * DIM;
     constexpr int NE = (ND * ND + 255) / 256;
-    __shared__ double sC[ND], sG[ND], sD[36], sDB[6 * ND], sIJ[9], sCoef, sH[NEN];
+    extern __shared__ double sm[];
     const int64_t e = G.first + blockIdx.x;
     const int nip = G.nip;
+    double *sC = sm;                  // ND
+    double *sG = sC + ND;             // nip x ND: dN/dX
+    double *sS = sG + nip * ND;       // nip x ND: dN/dX / sqrt(2)
+    double *sD = sS + nip * ND;       // nip x 36
+    double *sJ = sD + nip * 36;       // nip x JJ
+    double *sIJ = sJ + nip * JJ;      // nip x JJ
+    double *sCoef = sIJ + nip * JJ;   // nip
+    double *sH = sCoef + nip;         // nip x NEN
+    double *sDB = sH + nip * NEN;     // chunk x 6 x ND
     const bool ps = (M.stressmodel == AMR_PLANESTRESS);
     const bool axi = DIM == 2 && M.stressmodel == AMR_AXISYMMETRIC;
     for (int t = threadIdx.x; t < ND; t += blockDim.x) {
@@ -807,35 +822,33 @@ __global__ void __launch_bounds__(256) stiffness_ref_kernel(ModelArgs M, GroupAr
     for (int q = 0; q < NE; q++) acc[q] = 0.0;
     const double *par = M.mat_par + 8 * e;
     __syncthreads();
-    for (int ip = 0; ip < nip; ip++) {
+    for (int t = threadIdx.x; t < nip * JJ; t += blockDim.x) {  // J = C' dN/dR
+        const int ip = t / JJ, a = t % JJ / DIM, b = t % DIM;
         const double *dNdR = G.tab + ip * ND;
-        if (threadIdx.x == 0) {
-            double J[9];
-            for (int a = 0; a < DIM; a++)
-                for (int b = 0; b < DIM; b++) {
-                    double s = 0.0;
-                    for (int i = 0; i < NEN; i++) s = RADD(s, RMUL(sC[i * DIM + a], dNdR[i * DIM + b]));
-                    J[a * DIM + b] = s;
-                }
-            double det;
-            if (DIM == 2) {
-                det = RSUB(RMUL(J[0], J[3]), RMUL(J[1], J[2]));
-                sIJ[0] = RDIV(J[3], det); sIJ[1] = RDIV(-J[1], det); sIJ[2] = RDIV(-J[2], det); sIJ[3] = RDIV(J[0], det);
-            } else {
-                double c0 = RSUB(RMUL(J[4], J[8]), RMUL(J[5], J[7]));
-                double c1 = RSUB(RMUL(J[3], J[8]), RMUL(J[5], J[6]));
-                double c2 = RSUB(RMUL(J[3], J[7]), RMUL(J[4], J[6]));
-                det = RADD(RSUB(RMUL(J[0], c0), RMUL(J[1], c1)), RMUL(J[2], c2));
-                sIJ[0] = RDIV(c0, det);
-                sIJ[1] = RDIV(RSUB(RMUL(J[2], J[7]), RMUL(J[1], J[8])), det);
-                sIJ[2] = RDIV(RSUB(RMUL(J[1], J[5]), RMUL(J[2], J[4])), det);
-                sIJ[3] = RDIV(RSUB(RMUL(J[5], J[6]), RMUL(J[3], J[8])), det);
-                sIJ[4] = RDIV(RSUB(RMUL(J[0], J[8]), RMUL(J[2], J[6])), det);
-                sIJ[5] = RDIV(RSUB(RMUL(J[2], J[3]), RMUL(J[0], J[5])), det);
-                sIJ[6] = RDIV(RSUB(RMUL(J[3], J[7]), RMUL(J[4], J[6])), det);
-                sIJ[7] = RDIV(RSUB(RMUL(J[1], J[6]), RMUL(J[0], J[7])), det);
-                sIJ[8] = RDIV(RSUB(RMUL(J[0], J[4]), RMUL(J[1], J[3])), det);
-            }
+        double s = 0.0;
+        for (int i = 0; i < NEN; i++) s = RADD(s, RMUL(sC[i * DIM + a], dNdR[i * DIM + b]));
+        sJ[t] = s;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nip * JJ; t += blockDim.x) {  // inv(J) by cofactors; the determinant by each thread
+        const int ip = t / JJ, q = t % JJ;
+        const double *J = sJ + ip * JJ;
+        double det, num;
+        if (DIM == 2) {
+            det = RSUB(RMUL(J[0], J[3]), RMUL(J[1], J[2]));
+            num = q == 0 ? J[3] : q == 1 ? -J[1] : q == 2 ? -J[2] : J[0];
+        } else {
+            const double c0 = RSUB(RMUL(J[4], J[8]), RMUL(J[5], J[7]));
+            const double c1 = RSUB(RMUL(J[3], J[8]), RMUL(J[5], J[6]));
+            const double c2 = RSUB(RMUL(J[3], J[7]), RMUL(J[4], J[6]));
+            det = RADD(RSUB(RMUL(J[0], c0), RMUL(J[1], c1)), RMUL(J[2], c2));
+            // entry (r, c) of the inverse: cofactor (c, r), as a difference of two products
+            const int r = q / 3, c = q % 3;
+            const int r1 = (c + 1) % 3, r2 = (c + 2) % 3, c1i = (r + 1) % 3, c2i = (r + 2) % 3;
+            num = RSUB(RMUL(J[r1 * 3 + c1i], J[r2 * 3 + c2i]), RMUL(J[r1 * 3 + c2i], J[r2 * 3 + c1i]));
+        }
+        sIJ[t] = RDIV(num, det);
+        if (q == 0) {
             if (!(det > 0.0)) set_status(status, AMR_ENEGJAC, e);
             double th = M.thickness;
             if (axi) {  // r = ip.coord.x, th = 2 pi r (mech-solid.jl:143), h = N / r
@@ -843,26 +856,31 @@ __global__ void __launch_bounds__(256) stiffness_ref_kernel(ModelArgs M, GroupAr
                 double r = 0.0;
                 for (int i = 0; i < NEN; i++) r = RADD(r, RMUL(sC[i * DIM], N[i]));
                 th = RMUL(2 * M_PI, r);
-                for (int i = 0; i < NEN; i++) sH[i] = RDIV(N[i], r);
+                for (int i = 0; i < NEN; i++) sH[ip * NEN + i] = RDIV(N[i], r);
             } else {
-                for (int i = 0; i < NEN; i++) sH[i] = 0.0;
+                for (int i = 0; i < NEN; i++) sH[ip * NEN + i] = 0.0;
             }
-            sCoef = RMUL(RMUL(det, G.tab[nip * ND + ip]), th);
-            // D: calcDe (linear-elastic.jl:98-119), plastic part as De - gamma m m^T
-            double E = par[0], nu = par[1];
-            for (int q = 0; q < 36; q++) sD[q] = 0.0;
-            if (ps) {
-                double c = RDIV(E, RSUB(1.0, RMUL(nu, nu)));
-                sD[0] = c; sD[1] = RMUL(c, nu); sD[6] = RMUL(c, nu); sD[7] = c;
-                double sh = RMUL(c, RSUB(1.0, nu));
-                sD[21] = sh; sD[28] = sh; sD[35] = sh;
-            } else {
-                double c = RDIV(E, RMUL(RADD(1.0, nu), RSUB(1.0, RMUL(2.0, nu))));
-                for (int i = 0; i < 3; i++)
-                    for (int j = 0; j < 3; j++) sD[6 * i + j] = (i == j) ? RMUL(c, RSUB(1.0, nu)) : RMUL(c, nu);
-                double sh = RMUL(c, RSUB(1.0, RMUL(2.0, nu)));
-                sD[21] = sh; sD[28] = sh; sD[35] = sh;
-            }
+            sCoef[ip] = RMUL(RMUL(det, G.tab[nip * ND + ip]), th);
+        }
+    }
+    // D: calcDe (linear-elastic.jl:98-119), plastic part as De - gamma m m'; the last threads, which have least to do above
+    for (int ip = blockDim.x - 1 - threadIdx.x; ip < nip; ip += blockDim.x) {
+        double *D = sD + ip * 36;
+        const double E = par[0], nu = par[1];
+        for (int q = 0; q < 36; q++) D[q] = 0.0;
+        if (ps) {
+            double c = RDIV(E, RSUB(1.0, RMUL(nu, nu)));
+            D[0] = c; D[1] = RMUL(c, nu); D[6] = RMUL(c, nu); D[7] = c;
+            double sh = RMUL(c, RSUB(1.0, nu));
+            D[21] = sh; D[28] = sh; D[35] = sh;
+        } else {
+            double c = RDIV(E, RMUL(RADD(1.0, nu), RSUB(1.0, RMUL(2.0, nu))));
+            for (int i = 0; i < 3; i++)
+                for (int j = 0; j < 3; j++) D[6 * i + j] = (i == j) ? RMUL(c, RSUB(1.0, nu)) : RMUL(c, nu);
+            double sh = RMUL(c, RSUB(1.0, RMUL(2.0, nu)));
+            D[21] = sh; D[28] = sh; D[35] = sh;
+        }
+        if (M.mat_type[e] != AMR_LINEAR_ELASTIC) {
             int64_t gi = M.ip_ptr[e] + ip;
             double sig[6], m[6], lam, mu;
             for (int i = 0; i < 6; i++) sig[i] = st[i * M.nip_total + gi];
@@ -871,37 +889,53 @@ __global__ void __launch_bounds__(256) stiffness_ref_kernel(ModelArgs M, GroupAr
                                          st[AMR_ST_DL * M.nip_total + gi], lam, mu, m);
             if (gam != 0.0)
                 for (int i = 0; i < 6; i++)
-                    for (int j = 0; j < 6; j++) sD[6 * i + j] -= gam * m[i] * m[j];
+                    for (int j = 0; j < 6; j++) D[6 * i + j] -= gam * m[i] * m[j];
         }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < nip * ND; t += blockDim.x) {  // dNdX = dNdR * inv(J)
+        const int ip = t / ND, i = t % ND / DIM, b = t % DIM;
+        const double *dNdR = G.tab + ip * ND, *iJ = sIJ + ip * JJ;
+        double s = 0.0;
+        for (int a = 0; a < DIM; a++) s = RADD(s, RMUL(dNdR[i * DIM + a], iJ[a * DIM + b]));
+        sG[t] = s;
+        sS[t] = RDIV(s, SQ2);
+    }
+    for (int ip0 = 0; ip0 < nip; ip0 += kRefChunk) {
+        const int nc = min(kRefChunk, nip - ip0);
         __syncthreads();
-        for (int t = threadIdx.x; t < ND; t += blockDim.x) {  // dNdX = dNdR * inv(J)
-            int i = t / DIM, b = t % DIM;
+        for (int t = threadIdx.x; t < nc * 6 * ND; t += blockDim.x) {  // DB = D * B
+            const int ip = ip0 + t / (6 * ND), k = t / ND % 6, j = t % ND, b = j / DIM, d = j % DIM;
+            const double *g = sG + ip * ND + b * DIM, *gs = sS + ip * ND + b * DIM, *D = sD + ip * 36 + 6 * k;
+            const double hb = sH[ip * NEN + b];
             double s = 0.0;
-            for (int a = 0; a < DIM; a++) s = RADD(s, RMUL(dNdR[i * DIM + a], sIJ[a * DIM + b]));
-            sG[t] = s;
-        }
-        __syncthreads();
-        for (int t = threadIdx.x; t < 6 * ND; t += blockDim.x) {  // DB = D * B
-            int k = t / ND, j = t % ND;
-            const double *gb = sG + (j / DIM) * DIM;
-            double s = 0.0;
-            for (int l = 0; l < 6; l++) s = RADD(s, RMUL(sD[6 * k + l], ref_B<DIM>(l, j % DIM, gb, sH[j / DIM])));
+#pragma unroll
+            for (int q = 0; q < kRefTerms; q++)
+                s = RADD(s, RMUL(D[ref_row<DIM>(q, d)], ref_value<DIM>(q, d, g, gs, hb)));
             sDB[t] = s;
         }
         __syncthreads();
-        const double coef = sCoef;
 #pragma unroll
         for (int q = 0; q < NE; q++) {  // K += coef * B' * DB
-            int idx = threadIdx.x + q * 256;
+            const int idx = threadIdx.x + q * 256;
             if (idx < ND * ND) {
-                int i = idx / ND, j = idx % ND;
-                const double *gi = sG + (i / DIM) * DIM;
-                double s = 0.0;
-                for (int k = 0; k < 6; k++) s = RADD(s, RMUL(ref_B<DIM>(k, i % DIM, gi, sH[i / DIM]), sDB[k * ND + j]));
-                acc[q] = RADD(acc[q], RMUL(coef, s));
+                const int i = idx / ND, j = idx % ND, a = i / DIM, c = i % DIM;
+                double v = acc[q];
+                for (int l = 0; l < nc; l++) {
+                    const int ip = ip0 + l;
+                    const double *g = sG + ip * ND + a * DIM, *gs = sS + ip * ND + a * DIM, *DB = sDB + l * 6 * ND + j;
+                    const double hb = DIM == 2 ? sH[ip * NEN + a] : 0.0;
+                    double s = 0.0;
+#pragma unroll
+                    for (int u = 0; u < kRefTerms; u++) {
+                        const double x = RMUL(ref_value<DIM>(u, c, g, gs, hb), DB[ref_row<DIM>(u, c) * ND]);
+                        s = u == 0 ? x : RADD(s, x);
+                    }
+                    v = RADD(v, RMUL(sCoef[ip], s));
+                }
+                acc[q] = v;
             }
         }
-        __syncthreads();
     }
     const int64_t base = M.kel_ptr[e];
 #pragma unroll
@@ -1413,10 +1447,27 @@ void launch_stiff(amr_model *m, const AmrGroup &g) {
     AMR_CUDA(cudaGetLastError());
 }
 
+// allows a kernel the most dynamic shared memory that it is launched with, once per kernel and device: a launch that set
+// its own size each time would race with other handles' threads
+void allow_shared(const void *kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::set<std::pair<const void *, int>> done;
+    if (bytes <= 48 * 1024) return;
+    int dev = 0;
+    AMR_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if (!done.insert({kernel, dev}).second) return;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) done.erase({kernel, dev});
+    AMR_CUDA(e);
+}
+
 template <int DIM, int NEN>
 void launch_stiff_ref(amr_model *m, const AmrGroup &g) {
     GroupArgs ga{g.tab, g.nip, g.first, g.count};
-    stiffness_ref_kernel<DIM, NEN><<<(unsigned)g.count, 256, 0, m->stream>>>(margs(m), ga, m->Kel, m->st, m->d_status);
+    const size_t smem = sizeof(double) * ref_doubles<DIM, NEN>(g.nip);
+    allow_shared((const void *)stiffness_ref_kernel<DIM, NEN>, sizeof(double) * ref_doubles<DIM, NEN>(AMR_MAXIP));
+    stiffness_ref_kernel<DIM, NEN><<<(unsigned)g.count, 256, smem, m->stream>>>(margs(m), ga, m->Kel, m->st, m->d_status);
     AMR_COUNT(1);
     AMR_CUDA(cudaGetLastError());
 }
