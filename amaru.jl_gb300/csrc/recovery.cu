@@ -14,6 +14,10 @@
 //   k_ip_fields   thread per IP: ip_state_vals of the IP's material
 //                 (linear-elastic.jl:140-164, von-mises.jl:159-168,330-341,
 //                 drucker-prager.jl:152-163 over tensors.jl:162-215)
+//   k_elem_moments  lanes of a warp per element: sums over its IPs of the monomials that the normal matrices need, and
+//                 the moments of the fields with the regression terms, about the element's centre
+//   k_patch_gram  eight lanes per task: the elements' sums translated to the patch centre, the normal matrix
+//                 and its Cholesky factor
 //   k_patch_fit   warp per task: the least-squares polynomial of reg_terms
 //                 (fe-model.jl:488-501) through the task's IP values, evaluated at
 //                 its nodes.  The regression runs in patch-centred coordinates
@@ -35,6 +39,7 @@
 #include <algorithm>
 #include <array>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <numeric>
 #include <vector>
@@ -46,8 +51,13 @@ namespace {
 constexpr double SR2 = 1.4142135623730951;  // src/tools/constants.jl:3
 constexpr int kFitWarps = 4;                 // warps per CTA of the fit kernels
 constexpr int kTermPad = 8;                  // doubles per regression row (<= 7 terms)
-constexpr int kRedStride = 29;               // Gram partials per lane in shared memory (28 + pad)
-constexpr int kInvDiag = 72;                 // offset of the reciprocal Cholesky pivots in the factor area
+constexpr int kFitDoubles = 14 * 32;         // a warp's coefficients (7 x 32) and terms of 32 nodes (7 each)
+constexpr int kFitArea = 928;                // their area beside a task's IPs; its size sets the largest patch
+constexpr int kInvDiag = 28;                 // a task's record: packed Cholesky factor, reciprocal pivots, scales
+constexpr int kScale = 35;
+constexpr int kTaskRec = 38;
+constexpr int kElemRec = 32;                 // an element's record: sums of monomials, centre, IP bounds per axis
+constexpr int kElemCentre = 23, kElemLow = 26, kElemHigh = 29;
 
 // ---------------------------------------------------------------------------
 // host tables
@@ -253,11 +263,6 @@ __device__ __forceinline__ double warp_sum_d(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_max_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 
 struct FitArgs {
     int64_t ntasks;
@@ -269,13 +274,16 @@ struct FitArgs {
     int nf, m_max, e_max;
     double *vst;
     int32_t *t_flag;
+    double *t_rec;       // ntasks x kTaskRec
+    double *geo, *mom;   // nelems x kElemRec; nelems x terms x nf (null: the moments come from the IPs)
+    int64_t nelems;
 };
 
 // per-warp shared memory, in doubles
 __host__ __device__ inline int64_t fit_warp_doubles(int m_max, int e_max) {
     return (int64_t)m_max * kTermPad     // scaled regression rows
            + m_max                       // IP global indices
-           + 32 * kRedStride             // Gram partials
+           + kFitArea                    // coefficients and terms of the nodes
            + AMR_NFIELD_CODES * kTermPad // right-hand sides / coefficients
            + 2 * kTermPad * kTermPad     // Cholesky factor / right singular vectors
            + (e_max + 2) / 2 + 1;        // element IP offsets (int32)
@@ -292,20 +300,18 @@ __device__ __forceinline__ WarpMem warp_mem(double *smem, int warp, int m_max, i
     double *b = smem + warp * fit_warp_doubles(m_max, e_max);
     w.phi = b; b += (int64_t)m_max * kTermPad;
     w.gidx = (int64_t *)b; b += m_max;
-    w.red = b; b += 32 * kRedStride;
+    w.red = b; b += kFitArea;
     w.bA = b; b += AMR_NFIELD_CODES * kTermPad;
     w.R = b; b += 2 * kTermPad * kTermPad;
     w.eoff = (int32_t *)b;
     return w;
 }
 
-// Loads the task's IPs: global indices, scaled regression rows; returns the number of terms, the centre c
-// of the coordinates and their reciprocal scales h (x_scaled = (x - c) * h).
-// raw: the reference's own basis (global coordinates, no centring or scaling)
+// Loads the task's IPs: global indices and regression rows about the centre c with the reciprocal scales h
+// (x_scaled = (x - c) * h)
 template <int DIM>
-__device__ int load_task(const FitArgs &A, int64_t t, const WarpMem &w, int lane, double *c, double *h, bool raw) {
-    const int m = A.t_m[t];
-    const int nt = nterms<DIM>(m);
+__device__ void load_task(const FitArgs &A, int64_t t, const WarpMem &w, int lane, int m, int nt, const double *c,
+                          const double *h) {
     const int64_t e0 = A.t_elem_ptr[t], ne = A.t_elem_ptr[t + 1] - e0;
     if (lane == 0) {
         int32_t o = 0;
@@ -317,9 +323,6 @@ __device__ int load_task(const FitArgs &A, int64_t t, const WarpMem &w, int lane
         w.eoff[ne] = o;
     }
     __syncwarp();
-    const int32_t cn = A.t_center[t];
-    for (int d = 0; d < 3; d++) c[d] = A.coords[3 * (int64_t)cn + d];
-    double hm[3] = {0.0, 0.0, 0.0};
     for (int i = lane; i < m; i += 32) {
         int lo = 0, hi = (int)ne - 1;  // element j with eoff[j] <= i < eoff[j+1]
         while (lo < hi) {
@@ -328,23 +331,12 @@ __device__ int load_task(const FitArgs &A, int64_t t, const WarpMem &w, int lane
         }
         const int64_t gi = A.ip_ptr[A.t_elem[e0 + lo]] + (i - w.eoff[lo]);
         w.gidx[i] = gi;
-        for (int d = 0; d < DIM; d++) hm[d] = fmax(hm[d], fabs(A.ipx[3 * gi + d] - c[d]));
-    }
-    for (int d = 0; d < DIM; d++) {  // h holds the reciprocal scale from here on
-        const double hd = warp_max_d(hm[d]);
-        h[d] = (!(hd > 0.0) || raw) ? 1.0 : 1.0 / hd;
-    }
-    if (raw) c[0] = c[1] = c[2] = 0.0;
-    __syncwarp();
-    for (int i = lane; i < m; i += 32) {
         double x[3], p[kTermPad];
-        const int64_t gi = w.gidx[i];
         for (int d = 0; d < DIM; d++) x[d] = (A.ipx[3 * gi + d] - c[d]) * h[d];
         terms<DIM>(x, nt, p);
         for (int k = 0; k < nt; k++) w.phi[i * kTermPad + k] = p[k];
     }
     __syncwarp();
-    return nt;
 }
 
 // values at the task's nodes from the coefficients in w.bA (field k of the mask at bA[k*kTermPad])
@@ -383,108 +375,371 @@ __device__ void field_moments(const FitArgs &A, const WarpMem &w, int lane, int 
     __syncwarp();
 }
 
+// The monomials of the normal matrix's entries: products of two regression terms, exponents per axis.  The first
+// kTerms are the terms themselves, in their order.
 template <int DIM>
-__global__ void __launch_bounds__(32 * kFitWarps) k_patch_fit(FitArgs A) {
-    extern __shared__ double smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const WarpMem w = warp_mem(smem, warp, A.m_max, A.e_max);
-    for (int64_t t = (int64_t)blockIdx.x * kFitWarps + warp; t < A.ntasks; t += (int64_t)gridDim.x * kFitWarps) {
-        double c[3], h[3];
-        const int m = A.t_m[t];
-        const int nt = load_task<DIM>(A, t, w, lane, c, h, false);
-        // Gram matrix of the scaled rows: lane partials, then lane k sums entry k over the lanes
-        double g[28];
+constexpr int kMono = DIM == 3 ? 23 : 15;
+template <int DIM>
+constexpr int kTerms = DIM == 3 ? 7 : 6;
+template <int DIM>
+__host__ __device__ constexpr int mono_exp(int i, int d) {
+    constexpr int T3[23][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 1, 0}, {0, 1, 1}, {1, 0, 1}, {2, 0, 0},
+                               {0, 2, 0}, {0, 0, 2}, {2, 1, 0}, {1, 2, 0}, {0, 2, 1}, {0, 1, 2}, {2, 0, 1}, {1, 0, 2},
+                               {1, 1, 1}, {2, 2, 0}, {0, 2, 2}, {2, 0, 2}, {2, 1, 1}, {1, 2, 1}, {1, 1, 2}};
+    constexpr int T2[15][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {1, 1, 0}, {2, 0, 0}, {0, 2, 0}, {3, 0, 0}, {2, 1, 0},
+                               {1, 2, 0}, {0, 3, 0}, {4, 0, 0}, {3, 1, 0}, {2, 2, 0}, {1, 3, 0}, {0, 4, 0}};
+    return DIM == 3 ? T3[i][d] : T2[i < 15 ? i : 0][d];
+}
+template <int DIM>
+__host__ __device__ constexpr int mono_find(int a, int b, int c) {
+    for (int i = 0; i < kMono<DIM>; i++)
+        if (mono_exp<DIM>(i, 0) == a && mono_exp<DIM>(i, 1) == b && mono_exp<DIM>(i, 2) == c) return i;
+    return -1;
+}
+
+// sums of the monomials of x + t from those of x, axis by axis (Taylor shift by repeated passes)
+template <int DIM, int AXIS>
+__device__ __forceinline__ void shift_axis(double *m, double t) {
+    constexpr int TOP = DIM == 3 ? 2 : 4;
 #pragma unroll
-        for (int k = 0; k < 28; k++) g[k] = 0.0;
-        for (int i = lane; i < m; i += 32) {
-            const double *p = w.phi + i * kTermPad;
-            int k = 0;
+    for (int pass = 1; pass <= TOP; pass++)
 #pragma unroll
-            for (int a = 0; a < 7; a++)
+        for (int a = TOP; a >= 1; a--)
 #pragma unroll
-                for (int b = a; b < 7; b++, k++)
-                    if (b < nt) g[k] = fma(p[a], p[b], g[k]);
+            for (int i = 0; i < kMono<DIM>; i++)
+                if (a >= pass && mono_exp<DIM>(i, AXIS) == a)
+                    m[i] = fma(t, m[mono_find<DIM>(mono_exp<DIM>(i, 0) - (AXIS == 0), mono_exp<DIM>(i, 1) - (AXIS == 1),
+                                                   mono_exp<DIM>(i, 2) - (AXIS == 2))], m[i]);
+}
+
+// order of doubles as integers (no NaN), so that bounds are found off the FP64 pipe
+__device__ __forceinline__ long long ordered(double x) {
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double unordered(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+
+// W lanes per element, W >= its number of IPs.  The FP64 pipe (2 operations per SM and cycle) bounds all of the fit, so
+// the sums over IPs, which every patch of an element took again, are taken once per element about its centre and
+// translated: at 27 points and 16 fields a patch of eight elements needs 41 000 operations from the points and 15 000 from
+// the moments.  41 x 17 x 17 HEX20: the one kernel per patch took 1.16 ms at 81 % of the pipe; a whole
+// recovery took 1.73 ms and takes 1.01 (20 x 20 x 20: the fit alone 0.78 and 0.30 ms).
+constexpr int kElemWarps = 4;
+constexpr int kMonoPad = 25;
+template <int DIM, bool MOM, int W>
+__global__ void __launch_bounds__(32 * kElemWarps) k_elem_moments(FitArgs A) {
+    constexpr int ROWS = W < AMR_MAXIP ? W : AMR_MAXIP;
+    __shared__ double s_mono[32 / W * kElemWarps][ROWS * kMonoPad];
+    const int slot = threadIdx.x / W, sub = threadIdx.x % W;
+    const int64_t e = (int64_t)blockIdx.x * (32 / W * kElemWarps) + slot;
+    const bool any = e < A.nelems;
+    double *mono = s_mono[slot];
+    const int64_t g0 = any ? A.ip_ptr[e] : 0;
+    const int nip = any ? min((int)(A.ip_ptr[e + 1] - g0), ROWS) : 0;
+    const bool on = sub < nip;
+    double x[3] = {0.0, 0.0, 0.0}, ce[3] = {0.0, 0.0, 0.0}, lo[3] = {0.0, 0.0, 0.0}, hi[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+        if (on) x[d] = A.ipx[3 * (g0 + sub) + d];
+        long long kl = on ? ordered(x[d]) : LLONG_MAX, kh = on ? ordered(x[d]) : LLONG_MIN;
+#pragma unroll
+        for (int o = W / 2; o > 0; o >>= 1) {
+            kl = min(kl, __shfl_xor_sync(0xffffffffu, kl, o));
+            kh = max(kh, __shfl_xor_sync(0xffffffffu, kh, o));
+        }
+        lo[d] = unordered(kl);
+        hi[d] = unordered(kh);
+        ce[d] = 0.5 * (lo[d] + hi[d]);
+        x[d] -= ce[d];
+    }
+    if (on) {
+        double pw[3][5];
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            pw[d][0] = 1.0;
+#pragma unroll
+            for (int a = 1; a <= (DIM == 3 ? 2 : 4); a++) pw[d][a] = pw[d][a - 1] * x[d];
         }
 #pragma unroll
-        for (int k = 0; k < 28; k++) w.red[lane * kRedStride + k] = g[k];
-        __syncwarp();
-        if (lane < 28) {
-            double s = 0.0;
-            for (int l = 0; l < 32; l++) s += w.red[l * kRedStride + lane];
-            w.bA[lane] = s;  // packed upper triangle, row by row (bA is free until the moments)
+        for (int i = 0; i < kMono<DIM>; i++) {
+            double v = pw[0][mono_exp<DIM>(i, 0)] * pw[1][mono_exp<DIM>(i, 1)];
+            if (DIM == 3) v *= pw[2][mono_exp<DIM>(i, 2)];
+            mono[sub * kMonoPad + i] = v;
         }
-        __syncwarp();
-        // Cholesky G = R'R: the pivots on every lane, row j's off-diagonal entries on lanes i > j.
-        // R[j][i] at R[j*kTermPad+i], the reciprocal pivots at R[kInvDiag+j]
-        const double *G = w.bA;
-        double *R = w.R;
-        bool ok = true;
-        double dmin = DBL_MAX, dmax = 0.0;
+    }
+    __syncwarp();
+    if (!any) return;
+    double *geo = A.geo + e * kElemRec;
+    for (int q = sub; q < kMono<DIM>; q += W) {
+        double s = 0.0;
+        for (int i = 0; i < nip; i++) s += mono[i * kMonoPad + q];
+        geo[q] = s;
+    }
+    if (sub == 0)
 #pragma unroll
-        for (int j = 0; j < 7; j++) {
-            if (j >= nt) break;
-            double d = G[packed(j, j)];
+        for (int d = 0; d < DIM; d++) {
+            geo[kElemCentre + d] = ce[d];
+            geo[kElemLow + d] = lo[d];
+            geo[kElemHigh + d] = hi[d];
+        }
+    if (!MOM) return;
+    const int P = kTerms<DIM> * A.nf;
+    const double *v = A.ipv + g0 * A.nf;
+    double *out = A.mom + e * P;
+    constexpr int U = 4;  // pairs (term, field) of a lane at a time
+    for (int p0 = sub; p0 < P; p0 += W * U) {
+        double acc[U];
+        int q[U], k[U];
 #pragma unroll
-            for (int q = 0; q < 7; q++)
-                if (q < j) d -= R[q * kTermPad + j] * R[q * kTermPad + j];
-            if (!(d > 0.0)) { ok = false; break; }
-            const double r = sqrt(d), ir = 1.0 / r;
+        for (int u = 0; u < U; u++) {
+            const int p = min(p0 + W * u, P - 1);
+            q[u] = p / A.nf;
+            k[u] = p % A.nf;
+            acc[u] = 0.0;
+        }
+        for (int i = 0; i < nip; i++)
+#pragma unroll
+            for (int u = 0; u < U; u++) acc[u] = fma(mono[i * kMonoPad + q[u]], v[i * A.nf + k[u]], acc[u]);
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (p0 + W * u < P) out[p0 + W * u] = acc[u];
+    }
+}
+
+// Eight lanes per task sum the elements' translated monomials; then a thread per task factors the normal matrix, whose
+// chain of square roots and divisions costs a warp as much as all moments when each warp does its own (7 pivots, 32
+// lanes alike).
+constexpr int kGramTasks = 16;
+template <int DIM>
+__global__ void __launch_bounds__(8 * kGramTasks) k_patch_gram(FitArgs A) {
+    constexpr int NM = kMono<DIM>, NT = kTerms<DIM>;
+    __shared__ double s_mono[kGramTasks][kMonoPad + 4];
+    const int sub = threadIdx.x & 7, slot = threadIdx.x >> 3;
+    const int64_t t0 = (int64_t)blockIdx.x * kGramTasks, t = t0 + slot;
+    double m[NM], hm[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < NM; i++) m[i] = 0.0;
+    if (t < A.ntasks) {
+        const double *c = A.coords + 3 * (int64_t)A.t_center[t];
+        for (int64_t j = A.t_elem_ptr[t] + sub; j < A.t_elem_ptr[t + 1]; j += 8) {
+            const double *geo = A.geo + (int64_t)A.t_elem[j] * kElemRec;
+            double v[NM];
+#pragma unroll
+            for (int i = 0; i < NM; i++) v[i] = geo[i];
+            shift_axis<DIM, 0>(v, geo[kElemCentre] - c[0]);
+            shift_axis<DIM, 1>(v, geo[kElemCentre + 1] - c[1]);
+            if (DIM == 3) shift_axis<DIM, 2>(v, geo[kElemCentre + 2] - c[2]);
+#pragma unroll
+            for (int i = 0; i < NM; i++) m[i] += v[i];
+#pragma unroll
+            for (int d = 0; d < DIM; d++)  // the largest |x - c| over the IPs: rounding is monotonic
+                hm[d] = fmax(hm[d], fmax(fabs(geo[kElemLow + d] - c[d]), fabs(geo[kElemHigh + d] - c[d])));
+        }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+#pragma unroll
+        for (int i = 0; i < NM; i++) m[i] += __shfl_xor_sync(0xffffffffu, m[i], o);
+#pragma unroll
+        for (int d = 0; d < DIM; d++) hm[d] = fmax(hm[d], __shfl_xor_sync(0xffffffffu, hm[d], o));
+    }
+    if (sub == 0) {
+#pragma unroll
+        for (int i = 0; i < NM; i++) s_mono[slot][i] = m[i];
+#pragma unroll
+        for (int d = 0; d < DIM; d++) s_mono[slot][kMonoPad + d] = hm[d];
+    }
+    __syncthreads();
+    const int64_t tt = t0 + threadIdx.x;
+    if (threadIdx.x >= kGramTasks || tt >= A.ntasks) return;
+    const double *sm = s_mono[threadIdx.x];
+    double *rec = A.t_rec + tt * kTaskRec;
+    const int nt = nterms<DIM>(A.t_m[tt]);
+    double hp[3][5];
+#pragma unroll
+    for (int d = 0; d < DIM; d++) {
+        const double hd = sm[kMonoPad + d];
+        const double h = hd > 0.0 ? 1.0 / hd : 1.0;
+        rec[kScale + d] = h;
+        hp[d][0] = 1.0;
+#pragma unroll
+        for (int a = 1; a <= (DIM == 3 ? 2 : 4); a++) hp[d][a] = hp[d][a - 1] * h;
+    }
+#pragma unroll
+    for (int i = 0; i < NM; i++) {
+        double v = sm[i] * hp[0][mono_exp<DIM>(i, 0)];
+        v *= hp[1][mono_exp<DIM>(i, 1)];
+        if (DIM == 3) v *= hp[2][mono_exp<DIM>(i, 2)];
+        m[i] = v;
+    }
+    // Cholesky G = R'R, R packed by rows; beyond the nt terms G is the unit matrix
+    double R[28];
+    bool ok = true;
+    double dmin = DBL_MAX, dmax = 0.0;
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        double d = j < nt ? m[mono_find<DIM>(2 * mono_exp<DIM>(j, 0), 2 * mono_exp<DIM>(j, 1), 2 * mono_exp<DIM>(j, 2))] : 1.0;
+#pragma unroll
+        for (int q = 0; q < NT; q++)
+            if (q < j) d -= R[packed(q, j)] * R[packed(q, j)];
+        if (!(d > 0.0)) ok = false;
+        const double r = sqrt(d), ir = 1.0 / r;
+        if (j < nt) {
             dmin = fmin(dmin, r);
             dmax = fmax(dmax, r);
-            if (lane > j && lane < nt) {
-                double v = G[packed(j, lane)];
+        }
+        R[packed(j, j)] = r;
+        rec[kInvDiag + j] = ir;
 #pragma unroll
-                for (int q = 0; q < 7; q++)
-                    if (q < j) v -= R[q * kTermPad + j] * R[q * kTermPad + lane];
-                R[j * kTermPad + lane] = v * ir;
-            } else if (lane == j) {
-                R[j * kTermPad + j] = r;
-                R[kInvDiag + j] = ir;
+        for (int i = 0; i < NT; i++)
+            if (i > j) {
+                double v = 0.0;
+                if (i < nt) {
+                    v = m[mono_find<DIM>(mono_exp<DIM>(i, 0) + mono_exp<DIM>(j, 0), mono_exp<DIM>(i, 1) + mono_exp<DIM>(j, 1),
+                                         mono_exp<DIM>(i, 2) + mono_exp<DIM>(j, 2))];
+#pragma unroll
+                    for (int q = 0; q < NT; q++)
+                        if (q < j) v -= R[packed(q, j)] * R[packed(q, i)];
+                    v *= ir;
+                }
+                R[packed(j, i)] = v;
+                rec[packed(j, i)] = v;
             }
-            __syncwarp();
-        }
-        // the normal equations square the condition number: patches conditioned worse than 1e4 go to
-        // the SVD path
-        if (ok && !(dmin > 1e-4 * dmax)) ok = false;
-        if (lane == 0) A.t_flag[t] = ok ? 0 : 1;
-        if (!ok) {
-            __syncwarp();
-            continue;
-        }
+    }
+    // the normal equations square the condition number: patches conditioned worse than 1e4 go to the SVD path
+    if (!(dmin > 1e-4 * dmax)) ok = false;
+    A.t_flag[tt] = ok ? 0 : 1;
+}
+
+// Warp per task.  MOM: the right-hand sides from the elements' moments, half a warp per element where the fields fit;
+// otherwise from the IPs (elements of few points, where the translation would cost more than the sum).
+template <int DIM, bool MOM>
+__global__ void __launch_bounds__(32 * kFitWarps) k_patch_fit(FitArgs A) {
+    constexpr int NT = kTerms<DIM>;
+    extern __shared__ double smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // coefficients [term][field] and terms of 32 nodes [node][term]; where the IPs are loaded too, in their area
+    double *cf = MOM ? smem + warp * kFitDoubles : warp_mem(smem, warp, A.m_max, A.e_max).red;
+    double *tm = cf + 7 * 32;
+    for (int64_t t = (int64_t)blockIdx.x * kFitWarps + warp; t < A.ntasks; t += (int64_t)gridDim.x * kFitWarps) {
+        if (A.t_flag[t]) continue;
+        const int m = A.t_m[t], nt = nterms<DIM>(m);
         const int mk = A.t_mask[t];
         const int nfm = A.mask_nf[mk];
         const int32_t *flds = A.mask_fields + mk * AMR_NFIELD_CODES;
-        field_moments(A, w, lane, m, nt, nfm, flds);
-        // coefficients: R'y = b, R a = y (lane per field)
-        if (lane < nfm) {
-            double y[7];
-            double *b = w.bA + lane * kTermPad;
+        const double *rec = A.t_rec + t * kTaskRec;
+        double c[3], h[3];
 #pragma unroll
-            for (int j = 0; j < 7; j++) {
-                if (j < nt) {
-                    double v = b[j];
-#pragma unroll
-                    for (int q = 0; q < 7; q++)
-                        if (q < j) v -= R[q * kTermPad + j] * y[q];
-                    y[j] = v * R[kInvDiag + j];
-                }
-            }
-#pragma unroll
-            for (int j = 6; j >= 0; j--) {
-                if (j < nt) {
-                    double v = y[j];
-#pragma unroll
-                    for (int q = 0; q < 7; q++)
-                        if (q > j && q < nt) v -= R[j * kTermPad + q] * y[q];
-                    y[j] = v * R[kInvDiag + j];
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 7; j++)
-                if (j < nt) b[j] = y[j];
+        for (int d = 0; d < DIM; d++) {
+            c[d] = A.coords[3 * (int64_t)A.t_center[t] + d];
+            h[d] = rec[kScale + d];
         }
-        __syncwarp();
-        write_nodes<DIM>(A, t, w, lane, nt, nfm, flds, c, h);
+        double b[NT];
+#pragma unroll
+        for (int q = 0; q < NT; q++) b[q] = 0.0;
+        if (MOM) {
+            const bool half = nfm <= 16;
+            const int k = half ? lane & 15 : lane, step = half ? 2 : 1;
+            if (k < nfm) {
+                const int f = flds[k];
+                for (int64_t j = A.t_elem_ptr[t] + (half ? lane >> 4 : 0); j < A.t_elem_ptr[t + 1]; j += step) {
+                    const int64_t e = A.t_elem[j];
+                    const double *ce = A.geo + e * kElemRec + kElemCentre;
+                    const double *mo = A.mom + e * NT * A.nf + f;
+                    double v[NT], s[3];
+#pragma unroll
+                    for (int q = 0; q < NT; q++) v[q] = mo[q * A.nf];
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) s[d] = ce[d] - c[d];
+                    if (DIM == 3) {  // 1 x y z xy yz xz
+                        const double x0 = v[1], y0 = v[2], z0 = v[3];
+                        v[1] = fma(s[0], v[0], x0);
+                        v[2] = fma(s[1], v[0], y0);
+                        v[3] = fma(s[2], v[0], z0);
+                        v[4] = fma(s[0], v[2], fma(s[1], x0, v[4]));
+                        v[5] = fma(s[1], v[3], fma(s[2], y0, v[5]));
+                        v[6] = fma(s[0], v[3], fma(s[2], x0, v[6]));
+                    } else {  // 1 x y xy xx yy
+                        const double x0 = v[1], y0 = v[2];
+                        v[1] = fma(s[0], v[0], x0);
+                        v[2] = fma(s[1], v[0], y0);
+                        v[3] = fma(s[0], v[2], fma(s[1], x0, v[3]));
+                        v[4] = fma(s[0], v[1] + x0, v[4]);
+                        v[5] = fma(s[1], v[2] + y0, v[5]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < NT; q++) b[q] += v[q];
+                }
+            }
+            if (half)
+#pragma unroll
+                for (int q = 0; q < NT; q++) b[q] += __shfl_xor_sync(0xffffffffu, b[q], 16);
+            if (DIM == 3) {
+                b[1] *= h[0]; b[2] *= h[1]; b[3] *= h[2];
+                b[4] *= h[0] * h[1]; b[5] *= h[1] * h[2]; b[6] *= h[0] * h[2];
+            } else {
+                b[1] *= h[0]; b[2] *= h[1];
+                b[3] *= h[0] * h[1]; b[4] *= h[0] * h[0]; b[5] *= h[1] * h[1];
+            }
+        } else {
+            const WarpMem w = warp_mem(smem, warp, A.m_max, A.e_max);
+            load_task<DIM>(A, t, w, lane, m, nt, c, h);
+            field_moments(A, w, lane, m, nt, nfm, flds);
+            if (lane < nfm)
+#pragma unroll
+                for (int q = 0; q < NT; q++)
+                    if (q < nt) b[q] = w.bA[lane * kTermPad + q];
+        }
+        // coefficients: R'y = b, R a = y (lane per field); the terms beyond nt have none
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            double v = j < nt ? b[j] : 0.0;
+#pragma unroll
+            for (int q = 0; q < NT; q++)
+                if (q < j) v -= rec[packed(q, j)] * b[q];
+            b[j] = v * rec[kInvDiag + j];
+        }
+#pragma unroll
+        for (int j = NT - 1; j >= 0; j--) {
+            double v = b[j];
+#pragma unroll
+            for (int q = 0; q < NT; q++)
+                if (q > j) v -= rec[packed(j, q)] * b[q];
+            b[j] = v * rec[kInvDiag + j];
+        }
+        if (lane < nfm)
+#pragma unroll
+            for (int q = 0; q < NT; q++) cf[q * 32 + lane] = b[q];
+        // values at the nodes, 32 nodes at a time, lanes over (node, field): all lanes busy, stores side by side
+        const int64_t s0 = A.t_node_ptr[t];
+        const int n = (int)(A.t_node_ptr[t + 1] - s0);
+        const int dj = 32 / nfm, dk = 32 % nfm;
+        for (int n0 = 0; n0 < n; n0 += 32) {
+            __syncwarp();
+            if (n0 + lane < n) {
+                const int32_t node = A.t_node[s0 + n0 + lane];
+                double x[3], p[kTermPad];
+#pragma unroll
+                for (int d = 0; d < DIM; d++) x[d] = (A.coords[3 * (int64_t)node + d] - c[d]) * h[d];
+                terms<DIM>(x, NT, p);
+#pragma unroll
+                for (int q = 1; q < NT; q++) tm[lane * 7 + q] = p[q];
+            }
+            __syncwarp();
+            const int nn = min(32, n - n0);
+            int j = lane / nfm, k = lane % nfm;
+            while (j < nn) {
+                double v = cf[k];
+#pragma unroll
+                for (int q = 1; q < NT; q++) v = fma(tm[j * 7 + q], cf[q * 32 + k], v);
+                A.vst[(s0 + n0 + j) * A.nf + flds[k]] = v;
+                j += dj;
+                k += dk;
+                if (k >= nfm) { k -= nfm; j++; }
+            }
+        }
         __syncwarp();
     }
 }
@@ -497,9 +752,9 @@ __global__ void __launch_bounds__(32 * kFitWarps) k_patch_svd(FitArgs A) {
     const WarpMem w = warp_mem(smem, warp, A.m_max, A.e_max);
     for (int64_t t = (int64_t)blockIdx.x * kFitWarps + warp; t < A.ntasks; t += (int64_t)gridDim.x * kFitWarps) {
         if (!A.t_flag[t]) continue;
-        double c[3], h[3];
-        const int m = A.t_m[t];
-        const int nt = load_task<DIM>(A, t, w, lane, c, h, true);
+        const double c[3] = {0.0, 0.0, 0.0}, h[3] = {1.0, 1.0, 1.0};  // the reference's own basis
+        const int m = A.t_m[t], nt = nterms<DIM>(m);
+        load_task<DIM>(A, t, w, lane, m, nt, c, h);
         double *V = w.R;  // nt x nt right singular vectors, row-major
         if (lane < kTermPad * kTermPad) {
             V[lane] = (lane / kTermPad == lane % kTermPad) ? 1.0 : 0.0;
@@ -593,10 +848,11 @@ struct AmrRecovery {
     int nf = 0, nmask = 0, m_max = 1, e_max = 1;
     std::vector<int32_t> codes;      // output field codes, reference order
     int64_t ntasks = 0, nslots = 0, ncontrib = 0;
-    double fit_flops = 0.0;          // algorithmic FP64 operations of one k_patch_fit launch
+    double fit_flops = 0.0;          // FP64 operations of one fit, its sums taken over each patch's points
     int64_t n_svd = 0;               // tasks on the SVD path (known after a launch)
     // device
     double *ipx = nullptr, *ipv = nullptr, *vst = nullptr;
+    double *geo = nullptr, *mom = nullptr, *t_rec = nullptr;  // element and task records; mom only where it is used
     int32_t *ip_elem = nullptr, *fmap = nullptr, *mask_nf = nullptr, *mask_fields = nullptr, *field_mask = nullptr;
     int64_t *t_elem_ptr = nullptr, *t_node_ptr = nullptr, *c_ptr = nullptr, *c_slot = nullptr;
     int32_t *t_elem = nullptr, *t_node = nullptr, *t_mask = nullptr, *t_center = nullptr, *t_m = nullptr,
@@ -610,6 +866,12 @@ void put(T **d, const std::vector<T> &h, cudaStream_t s) {
     amr_alloc(d, h.size());
     if (!h.empty()) AMR_CUDA(cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
 }
+
+// Field moments per element, translated for each patch, or the sums over each patch's IPs?  A translation costs 16 (2-D:
+// 12) operations per field and element, a sum 7 (6) per field and IP, and a 3-D element is in 8 patches, a 2-D one in 4.
+// The fit from moments / from IPs: TET4 of 1 point 144 / 110 us, TET10 of 4 135 / 162, HEX8 of 8 540 / 718, HEX20
+// of 27 295 / 617; TRI6 of 3 309 / 273, QUAD4 of 4 425 / 398, QUAD8 of 9 345 / 389.
+bool by_elements(const amr_model *m) { return m->nip_total >= (m->ndim == 3 ? 4 : 8) * m->nelems; }
 
 void build(amr_model *m) {
     auto *R = new AmrRecovery();
@@ -801,6 +1063,9 @@ void build(amr_model *m) {
     amr_alloc(&R->ipx, 3 * m->nip_total);
     amr_alloc(&R->ipv, std::max<int64_t>(1, m->nip_total * R->nf));
     amr_alloc(&R->vst, std::max<int64_t>(1, R->nslots * R->nf));
+    amr_alloc(&R->geo, ne * kElemRec);
+    amr_alloc(&R->t_rec, std::max<int64_t>(1, R->ntasks * kTaskRec));
+    if (by_elements(m)) amr_alloc(&R->mom, ne * R->nf * (m->ndim == 3 ? kTerms<3> : kTerms<2>));
     AMR_CUDA(cudaMemsetAsync(R->ipx, 0, 3 * m->nip_total * sizeof(double), s));
     for (const AmrGroup &g : m->groups) {
         const double *Ntab = g.tab + (size_t)g.nip * g.nen * m->ndim + g.nip;
@@ -821,24 +1086,46 @@ FitArgs fit_args(amr_model *m) {
     A.t_mask = R->t_mask; A.t_center = R->t_center; A.t_m = R->t_m; A.mask_nf = R->mask_nf;
     A.mask_fields = R->mask_fields; A.ip_ptr = m->ip_ptr; A.ipx = R->ipx; A.coords = m->coords; A.ipv = R->ipv;
     A.nf = R->nf; A.m_max = R->m_max; A.e_max = R->e_max; A.vst = R->vst; A.t_flag = R->t_flag;
+    A.t_rec = R->t_rec; A.geo = R->geo; A.mom = R->mom; A.nelems = m->nelems;
     return A;
 }
 
-unsigned fit_grid(amr_model *m, size_t smem) {
+template <class K>
+unsigned fit_grid(amr_model *m, K kernel, size_t smem) {
     int dev = 0, sms = 0, per_sm = 0;
     AMR_CUDA(cudaGetDevice(&dev));
     AMR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (m->ndim == 3)
-        AMR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_patch_fit<3>, 32 * kFitWarps, smem));
-    else
-        AMR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_patch_fit<2>, 32 * kFitWarps, smem));
+    AMR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * kFitWarps, smem));
     const int64_t need = (m->rec->ntasks + kFitWarps - 1) / kFitWarps;
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)sms * std::max(1, per_sm)));
 }
 
 template <class K>
-void set_smem(K kernel, size_t smem) {
-    if (smem > 48 * 1024) AMR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+void launch_tasks(amr_model *m, K kernel, const FitArgs &A, size_t smem) {
+    // the most that build() accepts, whatever this launch takes: other handles' threads set it too
+    if (smem > 48 * 1024) AMR_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    kernel<<<fit_grid(m, kernel, smem), 32 * kFitWarps, smem, m->stream>>>(A);
+    AMR_COUNT(1);
+    AMR_CUDA(cudaGetLastError());
+}
+
+template <int DIM, bool MOM, int W>
+void launch_elements(amr_model *m, const FitArgs &A) {
+    const int64_t per = 32 / W * kElemWarps;
+    k_elem_moments<DIM, MOM, W><<<(unsigned)((m->nelems + per - 1) / per), 32 * kElemWarps, 0, m->stream>>>(A);
+}
+
+template <int DIM, bool MOM>
+void launch_fit_dim(amr_model *m, const FitArgs &A, size_t smem) {
+    int nip = 1;
+    for (const AmrGroup &g : m->groups) nip = std::max(nip, (int)g.nip);
+    if (nip <= 4) launch_elements<DIM, MOM, 4>(m, A);
+    else if (nip <= 8) launch_elements<DIM, MOM, 8>(m, A);
+    else launch_elements<DIM, MOM, 32>(m, A);
+    k_patch_gram<DIM><<<(unsigned)((A.ntasks + kGramTasks - 1) / kGramTasks), 8 * kGramTasks, 0, m->stream>>>(A);
+    AMR_COUNT(2);
+    AMR_CUDA(cudaGetLastError());
+    launch_tasks(m, k_patch_fit<DIM, MOM>, A, MOM ? kFitWarps * kFitDoubles * sizeof(double) : smem);
 }
 
 // the fit and SVD launches over all tasks
@@ -846,24 +1133,16 @@ void launch_fit(amr_model *m, bool svd) {
     AmrRecovery *R = m->rec;
     if (!R->ntasks) return;
     const size_t smem = (size_t)fit_warp_doubles(R->m_max, R->e_max) * sizeof(double) * kFitWarps;
-    FitArgs A = fit_args(m);
+    const FitArgs A = fit_args(m);
     if (m->ndim == 3) {
-        set_smem(k_patch_fit<3>, smem);
-        set_smem(k_patch_svd<3>, smem);
+        if (svd) launch_tasks(m, k_patch_svd<3>, A, smem);
+        else if (A.mom) launch_fit_dim<3, true>(m, A, smem);
+        else launch_fit_dim<3, false>(m, A, smem);
     } else {
-        set_smem(k_patch_fit<2>, smem);
-        set_smem(k_patch_svd<2>, smem);
+        if (svd) launch_tasks(m, k_patch_svd<2>, A, smem);
+        else if (A.mom) launch_fit_dim<2, true>(m, A, smem);
+        else launch_fit_dim<2, false>(m, A, smem);
     }
-    const unsigned grid = fit_grid(m, smem);
-    if (!svd) {
-        if (m->ndim == 3) k_patch_fit<3><<<grid, 32 * kFitWarps, smem, m->stream>>>(A);
-        else k_patch_fit<2><<<grid, 32 * kFitWarps, smem, m->stream>>>(A);
-    } else {
-        if (m->ndim == 3) k_patch_svd<3><<<grid, 32 * kFitWarps, smem, m->stream>>>(A);
-        else k_patch_svd<2><<<grid, 32 * kFitWarps, smem, m->stream>>>(A);
-    }
-    AMR_COUNT(1);
-    AMR_CUDA(cudaGetLastError());
 }
 
 }  // namespace
@@ -936,6 +1215,7 @@ void amr_recovery_free(amr_model *m) {
     amr_free(R->mask_nf); amr_free(R->mask_fields); amr_free(R->field_mask); amr_free(R->t_elem_ptr);
     amr_free(R->t_node_ptr); amr_free(R->c_ptr); amr_free(R->c_slot); amr_free(R->t_elem); amr_free(R->t_node);
     amr_free(R->t_mask); amr_free(R->t_center); amr_free(R->t_m); amr_free(R->t_flag);
+    amr_free(R->geo); amr_free(R->mom); amr_free(R->t_rec);
     delete R;
     m->rec = nullptr;
 }
