@@ -1244,14 +1244,7 @@ __global__ void __launch_bounds__(256, 2) internal_kernel(ModelArgs M, GroupArgs
         int64_t e = e0 + el;
         if (elem_skipped(M, e)) continue;
         double g[NEN * DIM];
-        double det = 0.0, wc = 0.0;  // (with the cache: wc = detJ * weight * thickness from it)
-        if (DIM == 3 && G.geo_g) {
-            const int64_t el0 = e - G.first;
-            for (int q = 0; q < NEN * DIM; q++) g[q] = G.geo_g[(el0 * NEN * DIM + q) * nip + ip];
-            wc = G.geo_w[el0 * nip + ip];
-        } else {
-            det = ip_geometry<DIM>(NEN, dNdR + ip * NEN * DIM, sC + el * NEN * DIM, g);
-        }
+        const double det = ip_geometry<DIM>(NEN, dNdR + ip * NEN * DIM, sC + el * NEN * DIM, g);
         const double *u = sU + el * NEN * DIM;
         double de[6] = {0, 0, 0, 0, 0, 0};
         for (int a = 0; a < NEN; a++) {
@@ -1290,7 +1283,7 @@ __global__ void __launch_bounds__(256, 2) internal_kernel(ModelArgs M, GroupArgs
             for (int i = 0; i < 6; i++) ds[i] = 0.0;
         }
         for (int f = 0; f < AMR_NST; f++) st[f * M.nip_total + gi] = s1[f];
-        const double coef = (DIM == 3 && G.geo_g) ? wc : det * wq[ip] * th;
+        const double coef = det * wq[ip] * th;
         double *fo = sF + (el * nip + ip) * NEN * DIM;
         for (int a = 0; a < NEN; a++) {
             double v[DIM];
@@ -1306,6 +1299,77 @@ __global__ void __launch_bounds__(256, 2) internal_kernel(ModelArgs M, GroupArgs
         if (elem_skipped(M, e0 + el)) continue;
         double s = 0.0;
         for (int ip = 0; ip < nip; ip++) s += sF[(el * nip + ip) * NEN * DIM + q];
+        Fel[M.fel_ptr[e0 + el] + q] = s;
+    }
+}
+
+// The same with the 3-D geometry cache, which is read where it is used: a thread per IP for the strains and the
+// constitutive update, then a thread per force component, which sums B' (coef ds) over the IPs in their order.  dN/dX held
+// in registers from one to the other (60 doubles for HEX20) spilled, and the IPs' forces passed through shared memory left
+// two CTAs of half-idle threads on an SM.  FP64 bounds it (82 % of the pipe), so the factors 1 / sqrt(2) and coef are taken
+// once per IP, not at each node: 31 x 13 x 13 HEX20, 141 500 IPs in von Mises flow, 251 us before and 176 now.
+constexpr int kIntThreads = 64;
+template <int NEN>
+__global__ void __launch_bounds__(kIntThreads) internal_cached_kernel(ModelArgs M, GroupArgs G, int epb, const double *dU,
+                                                                      const double *stbk, double *st, double *Fel,
+                                                                      int32_t *status) {
+    constexpr int ND = NEN * 3;
+    extern __shared__ double sm[];
+    const int nip = G.nip;
+    double *sU = sm;              // epb x ND
+    double *sM = sU + epb * ND;   // epb x nip x 7 (6 used: no bank conflicts): coef ds, the shear terms / sqrt(2)
+    const int64_t e0 = G.first + (int64_t)blockIdx.x * epb, el0 = (int64_t)blockIdx.x * epb;
+    const int ne = (int)min((int64_t)epb, G.count - el0);
+    for (int t = threadIdx.x; t < ne * ND; t += kIntThreads) {
+        const int el = t / ND, q = t % ND;
+        sU[t] = dU[(int64_t)M.conn[M.conn_ptr[e0 + el] + q / 3] * 3 + q % 3];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ne * nip; t += kIntThreads) {
+        const int el = t / nip, ip = t % nip;
+        const int64_t e = e0 + el;
+        if (elem_skipped(M, e)) continue;
+        const double *geo = G.geo_g + (el0 + el) * ND * nip + ip, *u = sU + el * ND;
+        const int64_t gi = M.ip_ptr[e] + ip;
+        double s0[AMR_NST], s1[AMR_NST], ds[6];
+        for (int f = 0; f < AMR_NST; f++) s0[f] = stbk[f * M.nip_total + gi];
+        double de[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 5
+        for (int a = 0; a < NEN; a++) {
+            const double ga[3] = {geo[(3 * a) * nip], geo[(3 * a + 1) * nip], geo[(3 * a + 2) * nip]};
+            const double *ua = u + a * 3;
+            de[0] += ga[0] * ua[0];
+            de[1] += ga[1] * ua[1];
+            de[2] += ga[2] * ua[2];
+            de[3] = fma(ga[2], ua[1], fma(ga[1], ua[2], de[3]));
+            de[4] = fma(ga[2], ua[0], fma(ga[0], ua[2], de[4]));
+            de[5] = fma(ga[1], ua[0], fma(ga[0], ua[1], de[5]));
+        }
+        for (int i = 3; i < 6; i++) de[i] *= ISQ2;
+        int rc = material_update(M.mat_type[e], M.mat_par + 8 * e, M.stressmodel == AMR_PLANESTRESS, s0, s1, de, ds);
+        if (rc) {
+            if (M.part_err) atomicCAS(&M.part_err[M.elem_part[e]], 0, rc);
+            else set_status(status, rc, e);
+            for (int f = 0; f < AMR_NST; f++) s1[f] = s0[f];
+            for (int i = 0; i < 6; i++) ds[i] = 0.0;
+        }
+        for (int f = 0; f < AMR_NST; f++) st[f * M.nip_total + gi] = s1[f];
+        const double coef = G.geo_w[(el0 + el) * nip + ip], cs = coef * ISQ2;
+#pragma unroll
+        for (int i = 0; i < 6; i++) sM[t * 7 + i] = (i < 3 ? coef : cs) * ds[i];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ne * ND; t += kIntThreads) {
+        const int el = t / ND, q = t % ND, c = q % 3;
+        if (elem_skipped(M, e0 + el)) continue;
+        // row c of the symmetric tensor, as places in (11, 22, 33, 23, 13, 12)
+        const int r0 = c == 0 ? 0 : c == 1 ? 5 : 4, r1 = c == 0 ? 5 : c == 1 ? 1 : 3, r2 = c == 0 ? 4 : c == 1 ? 3 : 2;
+        const double *g = G.geo_g + ((el0 + el) * ND + (q - c)) * nip, *m = sM + el * nip * 7;
+        double s = 0.0;
+#pragma unroll 4
+        for (int ip = 0; ip < nip; ip++, m += 7) {
+            s = fma(m[r2], g[2 * nip + ip], fma(m[r1], g[nip + ip], fma(m[r0], g[ip], s)));
+        }
         Fel[M.fel_ptr[e0 + el] + q] = s;
     }
 }
@@ -1475,6 +1539,16 @@ void launch_stiff_ref(amr_model *m, const AmrGroup &g) {
 template <int DIM, int NEN>
 void launch_internal(amr_model *m, const AmrGroup &g, const double *dU) {
     GroupArgs ga{g.tab, g.nip, g.first, g.count, m->geo_valid ? g.geo_g : nullptr, m->geo_valid ? g.geo_w : nullptr};
+    if constexpr (DIM == 3)
+        if (ga.geo_g) {
+            const int epb = g.epb_int > 0 ? g.epb_int : std::max(1, kIntThreads / g.nip);
+            const size_t smem = sizeof(double) * (size_t)epb * (NEN * 3 + g.nip * 7);  // 24 KB at most: TET4, 64 elements
+            internal_cached_kernel<NEN><<<nblk(g.count, epb), kIntThreads, smem, m->stream>>>(
+                margs(m), ga, epb, dU, m->stbk, m->st, m->Fel, m->d_status);
+            AMR_COUNT(1);
+            AMR_CUDA(cudaGetLastError());
+            return;
+        }
     int epb = g.epb_int > 0 ? g.epb_int : ((g.nip >= 16) ? 4 : 16);
     size_t smem = sizeof(double) * (size_t)epb * (2 * NEN * DIM + g.nip * NEN * DIM);
     int threads = std::max(epb * g.nip, epb * NEN * DIM);
