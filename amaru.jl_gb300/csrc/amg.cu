@@ -48,6 +48,11 @@ constexpr int kSweepTile = 32;  // pivots of a step of the dense level's inversi
 
 // row lengths of the dense level's FP64 work matrix (whole tiles) and of its inverse
 inline int64_t dense_ld(int64_t nc) { return (nc + kSweepTile - 1) / kSweepTile * kSweepTile; }
+// doubles of the padded matrix, a step's two panels and two diagonal tiles, the panels' digits and their rows' scales
+constexpr int kDig = 7, kDigRow = kDig * kSweepTile;
+inline size_t sweep_doubles(int64_t ld) {
+    return (size_t)(ld * ld + 2 * ld * kSweepTile + 2 * kSweepTile * kSweepTile + 2 * ld * kDigRow / 4 + 2 * ld);
+}
 inline int64_t inverse_ld(int64_t nc) { return (nc + 3) / 4 * 4; }
 
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -594,10 +599,7 @@ static void amg_build_structure(amr_model *m) {
         H.push_back(std::move(hc));
     }
     if (g->nc > 32768) throw AmrError(AMR_EUNSUPPORTED, "the multigrid's coarsest level is too large to invert densely");
-    {  // the padded matrix, two panels of a sweep step and two diagonal tiles
-        const size_t ld = (size_t)dense_ld(g->nc);
-        amr_alloc(&g->Cd, ld * ld + 2 * ld * kSweepTile + 2 * kSweepTile * kSweepTile);
-    }
+    amr_alloc(&g->Cd, sweep_doubles(dense_ld(g->nc)));  // the padded matrix and a sweep step's panels
     amr_alloc(&g->Cinv, (size_t)g->nc * inverse_ld(g->nc));
     amr_alloc(&g->scratch, 8 + kNormCtas);
     amr_alloc(&g->ticket, 1);
@@ -1347,15 +1349,16 @@ __global__ void k_prolong_sa16(int64_t n, const int64_t *prp, const int32_t *pcj
 // ---------------------------------------------------------------------------
 // Dense coarsest level: the BSR matrix expanded to FP64, inverted by a blocked symmetric sweep, multiplied.
 //
-// The inverse of an SPD matrix of nc rows takes nc^3 / 2 FP64 FMAs when only one triangle is formed, and on this GPU
-// the FP64 pipe (two FMAs a clock per SM) is what bounds it: 61 us of every step's 68 us at nc = 1 428, 3.4 ms in
-// all.  An elimination with one launch per pivot moved the whole augmented matrix through L2 for every pivot:
-// 33.5 ms there (23.5 us a pivot), 3.8 ms at nc = 558 (now 0.9 ms).  Here 32 pivots are taken at a time:
+// The inverse of an SPD matrix of nc rows takes nc^3 / 2 FMAs when only one triangle is formed.  An elimination with one
+// launch per pivot moved the whole augmented matrix through L2 for every pivot: 33.5 ms at nc = 1 428 (23.5 us a pivot),
+// 3.8 ms at nc = 558.  Here 32 pivots are taken at a time:
 //   D = A_kk^-1 (in shared memory), W_i = A_ik D (k_sweep_panel), A_ij -= W_i A_kj for the other tiles of the
 //   lower triangle (k_sweep_update), A_ik = W_i, A_kk = -D;
-// after the last block the triangle holds -A^-1.  A 32 x 32 tile per CTA gives n = 1 332 some 900 tiles a step, six
-// even waves, and every tile is read and written once per 32 pivots.  The CTA that updates the next diagonal tile
-// inverts it in the same launch, beside the other tiles, so a step costs two launches.
+// after the last block the triangle holds -A^-1.  A 32 x 32 tile per CTA gives n = 1 332 some 900 tiles a step, and every
+// tile is read and written once per 32 pivots.  The CTA that updates the next diagonal tile inverts it in the same launch,
+// beside the other tiles, so a step costs two launches.  With the update's products on the FP64 pipe (two FMAs a clock
+// per SM) that pipe bound a step: 61 of 68 us at nc = 1 428, 3.9 ms in all, 0.96 at nc = 558.  From exact slices on the
+// tensor cores it takes 2.25 and 0.74 ms, and the 32 pivots of the next diagonal tile, 28 us a step, bound it.
 //
 // A product with a zero factor is left out, and a tile pair without a nonzero is skipped: the level is block diagonal
 // over the parts of a batch, so a part's non-finite values stay in its own rows and columns, and the zero tiles
@@ -1465,10 +1468,54 @@ __global__ void __launch_bounds__(256) k_sweep_first(const double *C, int64_t ld
     store_inverse(T, D);
 }
 
+// The update's products W_i A_kj are formed on the tensor cores from exact slices (the splitting of Ozaki, Ogita, Oishi and
+// Rump, Numer. Algorithms 59, 2012; on matrix units Mukunoki et al. 2020): each row of W and of A_ik is scaled by a power
+// of two to integers of 55 bits, written as kDig signed digits of 8 bits, which bf16 holds exactly.  A product of two
+// digits has 14 bits, a sum of 32 of them and of the up to seven digit pairs of one weight 22, so the FP32 accumulators
+// are exact; the pairs (s, t), s + t <= kDig + 2, leave out 2^-64 of the rows' largest entries' product, and the weighted
+// sum is rounded once where 32 FP64 FMAs round 32 times.
+struct SweepDigits {
+    uint16_t *W, *P;   // ld rows of bf16 [digit][column]
+    double *ws, *ps;   // ld: 2^(e - 19) for rows of entries below 2^e; 0 for a zero row, NaN for a non-finite one
+};
+inline SweepDigits sweep_digits(double *C, int64_t ld) {
+    uint16_t *d = reinterpret_cast<uint16_t *>(C + ld * ld + 2 * ld * kSw + 2 * kSw * kSw);
+    double *sc = reinterpret_cast<double *>(d + 2 * ld * kDigRow);
+    return {d, d + ld * kDigRow, sc, sc + ld};
+}
+
+// the digits of a row, entry x of column lane on each lane of a warp
+__device__ __forceinline__ void row_digits(double x, uint16_t *dig, double *scale) {
+    const int lane = threadIdx.x & 31;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int ex = (int)(b >> 52 & 0x7ff);
+    const int top = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(ex, 1));
+    const bool any = __any_sync(0xffffffffu, nz(x));
+    unsigned long long mant = b & 0xfffffffffffffULL;
+    if (ex > 0) mant |= 1ULL << 52;
+    const int shift = top - max(ex, 1);  // |x| < 2^(top - 1022)
+    long long q = shift == 0 ? (long long)(mant << 2)
+                             : shift > 56 ? 0 : (long long)(((mant << 2) + (1ULL << (shift - 1))) >> shift);
+    if (b >> 63) q = -q;
+#pragma unroll
+    for (int s = kDig - 1; s >= 0; s--) {
+        const int d = s > 0 ? (int)(signed char)(q & 0xff) : (int)q;
+        q = (q - d) >> 8;
+        dig[s * kSw + lane] = (uint16_t)(__float_as_uint((float)d) >> 16);
+    }
+    if (lane == 0) *scale = !any ? 0.0 : top == 0x7ff ? __longlong_as_double(0x7ff8000000000000LL) : scalbn(1.0, top - 1041);
+}
+
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
 // W_i = A_ik D for 8 rows of a tile row i != k per CTA (four CTAs a tile row), written over A_ik and to Wb, with the old
-// A_ik in Pb; the last CTA writes A_kk = -D.
+// A_ik in Pb, and both as digits; the last CTA writes A_kk = -D.
 __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *C, const double *D, double *Wb,
-                                                     double *Pb) {
+                                                     double *Pb, SweepDigits dg) {
     constexpr int R = 8;
     __shared__ double sA[R][kSw + 1], sD[kSw][kSw + 1];
     if (blockIdx.x == gridDim.x - 1) {
@@ -1502,8 +1549,10 @@ __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *
     const int any = __syncthreads_or(nz(a)), all_finite = __syncthreads_and(fin);
     const int64_t row = (int64_t)i * kSw + r0 + r;
     Pb[row * kSw + q] = sA[r][q];
+    row_digits(sA[r][q], dg.P + row * kDigRow, dg.ps + row);
     if (!any) {  // W_i is zero as A_ik is
         Wb[row * kSw + q] = 0.0;
+        row_digits(0.0, dg.W + row * kDigRow, dg.ws + row);
         return;
     }
     double w = 0.0;
@@ -1515,6 +1564,7 @@ __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *
             if (nz(sA[r][t]) && nz(sD[t][q])) w = fma(sA[r][t], sD[t][q], w);
     }
     Wb[row * kSw + q] = w;
+    row_digits(w, dg.W + row * kDigRow, dg.ws + row);
     if (i > k) {
         C[row * ld + k * kSw + q] = w;
     } else {  // the transpose, written along the rows of the tile (k, i)
@@ -1526,9 +1576,11 @@ __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *
 }
 
 // A_ij -= W_i A_kj for a tile (i, j) of the lower triangle per CTA, i, j != k, m = tile rows - 1; the next diagonal
-// tile is CTA 0's, which also inverts it.
-__global__ void __launch_bounds__(256) k_sweep_update(int64_t ld, int k, int m, double *C, const double *Wb,
-                                                      const double *Pb, double *Dnext) {
+// tile is CTA 0's, which also inverts it.  A warp has 16 x 8 entries.  The columns of a row are taken in the order that
+// gives each lane 16 consecutive bytes of its row's digits (the same order on both sides: the sum runs over them).
+// Rows with a non-finite entry take the products in FP64, zero factors left out.
+__global__ void __launch_bounds__(256, 2) k_sweep_update(int64_t ld, int k, int m, double *C, const double *Wb,
+                                                         const double *Pb, SweepDigits dg, double *Dnext) {
     __shared__ SweepTile T;
     double(*sW)[kSw + 1] = T.S[0], (*sP)[kSw + 1] = T.S[1];
     // tile number t of the compressed triangle (block k left out); number 0 and the next diagonal tile change places
@@ -1546,53 +1598,114 @@ __global__ void __launch_bounds__(256) k_sweep_update(int64_t ld, int k, int m, 
     if (i >= k) i++;
     if (j >= k) j++;
     const bool next = has_next && i == k + 1 && j == k + 1;
-    const int ty = threadIdx.x / kSw, tx = threadIdx.x % kSw;
     double *tile = C + ((int64_t)i * kSw) * ld + (int64_t)j * kSw;
-    double v[4], w[4], p[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        w[u] = Wb[(int64_t)i * kSw * kSw + threadIdx.x + 256 * u];
-        p[u] = Pb[(int64_t)j * kSw * kSw + threadIdx.x + 256 * u];
-        v[u] = tile[(ty + 8 * u) * ld + tx];
-    }
-    bool aw = false, ap = false, fin = true;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        sW[ty + 8 * u][tx] = w[u];
-        sP[ty + 8 * u][tx] = p[u];
-        aw |= nz(w[u]);
-        ap |= nz(p[u]);
-        fin &= finite(w[u]) && finite(p[u]);
-    }
-    const int any_w = __syncthreads_or(aw), any_p = __syncthreads_or(ap), all_finite = __syncthreads_and(fin);
-    const bool work = any_w && any_p;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double wl = dg.ws[(int64_t)i * kSw + lane], pl = dg.ps[(int64_t)j * kSw + lane];
+    const bool all_finite = __all_sync(0xffffffffu, finite(wl) && finite(pl));
+    const bool work = __any_sync(0xffffffffu, nz(wl)) && __any_sync(0xffffffffu, nz(pl));  // (uniform over the CTA)
     if (!work && !next) return;
-    if (work) {
-        if (all_finite) {  // (a zero factor then adds a zero)
-#pragma unroll 4
-            for (int q = 0; q < kSw; q++) {
-                const double x = -sP[tx][q];
+    if (all_finite) {
+        const int r = (warp & 1) * 16 + lane / 4, c = (warp >> 1) * 8 + lane % 4 * 2;  // entries (r, r + 8) x (c, c + 1)
+        double2 v0 = *reinterpret_cast<const double2 *>(tile + r * ld + c);
+        double2 v1 = *reinterpret_cast<const double2 *>(tile + (r + 8) * ld + c);
+        if (work) {
+            const uint4 *a0 = reinterpret_cast<const uint4 *>(dg.W + ((int64_t)i * kSw + r) * kDigRow) + lane % 4;
+            const uint4 *a1 = a0 + 8 * (kDigRow / 8);
+            const uint4 *b0 = reinterpret_cast<const uint4 *>(dg.P + ((int64_t)j * kSw + (warp >> 1) * 8 + lane / 4) * kDigRow) +
+                              lane % 4;
+            uint4 x[kDig], y[kDig];
 #pragma unroll
-                for (int u = 0; u < 4; u++) v[u] = fma(sW[ty + 8 * u][q], x, v[u]);
+            for (int s = 0; s < kDig; s++) {
+                x[s] = a0[s * (kSw / 8)];
+                y[s] = a1[s * (kSw / 8)];
             }
-        } else {
-            for (int q = 0; q < kSw; q++) {
-                const double x = -sP[tx][q];
+            constexpr int NS = kDig + 1;  // weights: digit pairs (s, u), s + u < NS
+            float acc[NS][4];
 #pragma unroll
-                for (int u = 0; u < 4; u++)
-                    if (nz(x) && nz(sW[ty + 8 * u][q])) v[u] = fma(sW[ty + 8 * u][q], x, v[u]);
+            for (int s = 0; s < NS; s++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) acc[s][q] = 0.0f;
+#pragma unroll
+            for (int u = 0; u < kDig; u++) {
+                const uint4 z = b0[u * (kSw / 8)];
+#pragma unroll
+                for (int s = 0; s < kDig; s++)
+                    if (s + u < NS) {
+                        const uint32_t lo[4] = {x[s].x, y[s].x, x[s].y, y[s].y}, hi[4] = {x[s].z, y[s].z, x[s].w, y[s].w};
+                        mma_bf16(acc[s + u], lo, z.x, z.y);
+                        mma_bf16(acc[s + u], hi, z.z, z.w);
+                    }
             }
+            const double w0 = dg.ws[(int64_t)i * kSw + r], w1 = dg.ws[(int64_t)i * kSw + r + 8];
+            const double p0 = dg.ps[(int64_t)j * kSw + c], p1 = dg.ps[(int64_t)j * kSw + c + 1];
+            double sum[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                long long h[2];  // the weights' two halves, integers below 2^47
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    h[g] = 0;
+#pragma unroll
+                    for (int s = 0; s < NS / 2; s++)  // (the bits of acc + 1.5 2^23 hold the integer acc)
+                        h[g] = h[g] * 256 + (__float_as_int(acc[g * (NS / 2) + s][q] + 12582912.0f) - 0x4B400000);
+                }
+                // integers as doubles by 1.5 2^52, whose last place is 1
+                const double H = __longlong_as_double(h[0] + 0x4338000000000000LL) - 6755399441055744.0;
+                const double L = __longlong_as_double(h[1] + 0x4338000000000000LL) - 6755399441055744.0;
+                sum[q] = fma(L, 0x1p-32, H);
+            }
+            v0.x = fma(-(sum[0] * w0), p0, v0.x);
+            v0.y = fma(-(sum[1] * w0), p1, v0.y);
+            v1.x = fma(-(sum[2] * w1), p0, v1.x);
+            v1.y = fma(-(sum[3] * w1), p1, v1.y);
+            *reinterpret_cast<double2 *>(tile + r * ld + c) = v0;
+            *reinterpret_cast<double2 *>(tile + (r + 8) * ld + c) = v1;
+        }
+        if (!next) return;
+        sW[r][c] = v0.x;
+        sW[r][c + 1] = v0.y;
+        sW[r + 8][c] = v1.x;
+        sW[r + 8][c + 1] = v1.y;
+    } else {
+        const int ty = threadIdx.x / kSw, tx = threadIdx.x % kSw;
+        double v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            sW[ty + 8 * u][tx] = Wb[(int64_t)i * kSw * kSw + threadIdx.x + 256 * u];
+            sP[ty + 8 * u][tx] = Pb[(int64_t)j * kSw * kSw + threadIdx.x + 256 * u];
+            v[u] = tile[(ty + 8 * u) * ld + tx];
+        }
+        __syncthreads();
+        for (int q = 0; q < kSw; q++) {
+            const double x = -sP[tx][q];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (nz(x) && nz(sW[ty + 8 * u][q])) v[u] = fma(sW[ty + 8 * u][q], x, v[u]);
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) tile[(ty + 8 * u) * ld + tx] = v[u];
-    }
-    if (!next) return;
-    __syncthreads();
+        if (!next) return;
+        __syncthreads();
 #pragma unroll
-    for (int u = 0; u < 4; u++) sW[ty + 8 * u][tx] = v[u];
+        for (int u = 0; u < 4; u++) sW[ty + 8 * u][tx] = v[u];
+    }
     __syncthreads();
     sweep_tile(T);
     store_inverse(T, Dnext);
+}
+
+// the launches of a whole inversion of C (ld rows, lower triangle; sweep_doubles(ld) in all)
+void sweep_steps(cudaStream_t s, double *C, int64_t ld) {
+    const int nt = (int)(ld / kSw);  // tile rows
+    double *Wb = C + ld * ld, *Pb = Wb + ld * kSw, *Db = Pb + ld * kSw;
+    const SweepDigits dg = sweep_digits(C, ld);
+    k_sweep_first<<<1, 256, 0, s>>>(C, ld, Db);
+    for (int k = 0; k < nt; k++) {
+        double *Dk = Db + (k & 1) * kSw * kSw, *Dn = Db + ((k + 1) & 1) * kSw * kSw;
+        k_sweep_panel<<<(unsigned)(4 * (nt - 1) + 1), 256, 0, s>>>(ld, k, C, Dk, Wb, Pb, dg);
+        const int64_t tiles = (int64_t)(nt - 1) * nt / 2;
+        if (tiles > 0) k_sweep_update<<<(unsigned)tiles, 256, 0, s>>>(ld, k, nt - 1, C, Wb, Pb, dg, Dn);
+    }
 }
 
 // the full inverse from the swept triangle, rows of ldc (padded with zeros)
@@ -1992,7 +2105,6 @@ struct Cycle {
         AmgLevel &D = g->L[nl - 1];
         const int64_t nc = g->nc, ld = dense_ld(nc), ldc = inverse_ld(nc);
         const int nt = (int)(ld / kSw);  // tile rows
-        double *Wb = g->Cd + ld * ld, *Pb = Wb + ld * kSw, *Db = Pb + ld * kSw;
         AMR_CUDA(cudaMemsetAsync(g->Cd, 0, ld * ld * sizeof(double), s));
         k_dense_expand<NM, V><<<(unsigned)D.n, 256, 0, s>>>(D.n, D.rp, D.cj, vals<V>(D).A, D.nbs, g->Cd, ld);
         k_dense_pad<<<1, kSw, 0, s>>>(nc, ld, g->Cd);
@@ -2001,13 +2113,7 @@ struct Cycle {
         if (!g->gj_exec) {
             cudaGraph_t gr = nullptr;
             AMR_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
-            k_sweep_first<<<1, 256, 0, s>>>(g->Cd, ld, Db);
-            for (int k = 0; k < nt; k++) {
-                double *Dk = Db + (k & 1) * kSw * kSw, *Dn = Db + ((k + 1) & 1) * kSw * kSw;
-                k_sweep_panel<<<(unsigned)(4 * (nt - 1) + 1), 256, 0, s>>>(ld, k, g->Cd, Dk, Wb, Pb);
-                const int64_t tiles = (int64_t)(nt - 1) * nt / 2;
-                if (tiles > 0) k_sweep_update<<<(unsigned)tiles, 256, 0, s>>>(ld, k, nt - 1, g->Cd, Wb, Pb, Dn);
-            }
+            sweep_steps(s, g->Cd, ld);
             const cudaError_t ce = cudaStreamEndCapture(s, &gr);
             if (ce == cudaSuccess) {
                 const cudaError_t ie = cudaGraphInstantiate(&g->gj_exec, gr, 0);

@@ -57,3 +57,20 @@ def test_dense_level_of_a_batch_is_block_diagonal():
         ana.addstage(bcs)
         assert ana.solve(solver="amg", linear_rtol=1e-10)[0]
         np.testing.assert_allclose(part.U, m.U, rtol=0, atol=1e-7 * np.abs(m.U).max())
+
+
+@pytest.mark.parametrize("scale", [1e-6, 1e6, 1e22])
+def test_dense_level_at_any_scale(scale):
+    """The inverse's digits and reciprocals follow the matrix's exponents: with all moduli scaled (upwards far; far below
+    1 element entries fall under the assembly's eps and are dropped), the same iterations
+    (one more or less, where the residual passes the tolerance) and the scaled solution (both solved to 1e-10, as
+    above)."""
+    out = []
+    for f in (1.0, scale):
+        model, (U0, F0) = _model(A.HEX8, (13, 5, 4))
+        model.dev.set_youngs(f * model.mat_params[:, 0])
+        model.dev.assemble_K()
+        U, _, st = model.dev.solve(U0, F0 * f, A._lib.default_solve_opts(method=A._lib.SOLVER_AMG, rtol=1e-10))
+        out.append((U, st.iterations))
+    assert abs(out[0][1] - out[1][1]) <= 1
+    assert np.abs(out[1][0] - out[0][0]).max() <= 1e-7 * np.abs(out[0][0]).max()
