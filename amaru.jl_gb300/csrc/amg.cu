@@ -789,19 +789,25 @@ __global__ void __launch_bounds__(128) k_sa_ap(int64_t nq, const int32_t *qrow, 
     for (int u = 0; u < BF * NM; u++) o[u] = acc[u];
 }
 
-// coarse operator P' (A P), thread per coarse block (I, J): sum over the fine rows i that P reaches I from
-// (block s), in order, of P_s' Q_iJ (if row i of A P has column J)
+// coarse operator P' (A P), kGalLanes lanes per coarse block (I, J): sum over the fine rows i that P reaches I from
+// (block s) of P_s' Q_iJ (if row i of A P has column J), the lanes' sums added in a fixed order.  Bound by the latency of
+// the search in row i: a thread per block walked some 200 rows one after another
+// (HEX20 100 x 40 x 40: the second level's operator 1.53 ms, now 0.24; the first level's, enough blocks for every thread,
+// 4.1 and 4.35).
+constexpr int kGalLanes = 8;
 template <int BF, int NM, class V>
 __global__ void k_sa_galerkin(int64_t ncb, const int32_t *crow, const int32_t *ccj, const int64_t *ptp,
                               const int32_t *pti, const int32_t *pts, const V *P, const int64_t *qrp,
                               const int32_t *qcj, const V *Q, V *Ac, int64_t nbsc) {
-    const int64_t cb = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (cb >= ncb) return;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, cb = t / kGalLanes;
+    const int lane = (int)(t % kGalLanes);
+    if (cb >= ncb) return;  // (uniform over a block's lanes)
+    const unsigned mask = ((1u << kGalLanes) - 1) << ((threadIdx.x & 31) / kGalLanes * kGalLanes);
     const int32_t I = crow[cb], J = ccj[cb];
     V acc[NM * NM];
 #pragma unroll
     for (int u = 0; u < NM * NM; u++) acc[u] = V(0);
-    for (int64_t e = ptp[I]; e < ptp[I + 1]; e++) {
+    for (int64_t e = ptp[I] + lane; e < ptp[I + 1]; e += kGalLanes) {
         const int64_t i = pti[e];
         int64_t lo = qrp[i], hi = qrp[i + 1];  // J in the sorted columns of row i of A P
         while (lo < hi) {
@@ -823,7 +829,12 @@ __global__ void k_sa_galerkin(int64_t ncb, const int32_t *crow, const int32_t *c
         }
     }
 #pragma unroll
-    for (int u = 0; u < NM * NM; u++) Ac[(int64_t)u * nbsc + cb] = acc[u];
+    for (int o = kGalLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < NM * NM; u++) acc[u] += __shfl_xor_sync(mask, acc[u], o);
+#pragma unroll
+    for (int u = 0; u < NM * NM; u++)
+        if (u % kGalLanes == lane) Ac[(int64_t)u * nbsc + cb] = acc[u];
 }
 
 // The FP32 cycle's prolongator rounded to FP16 (saturated at the FP16 range): P16 by rows, P16T by columns
@@ -2066,7 +2077,7 @@ struct Cycle {
         }
         k_sa_ap<BF, NM, V><<<grid(F.nq), 128, 0, s>>>(F.nq, F.qrow, F.qcj, F.rp, F.cj, A, nbs, F.prp, F.pcj,
                                                             fv.P, fv.Q, F.p_steps);
-        k_sa_galerkin<BF, NM, V><<<grid(C.nblocks), 128, 0, s>>>(C.nblocks, F.crow, C.cj, F.ptp, F.pti, F.pts,
+        k_sa_galerkin<BF, NM, V><<<grid(C.nblocks * kGalLanes), 128, 0, s>>>(C.nblocks, F.crow, C.cj, F.ptp, F.pti, F.pts,
                                                                        fv.P, F.qrp, F.qcj, fv.Q, cv.A, C.nbs);
         AMR_COUNT(3);
     }
