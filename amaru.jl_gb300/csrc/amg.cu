@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(128) k_sa_ap(int64_t nq, const int32_t *qrow, 
 // coarse operator P' (A P), kGalLanes lanes per coarse block (I, J): sum over the fine rows i that P reaches I from
 // (block s) of P_s' Q_iJ (if row i of A P has column J), the lanes' sums added in a fixed order.  Bound by the latency of
 // the search in row i: a thread per block walked some 200 rows one after another
-// (HEX20 100 x 40 x 40: the second level's operator 1.53 ms, now 0.24; the first level's, enough blocks for every thread,
+// (TET10 24 x 5 x 10: 461 us, now 84; HEX20 100 x 40 x 40: the second level's operator 1.53 ms, now 0.24; the first level's, enough blocks for every thread,
 // 4.1 and 4.35).
 constexpr int kGalLanes = 8;
 template <int BF, int NM, class V>

@@ -848,7 +848,7 @@ struct AmrRecovery {
     int nf = 0, nmask = 0, m_max = 1, e_max = 1;
     std::vector<int32_t> codes;      // output field codes, reference order
     int64_t ntasks = 0, nslots = 0, ncontrib = 0;
-    double fit_flops = 0.0;          // FP64 operations of one fit, its sums taken over each patch's points
+    double fit_flops = 0.0;          // FP64 operations of one fit (its three kernels)
     int64_t n_svd = 0;               // tasks on the SVD path (known after a launch)
     // device
     double *ipx = nullptr, *ipv = nullptr, *vst = nullptr;
@@ -984,8 +984,16 @@ void build(amr_model *m) {
     std::vector<int64_t> t_elem_ptr{0}, t_node_ptr{0};
     std::vector<int32_t> t_elem, t_node, t_mask, t_center, t_m;
     std::vector<int64_t> stamp(nn, -1);
-    const int nt_max = m->ndim == 3 ? 7 : 6;
-    double flops = 0.0;
+    const bool moments = by_elements(m);
+    // FP64 operations: the elements' sums of monomials and moments; translating and adding one element's monomials
+    const int nm = m->ndim == 3 ? kMono<3> : kMono<2>;
+    double flops = (double)m->nip_total * (nm + (moments ? 2.0 * (m->ndim == 3 ? kTerms<3> : kTerms<2>) * R->nf : 0.0));
+    double mono_ops = nm;
+    for (int i = 0; i < nm; i++)
+        for (int d = 0; d < m->ndim; d++) {
+            const int a = m->ndim == 3 ? mono_exp<3>(i, d) : mono_exp<2>(i, d);
+            mono_ops += a * (a + 1);  // a (a + 1) / 2 FMA
+        }
     for (int64_t n = 0; n < nn; n++) {
         if (!src[n]) continue;
         const int32_t *pb = src[n] == 1 ? &ip_list[ip_cnt[n]] : &bp_list[bp_cnt[n]];
@@ -1015,9 +1023,10 @@ void build(amr_model *m) {
             const int nt = m->ndim == 3 ? (mcount >= 7 ? 7 : mcount >= 4 ? 4 : 1)
                                         : (mcount >= 6 ? 6 : mcount >= 4 ? 4 : mcount >= 3 ? 3 : 1);
             const double nnod = (double)(t_node_ptr.back() - t_node_ptr[t_node_ptr.size() - 2]);
-            // Gram (nt(nt+1)/2 FMA per IP), moments (nt per IP and field), node values (nt per node and field)
-            flops += 2.0 * mcount * (nt * (nt + 1) / 2) + 2.0 * mcount * nt * mask_nf[mk] + 2.0 * nnod * nt * mask_nf[mk];
-            (void)nt_max;
+            // per element of the patch the translated monomials and moments (or nt FMA per IP and field), per node and
+            // field nt - 1 FMA
+            flops += ecount * mono_ops + (moments ? ecount * (m->ndim == 3 ? 25.0 : 20.0) : 2.0 * mcount * nt) * mask_nf[mk] +
+                     2.0 * nnod * (nt - 1) * mask_nf[mk];
         }
     }
     R->fit_flops = flops;
