@@ -266,6 +266,10 @@ struct AmrResidentShape {
 AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer, bool exact);
 size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s);  // of a slice of these sizes
 size_t amr_resident_max_bytes();
+// for tests: the shape of a model alone with this block pattern on a device of clusters of up to `most` CTAs; returns the
+// CTAs, their bounds (ctas + 1 values) and the shared memory of the largest slice.  Host only.
+extern "C" int amr_test_resident_shape(int32_t ndim, int64_t nnodes, const int64_t *row_ptr, const int32_t *col,
+                                       int64_t prefer, int32_t exact, int32_t most, int64_t *bounds, int64_t *bytes);
 // solves the parts list[0..nparts) (null: part 0) on `stream`: part p's slice bounds at slices[first[p]] (null: 0), the
 // slices' row orders in perm (per node of the model); x
 // (in: prescribed values, initial guess), b, reac node-major FP64; rows64: 2 x nnodes of scratch (exact shapes); stat per part; t0 / t1 (may be null) the

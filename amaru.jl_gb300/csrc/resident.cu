@@ -823,26 +823,33 @@ int device_cluster() {
 
 }  // namespace
 
+static size_t resident_bytes(int B, const AmrResidentShape &s) {
+    return B == 3 ? slice_bytes<3>(s.slots, s.rows, s.window) : slice_bytes<2>(s.slots, s.rows, s.window);
+}
+
 // The cluster size that solves nodes [P0, P1), and the largest slice: the smallest whose slices stay within `prefer`
 // bytes of shared memory, else the largest the device takes if its slices fit at all; 0: none.
-AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer, bool exact) {
+static AmrResidentShape shape_of(const int64_t *rp, const int32_t *col, int B, int64_t P0, int64_t P1, size_t prefer,
+                                 bool exact, int most) {
     AmrResidentShape best;
-    const int most = device_cluster();
     const int64_t len = P1 - P0;
     if (most == 0 || len <= 0 || len > (int64_t)most * 65535) return best;
-    const std::vector<int64_t> &rp = m->h_brow_ptr;
     std::vector<int64_t> place;
     for (int C = 1; C <= most; C *= 2) {
+        if (exact && (len - 1) / 64 < C - 1) break;  // fewer groups of 64 rows than CTAs
         AmrResidentShape s;
         s.ctas = C;
         s.bounds.resize(C + 1);
         for (int r = 0; r <= C; r++)
             s.bounds[r] = r == 0   ? P0
                           : r == C ? P1
-                                   : std::lower_bound(rp.begin() + P0, rp.begin() + P1, rp[P0] + (rp[P1] - rp[P0]) * r / C) -
-                                         rp.begin();
-        if (exact)  // whole groups of 64 rows
-            for (int r = 1; r < C; r++) s.bounds[r] = std::min(P1, P0 + (s.bounds[r] - P0 + 32) / 64 * 64);
+                                   : std::lower_bound(rp + P0, rp + P1, rp[P0] + (rp[P1] - rp[P0]) * r / C) - rp;
+        if (exact)
+            // Whole groups of 64 rows, one at least: a CTA's part in a sum is the sums of its rows, so one without rows
+            // sends nothing, no other CTA waits for it, and they could write the next sum over the one that it reads.
+            for (int r = 1; r < C; r++)
+                s.bounds[r] = std::min(std::max(P0 + (s.bounds[r] - P0 + 32) / 64 * 64, s.bounds[r - 1] + 64),
+                                       P0 + ((len - 1) / 64 - (C - 1 - r)) * 64);
         s.exact = exact;
         s.perm.resize(len);
         // a row's blocks, or with `exact` its runs of four blocks from a multiple of four
@@ -864,7 +871,7 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
         if (s.rows > (exact ? kT * kRowsPerThread : 65535) || most_rows > kT * kRowsPerThread) continue;
         least.rows = s.rows;
         least.exact = exact;
-        if (amr_resident_bytes(m, least) > (exact ? kMaxDynExact : kMaxDyn)) continue;
+        if (resident_bytes(B, least) > (exact ? kMaxDynExact : kMaxDyn)) continue;
         for (int r = 0; r < C; r++) {  // each slice's rows by falling width, equal ones in their order
             const int64_t n0 = s.bounds[r], n1 = s.bounds[r + 1];
             uint16_t *pm = s.perm.data() + (n0 - P0);
@@ -890,8 +897,8 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
             int64_t lo = n0, hi = n1, slots = 0;
             for (int64_t n = n0; n < n1; n++)
                 if (rp[n + 1] > rp[n]) {  // a row's columns ascend
-                    lo = std::min<int64_t>(lo, m->h_bcol[rp[n]]);
-                    hi = std::max<int64_t>(hi, m->h_bcol[rp[n + 1] - 1] + 1);
+                    lo = std::min<int64_t>(lo, col[rp[n]]);
+                    hi = std::max<int64_t>(hi, col[rp[n + 1] - 1] + 1);
                 }
             for (int64_t i = 0; i < n1 - n0; i += 32 / S) {  // the rows of a warp: the first is the longest
                 slots += 32 * (exact ? 4 : 1) * ((width(n0 + pm[i]) + S - 1) / S);
@@ -901,7 +908,7 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
             fits = s.window < 65536;
         }
         if (!fits) continue;
-        s.bytes = amr_resident_bytes(m, s);
+        s.bytes = resident_bytes(B, s);
         if (s.bytes > (exact ? kMaxDynExact : kMaxDyn)) continue;
         best = s;
         if (s.bytes <= prefer) break;
@@ -909,9 +916,19 @@ AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, 
     return best;
 }
 
-size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s) {
-    return m->B == 3 ? slice_bytes<3>(s.slots, s.rows, s.window) : slice_bytes<2>(s.slots, s.rows, s.window);
+AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer, bool exact) {
+    return shape_of(m->h_brow_ptr.data(), m->h_bcol.data(), m->B, P0, P1, prefer, exact, device_cluster());
 }
+
+int amr_test_resident_shape(int32_t ndim, int64_t nnodes, const int64_t *row_ptr, const int32_t *col, int64_t prefer,
+                            int32_t exact, int32_t most, int64_t *bounds, int64_t *bytes) {
+    const AmrResidentShape s = shape_of(row_ptr, col, ndim == 3 ? 3 : 2, 0, nnodes, (size_t)prefer, exact != 0, most);
+    std::copy(s.bounds.begin(), s.bounds.end(), bounds);
+    *bytes = (int64_t)s.bytes;
+    return s.ctas;
+}
+
+size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s) { return resident_bytes(m->B, s); }
 size_t amr_resident_max_bytes() { return kMaxDyn; }
 
 void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
