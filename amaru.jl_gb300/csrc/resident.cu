@@ -231,6 +231,9 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     if (a.active && !a.active[part]) return;  // (uniform over the cluster)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (a.t0 && tid == 0) atomicMin(a.t0, global_ns());
+    // Another CTA's shared memory may be touched only once that CTA runs: all arrive here and wait before the first remote
+    // store below, so that the set-up of the slice hides the wait.
+    if (C > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     auto barrier = [&]() {
         if (C > 1) cl.sync();
         else __syncthreads();
@@ -344,6 +347,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     }
 
     // every CTA's window; the ranks (bits) whose windows hold a row of this thread
+    if (C > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     if (tid < C) {
         *cl.map_shared_rank(&s_win[rank][0], tid) = w0;
         *cl.map_shared_rank(&s_win[rank][1], tid) = w0 + W;
