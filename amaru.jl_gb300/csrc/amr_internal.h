@@ -245,6 +245,11 @@ struct AmrSolveResult {
     int iterations, refinements;
     double rel_residual, seconds;
 };
+// what a failed solve's status says
+inline const char *amr_solve_failure(int status) {
+    return status == AMR_ETIMEOUT ? "solve_system!: a wait between the thread blocks of a solve gave up"
+                                  : "solve_system!: Krylov solver did not converge";
+}
 // Solves K11 x1 = b1 - K12 x2 on node-major device vectors: x (in: prescribed values at
 // prescribed slots; out: free slots), b (free slots), reac (out: K x at prescribed slots).
 AmrSolveResult amr_solve_device(amr_model *m, double *x, const double *b, double *reac, const amr_solve_opts &o);
@@ -263,6 +268,11 @@ struct AmrResidentShape {
     std::vector<int64_t> bounds;               // the slices' node ranges, ctas + 1 bounds
     std::vector<uint16_t> perm;                // per node, slice by slice: its rows by descending length, stable
 };
+// Shared memory a CTA's slice should stay within when a cluster of fewer CTAs would also do, for a model alone: fewer
+// CTAs mean shorter sums, smaller slices a shorter product.  An elastoplastic stage of 1 613 QUAD8 nodes (14 000
+// iterations) took 51.0 ms with 100 KB, 54.5 ms with 48 KB and 57.9 ms with all 206 KB; a stage of 525 HEX8 nodes 3.0 ms
+// with 24 to 100 KB and 3.2 ms with 206 KB.
+constexpr size_t kAmrSliceSingle = 100 * 1024;
 AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer, bool exact);
 size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s);  // of a slice of these sizes
 size_t amr_resident_max_bytes();
@@ -270,6 +280,10 @@ size_t amr_resident_max_bytes();
 // CTAs, their bounds (ctas + 1 values) and the shared memory of the largest slice.  Host only.
 extern "C" int amr_test_resident_shape(int32_t ndim, int64_t nnodes, const int64_t *row_ptr, const int32_t *col,
                                        int64_t prefer, int32_t exact, int32_t most, int64_t *bounds, int64_t *bytes);
+// for tests: the one-launch solve of the assembled model, of whose CTAs `rank` never sends its part of a sum, with waits
+// of limit_ms; status: every CTA's (16 at most)
+extern "C" int amr_test_resident_wait(amr_model *m, int32_t exact, int32_t rank, double limit_ms, int32_t *status,
+                                      int32_t *ctas);
 // solves the parts list[0..nparts) (null: part 0) on `stream`: part p's slice bounds at slices[first[p]] (null: 0), the
 // slices' row orders in perm (per node of the model); x
 // (in: prescribed values, initial guess), b, reac node-major FP64; rows64: 2 x nnodes of scratch (exact shapes); stat per part; t0 / t1 (may be null) the

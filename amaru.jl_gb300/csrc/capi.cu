@@ -764,7 +764,7 @@ int amr_solve(amr_model *m, double *U, double *F, const amr_solve_opts *opts, am
             stats->rel_residual = r.rel_residual;
             stats->seconds = r.seconds;
         }
-        if (r.status) throw AmrError(r.status, "solve_system!: Krylov solver did not converge (relative residual " + std::to_string(r.rel_residual) + ")");
+        if (r.status) throw AmrError(r.status, std::string(amr_solve_failure(r.status)) + " (relative residual " + std::to_string(r.rel_residual) + ")");
         double umax = amr_norm_inf(m, x, m->free_mask);
         if (std::isnan(umax) || std::isinf(umax)) throw AmrError(AMR_ENAN, "solve_system!: NaN values in the solution");
         if (umax > 1e8) throw AmrError(AMR_ESINGULAR, "solve_system!: Possible syngular matrix");
@@ -1171,7 +1171,7 @@ int amr_stage_device(amr_model *m, const double *Uex, const double *Fex, const a
                 AmrSolveResult sr = amr_solve_device(m, dUitr, Rtr, reac, p.linear);
                 st.krylov_iterations += sr.iterations;
                 st.solve_seconds += sr.seconds;
-                if (sr.status) { syserror = true; sysmsg = "solve_system!: Krylov solver did not converge"; break; }
+                if (sr.status) { syserror = true; sysmsg = amr_solve_failure(sr.status); break; }
                 double umax = amr_norm_inf(m, dUitr, m->free_mask);
                 if (!(umax <= 1e8)) { syserror = true; sysmsg = "solve_system!: Possible syngular matrix"; break; }
                 // restore states (update reads the committed copy) and update
@@ -1194,7 +1194,7 @@ int amr_stage_device(amr_model *m, const double *Uex, const double *Fex, const a
                     AmrSolveResult sc = amr_solve_device(m, dUi, Rtr, reac, p.linear);
                     st.krylov_iterations += sc.iterations;
                     st.solve_seconds += sc.seconds;
-                    if (sc.status) { syserror = true; sysmsg = "solve_system!: Krylov solver did not converge"; break; }
+                    if (sc.status) { syserror = true; sysmsg = amr_solve_failure(sc.status); break; }
                     double um = amr_norm_inf(m, dUi, m->free_mask);
                     if (!(um <= 1e8)) { syserror = true; sysmsg = "solve_system!: Possible syngular matrix"; break; }
                     vec(m, V_SET_AXPBY, 1.0, dUa, 1.0, dUi, dUt);

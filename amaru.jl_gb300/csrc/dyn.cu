@@ -250,7 +250,7 @@ int amr_dyn_stage_device(amr_model *m, const double *U0, const double *U1, const
             AmrSolveResult sr = amr_solve_device(m, A, Fex, reac, p.linear);
             st.krylov_iterations += sr.iterations;
             st.solve_seconds += sr.seconds;
-            if (sr.status) throw AmrError(AMR_ENOCONV, "initial accelerations: Krylov solver did not converge");
+            if (sr.status) throw AmrError(sr.status, std::string("initial accelerations: ") + amr_solve_failure(sr.status));
         }
         k_dyn_merge<<<blocks(n), kThreads, 0, s>>>(n, m->free_mask, Fex, reac, F);
         AMR_COUNT(1);

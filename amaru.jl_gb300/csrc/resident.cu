@@ -71,7 +71,11 @@ struct Args {
     double tol2;
     int max_iters, force_every;
     int kcap, wcap;                  // slots of blocks and window nodes of a slice at most
+    unsigned long long wait_ns;      // a wait for a sum gives up after this time
+    int withhold;                    // tests: the rank that never sends its part of p.q, and every rank reports its status
+                                     // at stat[rank] (-1: none)
 };
+constexpr unsigned long long kWaitNs = 2000000000ull;  // a sum takes microseconds
 
 // a value hi + lo of two FP32 numbers
 struct Pair {
@@ -117,9 +121,11 @@ __device__ __forceinline__ void store_async(uint32_t to, float v, uint32_t bar) 
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(to), "f"(v), "r"(bar)
                  : "memory");
 }
-// waits for the phase of an mbarrier to complete; false after a limit far above any wait here
-__device__ __forceinline__ bool wait_phase(uint32_t bar, unsigned parity) {
-    for (int i = 0; i < (1 << 20); i++) {
+// waits for the phase of an mbarrier to complete; false after `limit` nanoseconds (a try may suspend the thread for a time
+// that the device sets, so tries alone would not bound it)
+__device__ __forceinline__ bool wait_phase(uint32_t bar, unsigned parity, unsigned long long limit) {
+    unsigned long long start = 0;
+    for (int i = 0; i < (1 << 28); i++) {
         uint32_t done;
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
                      "selp.u32 %0, 1, 0, p;\n}"
@@ -127,6 +133,11 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, unsigned parity) {
                      : "r"(bar), "r"(parity)
                      : "memory");
         if (done) return true;
+        if (i % 16 == 15) {
+            const unsigned long long now = global_ns();
+            if (!start) start = now;
+            else if (now - start > limit) break;
+        }
     }
     return false;
 }
@@ -224,7 +235,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     __shared__ float s_slot[2][2][kMaxC];   // the cluster's partials of the two sums
     __shared__ double s_slotd[2][kMaxC], s_dwarp[2][kW], s_dtot[2], s_um[kMaxC];
     __shared__ __align__(8) uint64_t s_bar[2];                      // the two sums' arrivals
-    __shared__ int s_w0, s_w1, s_win[kMaxC][2], s_bytes;
+    __shared__ int s_w0, s_w1, s_win[kMaxC][2], s_bytes, s_abort;
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const long long part = a.list ? a.list[blockIdx.x / C] : 0;
@@ -253,7 +264,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     if (tid == 0) {
         s_w0 = (int)n0;
         s_w1 = (int)n1;
-        s_bytes = 0;
+        s_bytes = s_abort = 0;
         for (int i = 0; i < 2; i++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_addr(&s_bar[i])), "r"(1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -388,7 +399,11 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     const uint32_t slot_to = cluster_addr(shared_addr(&s_slot[0][half][rank]), min(hl, C - 1)),
                    bar_to = cluster_addr(shared_addr(&s_bar[0]), min(hl, C - 1));
     unsigned parity = 0;  // bit i: the phase of s_bar[i] to wait for
+    // A wait that gives up: this thread goes on, with values that mean nothing but stay in bounds, to the iteration's next
+    // __syncthreads_or, where its CTA leaves the loop as one.  The others learn of it (s_abort) at the next barrier of the
+    // cluster, before they store into another CTA again, and none has left by then.
     bool timeout = false;
+    const int senders = rank == a.withhold ? 0 : C;
     // the cluster's sums of v0 (and v1, with two), the same pairs in every thread; set: the slots used.  Two sums share
     // their steps, one in each half of a warp.
     auto cluster_sum = [&](auto two, int set, float v0, float v1, Pair &o0, Pair &o1) {
@@ -404,12 +419,12 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             t = s_warp[two_sums ? lane : hl];
 #pragma unroll
             for (int o = kW / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (hl < C && (two_sums || half == 0)) store_async(slot_to + set * 2 * kMaxC * 4, t, bar_to + set * 8);
+            if (hl < (two_sums ? C : senders) && (two_sums || half == 0)) store_async(slot_to + set * 2 * kMaxC * 4, t, bar_to + set * 8);
             if (lane == 0)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(&s_bar[set])),
                              "r"(two_sums ? bytes2 : C * 4) : "memory");
         }
-        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u);
+        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u, a.wait_ns);
         parity ^= 1u << set;
         Pair p{hl < C ? s_slot[set][two_sums ? half : 0][hl] : 0.0f, 0.0f};
 #pragma unroll
@@ -445,13 +460,13 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
                 t += __shfl_xor_sync(0xffffffffu, t, 8);
                 t += __shfl_xor_sync(0xffffffffu, t, 4);
             }
-            if (hl < C && (two_sums || half == 0))
+            if (hl < (two_sums ? C : senders) && (two_sums || half == 0))
                 store_async(cluster_addr(shared_addr(&s_grp[two_sums ? 1 + half : 0][g0 + g]), hl), t, bar_to + set * 8);
         }
         if (tid == 0)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(&s_bar[set])),
                          "r"(two_sums ? s_bytes + 8 * groups : 4 * groups) : "memory");
-        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u);
+        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u, a.wait_ns);
         parity ^= 1u << set;
     };
     auto lane_pair = [&](Pair p, int o) {
@@ -669,9 +684,8 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
         } else {
             cluster_sum(std::false_type(), 0, dot, 0.0f, pq, pq);
         }
-        if (timeout) { status = AMR_ETIMEOUT; break; }
-        if (!(pq.h > 0.0f)) { status = AMR_ENOCONV; break; }
-        const float alpha = pair_div(gam, pq);
+        const bool broken = !(pq.h > 0.0f);  // ends the solve below, where the CTA knows of waits that gave up
+        const float alpha = broken ? 0.0f : pair_div(gam, pq);
         // x += alpha p ; r -= alpha q ; z = Minv r
         float v0 = 0.0f, v1 = 0.0f;
 #pragma unroll
@@ -717,7 +731,8 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
         } else {
             cluster_sum(std::true_type(), 1, v0, v1, t2[0], t2[1]);
         }
-        if (timeout) { status = AMR_ETIMEOUT; break; }
+        if (__syncthreads_or(timeout)) { status = AMR_ETIMEOUT; break; }
+        if (broken) { status = AMR_ENOCONV; break; }
         beta = pair_div(t2[0], gam);
         gam = t2[0];
         iters++;
@@ -738,6 +753,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             }
             __threadfence();
             barrier();
+            if (__syncthreads_or(s_abort)) { status = AMR_ETIMEOUT; break; }
             residual64(rz64, rr_true);
             gam = split(rz64);
             thr = threshold();
@@ -747,6 +763,9 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             if (rr_true <= a.tol2 * bnorm2) done = true;
         }
     }
+    if (status == AMR_ETIMEOUT && tid < C) *cl.map_shared_rank(&s_abort, tid) = 1;  // (every CTA is still there)
+    barrier();
+    const bool aborted = __syncthreads_or(s_abort);  // from here on no store into another CTA
     // the largest |x| at free slots (NaN as +inf), and the part's statistics
     double um = 0.0;
     for (int64_t i = n0 * B + tid; i < n1 * B; i += kT)
@@ -761,11 +780,14 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     __syncthreads();
     if (tid == 0) {
         for (int w = 1; w < kW; w++) um = fmax(um, s_dwarp[0][w]);
-        *cl.map_shared_rank(&s_um[rank], 0) = um;
+        if (!aborted) *cl.map_shared_rank(&s_um[rank], 0) = um;
     }
     barrier();  // (also: no CTA leaves while a neighbour may read its shared memory)
-    if (rank == 0 && tid == 0) {
-        for (int r = 0; r < C; r++) um = fmax(um, s_um[r]);
+    if (a.withhold >= 0 && tid == 0) a.stat[rank].status = aborted ? AMR_ETIMEOUT : status;
+    else if (rank == 0 && tid == 0) {
+        if (aborted) status = AMR_ETIMEOUT;
+        else
+            for (int r = 0; r < C; r++) um = fmax(um, s_um[r]);
         AmrPartStat s;
         s.iters = iters;
         s.refreshes = refreshes;
@@ -935,16 +957,7 @@ int amr_test_resident_shape(int32_t ndim, int64_t nnodes, const int64_t *row_ptr
 size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s) { return resident_bytes(m->B, s); }
 size_t amr_resident_max_bytes() { return kMaxDyn; }
 
-void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
-                         const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active, const double *b, double *x, double *reac,
-                         double *rows64, AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1,
-                         double tol2, int max_iters, int force_every, cudaStream_t stream) {
-    if (nparts <= 0) return;
-    Args a;
-    a.slices = slices; a.first = first; a.perm = perm; a.list = list; a.active = active; a.nb = m->bstride; a.rp = m->brow_ptr; a.cj = m->bcol;
-    a.K32 = m->K32; a.K64 = m->K64; a.Minv = m->Minv32; a.fm = m->free_mask; a.b = b; a.x = x; a.reac = reac;
-    a.rows64 = rows64; a.nnodes = m->nnodes; a.stat = stat; a.t0 = t0; a.t1 = t1; a.tol2 = tol2; a.max_iters = max_iters; a.force_every = force_every;
-    a.kcap = (int)shape.slots; a.wcap = (int)shape.window;
+static void launch(int B, const AmrResidentShape &shape, int64_t nparts, const Args &a, cudaStream_t stream) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -956,8 +969,85 @@ void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t np
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    auto kernel = m->B == 3 ? (shape.exact ? k_resident_pcg<3, true> : k_resident_pcg<3, false>)
-                            : (shape.exact ? k_resident_pcg<2, true> : k_resident_pcg<2, false>);
+    auto kernel = B == 3 ? (shape.exact ? k_resident_pcg<3, true> : k_resident_pcg<3, false>)
+                         : (shape.exact ? k_resident_pcg<2, true> : k_resident_pcg<2, false>);
     AMR_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
     AMR_COUNT(1);
+}
+
+static Args args_of(const amr_model *m, const AmrResidentShape &shape, const int64_t *slices, const uint16_t *perm,
+                    const double *b, double *x, double *reac, double *rows64, AmrPartStat *stat) {
+    Args a{};
+    a.slices = slices; a.perm = perm;
+    a.nb = m->bstride; a.rp = m->brow_ptr; a.cj = m->bcol; a.K32 = m->K32; a.K64 = m->K64; a.Minv = m->Minv32;
+    a.fm = m->free_mask; a.b = b; a.x = x; a.reac = reac; a.rows64 = rows64; a.nnodes = m->nnodes; a.stat = stat;
+    a.kcap = (int)shape.slots; a.wcap = (int)shape.window;
+    a.wait_ns = kWaitNs;
+    a.withhold = -1;
+    return a;
+}
+
+void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
+                         const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active, const double *b, double *x, double *reac,
+                         double *rows64, AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1,
+                         double tol2, int max_iters, int force_every, cudaStream_t stream) {
+    if (nparts <= 0) return;
+    Args a = args_of(m, shape, slices, perm, b, x, reac, rows64, stat);
+    a.first = first; a.list = list; a.active = active; a.t0 = t0; a.t1 = t1;
+    a.tol2 = tol2; a.max_iters = max_iters; a.force_every = force_every;
+    launch(m->B, shape, nparts, a, stream);
+}
+
+// A cluster whose rank `rank` withholds its part of p.q, with waits of limit_ns at most: every CTA's status.
+static void withheld_sum(amr_model *m, bool exact, int rank, unsigned long long limit_ns, std::vector<int32_t> &status) {
+    const AmrResidentShape shape = amr_resident_shape(m, 0, m->nnodes, exact ? kAmrSliceSingle : kMaxDyn, exact);
+    if (!m->K_valid || !shape.ctas || rank < 0 || rank >= shape.ctas)
+        throw AmrError(AMR_EINVAL, "no such CTA in the one-launch solve of this model");
+    const int64_t n = m->nnodes * m->B;
+    struct Scratch {
+        int64_t *slices = nullptr;
+        uint16_t *perm = nullptr;
+        double *rows64 = nullptr, *b = nullptr, *x = nullptr, *reac = nullptr;
+        AmrPartStat *stat = nullptr;
+        ~Scratch() {
+            amr_free(slices); amr_free(perm); amr_free(rows64); amr_free(b); amr_free(x); amr_free(reac); amr_free(stat);
+        }
+    } w;
+    amr_alloc(&w.slices, shape.bounds.size());
+    amr_alloc(&w.perm, shape.perm.size());
+    amr_alloc(&w.rows64, 2 * m->nnodes);
+    amr_alloc(&w.b, n);
+    amr_alloc(&w.x, n);
+    amr_alloc(&w.reac, n);
+    amr_alloc(&w.stat, shape.ctas);
+    const std::vector<double> ones(n, 1.0);
+    amr_h2d(m, w.slices, shape.bounds.data(), shape.bounds.size() * sizeof(int64_t));
+    amr_h2d(m, w.perm, shape.perm.data(), shape.perm.size() * sizeof(uint16_t));
+    amr_h2d(m, w.b, ones.data(), n * sizeof(double));
+    AMR_CUDA(cudaMemsetAsync(w.x, 0, n * sizeof(double), m->stream));
+    AMR_CUDA(cudaMemsetAsync(w.stat, 0, shape.ctas * sizeof(AmrPartStat), m->stream));
+    Args a = args_of(m, shape, w.slices, w.perm, w.b, w.x, w.reac, w.rows64, w.stat);
+    a.tol2 = 1e-20; a.max_iters = 1000; a.force_every = 512; a.wait_ns = limit_ns; a.withhold = rank;
+    launch(m->B, shape, 1, a, m->stream);
+    std::vector<AmrPartStat> st(shape.ctas);
+    amr_d2h(m, st.data(), w.stat, st.size() * sizeof(AmrPartStat));
+    status.clear();
+    for (const AmrPartStat &s : st) status.push_back(s.status);
+}
+
+int amr_test_resident_wait(amr_model *m, int32_t exact, int32_t rank, double limit_ms, int32_t *status, int32_t *ctas) {
+    try {
+        AmrStreamScope scope(m->stream);
+        std::vector<int32_t> st;
+        withheld_sum(m, exact != 0, rank, (unsigned long long)(limit_ms * 1e6), st);
+        std::copy(st.begin(), st.end(), status);
+        *ctas = (int32_t)st.size();
+        return AMR_OK;
+    } catch (const AmrError &e) {
+        m->err = e.msg;
+        return e.code;
+    } catch (const std::exception &e) {
+        m->err = e.what();
+        return AMR_EINVAL;
+    }
 }

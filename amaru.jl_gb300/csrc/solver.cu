@@ -752,17 +752,11 @@ static void launch_pupdate32(amr_model *m, AmrSolveWork *w) {
     AMR_COUNT(1);
 }
 
-// Shared memory a CTA's slice should stay within when a cluster of fewer CTAs would also do, for a model alone: fewer
-// CTAs mean shorter sums, smaller slices a shorter product.  An elastoplastic stage of 1 613 QUAD8 nodes (14 000
-// iterations) took 51.0 ms with 100 KB, 54.5 ms with 48 KB and 57.9 ms with all 206 KB; a stage of 525 HEX8 nodes 3.0 ms
-// with 24 to 100 KB and 3.2 ms with 206 KB.
-constexpr size_t kSliceSingle = 100 * 1024;
-
 // solve_mixed in one launch, where the model's matrix fits the shared memory of a cluster; false: it does not
 static bool solve_resident(amr_model *m, AmrSolveWork *w, double *x, const double *b, double *reac,
                            const amr_solve_opts &o, AmrSolveResult &res) {
     if (!w->shape_known) {
-        w->shape = amr_resident_shape(m, 0, m->nnodes, kSliceSingle, true);
+        w->shape = amr_resident_shape(m, 0, m->nnodes, kAmrSliceSingle, true);
         w->shape_known = true;
         if (w->shape.ctas) {
             const std::vector<int64_t> &bounds = w->shape.bounds;
