@@ -195,6 +195,7 @@ struct AmrStreamScope {
     AmrStreamScope &operator=(const AmrStreamScope &) = delete;
 };
 void *amr_raw_alloc(size_t bytes);  // throws AmrError(AMR_ENOMEM)
+extern "C" void amr_test_fail_alloc(int64_t after);  // for tests: this thread's allocation number `after` from now fails
 void amr_raw_free(void *p);
 void amr_trim_pool();               // returns the pool's unused memory of the current device
 

@@ -48,11 +48,17 @@ cudaMemPool_t library_pool() {
 }
 }  // namespace
 
+// allocations of this thread until one fails, for tests (negative: none does)
+static thread_local int64_t t_fail_alloc = -1;
+void amr_test_fail_alloc(int64_t after) { t_fail_alloc = after; }
+
 void *amr_raw_alloc(size_t bytes) {
     void *p = nullptr;
     cudaError_t e;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (amr_tl_stream && cudaStreamIsCapturing(amr_tl_stream, &cap) == cudaSuccess &&
+    if (t_fail_alloc >= 0 && t_fail_alloc-- == 0) {
+        e = cudaErrorMemoryAllocation;
+    } else if (amr_tl_stream && cudaStreamIsCapturing(amr_tl_stream, &cap) == cudaSuccess &&
         cap == cudaStreamCaptureStatusNone) {
         e = cudaMallocFromPoolAsync(&p, bytes, library_pool(), amr_tl_stream);
         if (e == cudaSuccess) {

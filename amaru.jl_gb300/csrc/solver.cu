@@ -683,7 +683,7 @@ static AmrSolveWork *work(amr_model *m) {
     AmrSolveWork *w = m->sw;
     int64_t n = m->nnodes * m->B;
     if (w->n != n) {
-        w->n = n;
+        w->n = 0;  // set once all is there: after a failed allocation the next call starts again
         amr_free(w->x32); amr_free(w->r32); amr_free(w->z32); amr_free(w->p32[0]); amr_free(w->p32[1]);
         amr_free(w->q32);
         amr_free(w->s32);
@@ -708,10 +708,18 @@ static AmrSolveWork *work(amr_model *m) {
         if (!w->ctl) {
             amr_alloc(&w->ctl, 1);
             AMR_CUDA(cudaMemsetAsync(w->ctl, 0, sizeof(Ctl), m->stream));
-            w->h_ctl = (Ctl *)amr_pinned_alloc(sizeof(Ctl));
         }
+        if (!w->h_ctl) w->h_ctl = (Ctl *)amr_pinned_alloc(sizeof(Ctl));
+        w->n = n;
     }
     return w;
+}
+
+// the Krylov vectors of the all-FP64 comparators
+static void work_fp64(AmrSolveWork *w) {
+    if (w->q64) return;  // the last one: all are there
+    amr_free(w->r64); amr_free(w->z64); amr_free(w->p64);
+    amr_alloc(&w->r64, w->n); amr_alloc(&w->z64, w->n); amr_alloc(&w->p64, w->n); amr_alloc(&w->q64, w->n);
 }
 
 void amr_solver_free(amr_model *m) {
@@ -972,9 +980,7 @@ static AmrSolveResult solve_fp64(amr_model *m, double *x, const double *b, doubl
     AmrSolveWork *w = work(m);
     cudaStream_t s = m->stream;
     const int64_t nn = m->nnodes;
-    if (!w->r64) {
-        amr_alloc(&w->r64, w->n); amr_alloc(&w->z64, w->n); amr_alloc(&w->p64, w->n); amr_alloc(&w->q64, w->n);
-    }
+    work_fp64(w);
     AmrSolveResult res{AMR_OK, 0, 0, 0.0, 0.0};
     const double tol2 = o.rtol * o.rtol;
     AMR_CUDA(cudaMemsetAsync(w->p64, 0, w->n * sizeof(double), s));
@@ -1039,9 +1045,7 @@ static AmrSolveResult solve_amg_fp64(amr_model *m, double *x, const double *b, d
     AmrSolveWork *w = work(m);
     cudaStream_t s = m->stream;
     const int64_t nn = m->nnodes;
-    if (!w->r64) {
-        amr_alloc(&w->r64, w->n); amr_alloc(&w->z64, w->n); amr_alloc(&w->p64, w->n); amr_alloc(&w->q64, w->n);
-    }
+    work_fp64(w);
     AmrSolveResult res{AMR_OK, 0, 0, 0.0, 0.0};
     const double tol2 = o.rtol * o.rtol;
     AMR_CUDA(cudaMemsetAsync(w->p64, 0, w->n * sizeof(double), s));
@@ -1218,7 +1222,7 @@ static double time_spmv32(amr_model *m, int reps) {
 template <int B>
 static double time_spmv64(amr_model *m, int reps) {
     AmrSolveWork *w = work(m);
-    if (!w->p64) throw AmrError(AMR_EINVAL, "run an all-FP64 solve on the current K first");
+    if (!w->q64) throw AmrError(AMR_EINVAL, "run an all-FP64 solve on the current K first");
     cudaStream_t s = m->stream;
     Ctl c{};
     c.rz = 1.0;
