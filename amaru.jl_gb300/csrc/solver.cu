@@ -666,14 +666,19 @@ struct AmrSolveWork {
     Ctl *ctl = nullptr;
     Ctl *h_ctl = nullptr;        // pinned
     int grid = 0, grid_spmv = 0, grid_rows = 0;
-    // the mixed solve of a small model by one cluster of CTAs (resident.cu): its shape, slice bounds,
-    // row orders and statistics
+    // the mixed solve of a small model by one cluster of CTAs (resident.cu): its shape, slice bounds, row orders and
+    // statistics; the shape is known once all of them are there
     bool shape_known = false;
     AmrResidentShape shape;
     int64_t *slices = nullptr;
     uint16_t *perm = nullptr;
     double *rows64 = nullptr;
     AmrPartStat *stat = nullptr, *h_stat = nullptr;  // (h_stat pinned)
+    void free_resident() {
+        amr_free(slices); amr_free(perm); amr_free(rows64); amr_free(stat);
+        amr_pinned_free(h_stat);
+        h_stat = nullptr;
+    }
     // all-FP64 comparators: Krylov vectors (allocated on their first use)
     double *r64 = nullptr, *z64 = nullptr, *p64 = nullptr, *q64 = nullptr;
 };
@@ -730,8 +735,7 @@ void amr_solver_free(amr_model *m) {
     amr_free(w->partials); amr_free(w->ctl);
     amr_pinned_free(w->h_ctl);
     amr_free(w->r64); amr_free(w->z64); amr_free(w->p64); amr_free(w->q64);
-    amr_free(w->slices); amr_free(w->perm); amr_free(w->rows64); amr_free(w->stat);
-    amr_pinned_free(w->h_stat);
+    w->free_resident();
     delete w;
     m->sw = nullptr;
 }
@@ -760,22 +764,29 @@ static void launch_pupdate32(amr_model *m, AmrSolveWork *w) {
     AMR_COUNT(1);
 }
 
-// solve_mixed in one launch, where the model's matrix fits the shared memory of a cluster; false: it does not
+// solve_mixed in one launch, where the model's matrix fits the shared memory of a cluster; false: it does not, or there is
+// no device memory for its arrays (asked for again at the next solve)
 static bool solve_resident(amr_model *m, AmrSolveWork *w, double *x, const double *b, double *reac,
                            const amr_solve_opts &o, AmrSolveResult &res) {
     if (!w->shape_known) {
-        w->shape = amr_resident_shape(m, 0, m->nnodes, kAmrSliceSingle, true);
-        w->shape_known = true;
-        if (w->shape.ctas) {
-            const std::vector<int64_t> &bounds = w->shape.bounds;
-            amr_alloc(&w->slices, bounds.size());
-            amr_alloc(&w->perm, w->shape.perm.size());
-            amr_h2d(m, w->perm, w->shape.perm.data(), w->shape.perm.size() * sizeof(uint16_t));
-            amr_alloc(&w->rows64, 2 * m->nnodes);
-            amr_alloc(&w->stat, 1);
-            w->h_stat = (AmrPartStat *)amr_pinned_alloc(sizeof(AmrPartStat));
-            amr_h2d(m, w->slices, bounds.data(), bounds.size() * sizeof(int64_t));
+        AmrResidentShape shape = amr_resident_shape(m, 0, m->nnodes, kAmrSliceSingle, true);
+        if (shape.ctas) {
+            try {
+                amr_alloc(&w->slices, shape.bounds.size());
+                amr_alloc(&w->perm, shape.perm.size());
+                amr_alloc(&w->rows64, 2 * m->nnodes);
+                amr_alloc(&w->stat, 1);
+                w->h_stat = (AmrPartStat *)amr_pinned_alloc(sizeof(AmrPartStat));
+                amr_h2d(m, w->perm, shape.perm.data(), shape.perm.size() * sizeof(uint16_t));
+                amr_h2d(m, w->slices, shape.bounds.data(), shape.bounds.size() * sizeof(int64_t));
+            } catch (const AmrError &e) {
+                w->free_resident();
+                if (e.code == AMR_ENOMEM) return false;
+                throw;
+            }
         }
+        w->shape = std::move(shape);
+        w->shape_known = true;
     }
     if (!w->shape.ctas) return false;
     const int every = o.refine_every > 0 ? o.refine_every : 32;

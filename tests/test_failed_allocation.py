@@ -29,13 +29,13 @@ def _model(cell, n):
     return model, model.get_bc_vals(setup)
 
 
-def _each_failure(cell, n, method, first=0):
-    """The solve with allocation `first`, `first` + 1, .. failing until none is left to fail."""
+def _each_failure(cell, n, method):
+    """The solve with each of its allocations failing in turn; returns their number."""
     model, (U0, F0) = _model(cell, n)
     opts = L.default_solve_opts(method=method, rtol=1e-9)
     U, F, _ = model.dev.solve(U0, F0, opts)
     failures = 0
-    for after in range(first, 400):
+    for after in range(400):
         model, (U0, F0) = _model(cell, n)
         before = model.dev.alloc_count()
         _fail(after)
@@ -60,3 +60,9 @@ def _each_failure(cell, n, method, first=0):
     (A.QUAD8, (9, 7), L.SOLVER_FP64, 13), (A.HEX8, (6, 4, 3), L.SOLVER_AMG, 9), (A.HEX8, (6, 4, 3), L.SOLVER_AMG_FP64, 13)])
 def test_work_arrays_without_memory(cell, n, method, least):
     assert _each_failure(cell, n, method) >= least
+
+
+@pytest.mark.parametrize("cell,n", [(A.HEX8, (5, 3, 2)), (A.QUAD8, (9, 7))])
+def test_one_launch_solve_without_memory(cell, n):
+    """Without its own arrays the solve takes a launch per step, and gives the same."""
+    assert _each_failure(cell, n, L.SOLVER_MIXED) >= 13
