@@ -281,6 +281,8 @@ size_t amr_resident_max_bytes();
 // CTAs, their bounds (ctas + 1 values) and the shared memory of the largest slice.  Host only.
 extern "C" int amr_test_resident_shape(int32_t ndim, int64_t nnodes, const int64_t *row_ptr, const int32_t *col,
                                        int64_t prefer, int32_t exact, int32_t most, int64_t *bounds, int64_t *bytes);
+// for tests: quotients of sums as the one-launch solve takes them (exact: in integers in any case)
+extern "C" int amr_test_sum_quotient(int64_t cases, int32_t n, const float *a, const float *b, int32_t exact, float *out);
 // for tests: the one-launch solve of the assembled model, of whose CTAs `rank` never sends its part of a sum, with waits
 // of limit_ms; status: every CTA's (16 at most)
 extern "C" int amr_test_resident_wait(amr_model *m, int32_t exact, int32_t rank, double limit_ms, int32_t *status,

@@ -40,10 +40,6 @@ namespace {
 constexpr int kPartThreads = 512;  // fixed: the reduction order of a part depends on it
 constexpr int kWarps = kPartThreads / 32;
 constexpr int kCluster = 8;                 // CTAs that solve one large part together
-// Shared memory a CTA's slice should stay within when the part is solved with its matrix in shared memory: all of it, as
-// one such CTA fills an SM's registers anyway and a batch wants few CTAs per part (200 QUAD8 models of 10 to 40 cells
-// a side: 66 ms against 110 ms with 100 KB).
-constexpr size_t kSliceBatch = 224 * 1024;
 constexpr size_t kMaxC2 = 5;  // streams the groups of such parts run on at most (cluster sizes 1 to 16)
 constexpr int64_t kClusterMinNodes = 2048;  // parts with this many nodes or more are large (fixed: results depend on it)
 
@@ -1081,7 +1077,10 @@ void amr_batch_set(amr_model *m, int64_t nparts, const int64_t *ptr) {
         // the parts that do not fit a cluster's shared memory first, then those that do, by cluster size and, while
         // the largest slices of their blocks, rows and windows fit together, in one group
         std::vector<AmrResidentShape> shape(nparts);
-        for (int64_t i = 0; i < nparts; i++) shape[i] = amr_resident_shape(m, ptr[i], ptr[i + 1], kSliceBatch, false);
+        // (slices may take all of an SM's shared memory, as one such CTA fills its registers anyway and a batch wants few
+        // CTAs per part: 200 QUAD8 models of 10 to 40 cells a side took 66 ms, with 100 KB 110 ms)
+        for (int64_t i = 0; i < nparts; i++)
+            shape[i] = amr_resident_shape(m, ptr[i], ptr[i + 1], amr_resident_max_bytes(), false);
         std::stable_sort(order.begin(), order.end(), [&](int64_t x, int64_t y) {
             const int cx = shape[x].ctas ? shape[x].ctas : INT32_MAX, cy = shape[y].ctas ? shape[y].ctas : INT32_MAX;
             return cx > cy;

@@ -14,23 +14,25 @@
 //
 // Two forms.  For a model alone (Exact) the operations are those of solve_mixed's launch-per-step kernels in solver.cu,
 // in the same order: the eight partial sums of a row and their tree, the rows' products by warps and CTAs of 32, 64
-// and 256 rows, the refresh's FP64 sums over CTAs.  Only an iteration's sums over CTAs are pairs of FP32 numbers
-// instead of FP64: they reach the iteration as alpha and beta rounded to FP32, which 48 bits give as 53 do but for one
-// in some ten million.  So which form a model's size selects shows in its time and hardly ever in a bit of its
-// result.  For a batch's parts, which other CTAs summed anyway, the order is free: one sum per row, one per thread.
+// and 256 rows, the refresh's FP64 sums over CTAs.  Only an iteration's sums over CTAs are not FP64 numbers; what they
+// give, alpha and beta, is the nearest FP32 number to the quotient of the exact sums, which FP64 sums miss once in some
+// hundred million.  So which form a model's size selects shows in its time and hardly ever in a bit of its result.  For a
+// batch's parts, which other CTAs summed anyway, the order is free: one sum per row, one per thread, a warp's in FP32.
 //
 // What else bounds it is the chain of an iteration, two cluster-wide sums (p.q, then r.z and r.r).  So:
 //   * the direction needs no sum of its own: a CTA pushes the z of its rows into the windows of the CTAs that read them,
 //     and after the second sum each forms p = z + beta p over its whole window;
-//   * what a CTA sends, its partial sum and its z, goes by st.async into the others' shared memory and is counted by
-//     their mbarriers, so a sum is one CTA barrier and one way across the cluster, with no fence; every warp
-//     adds the cluster's partials itself.  As each CTA waits for all, a sum is a barrier of the cluster: the slots and
-//     windows are never written while they may be read;
-//   * nothing in an iteration takes the FP64 pipe (two lanes a clock per SM): the partials of the CTAs, FP32 as in
-//     solver.cu, are added as pairs hi + lo by two-sums (48 bits), and alpha and beta are quotients of such pairs.
-// Measured, three launches per iteration over all SMs before: 26 us an iteration, now 3.5 us with Exact and 2.7 us without
-// (1 613 QUAD8 nodes, 8 CTAs); a batch of 64 QUAD8 models of 10 to 60 cells a side 230 ms, now 44 ms.
+//   * what a CTA sends, its partial sums and its z, goes by st.async into the others' shared memory and is counted by
+//     their mbarriers, so a sum is one way across the cluster, with no fence; every CTA adds the cluster's partials
+//     itself.  As each CTA waits for all, a sum is a barrier of the cluster: the slots and windows are never written
+//     while they may be read;
+//   * nothing in an iteration takes the FP64 pipe (two lanes a clock per SM; FP64 trees and quotients took as long as the
+//     rest of an iteration): the partials, FP32 as in solver.cu, are added as pairs of FP32 numbers, and in the few cases
+//     where 48 bits do not settle alpha's or beta's rounding again as integers (in all cases: batch below 63 ms).
+// Measured, three launches per iteration over all SMs before: 26 us an iteration, now 3.5 us with Exact
+// (1 613 QUAD8 nodes, 8 CTAs); a batch of 64 QUAD8 models of 10 to 60 cells a side 230 ms, now 49 ms.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <mutex>
 #include <type_traits>
@@ -47,7 +49,7 @@ constexpr int kT = 512;             // threads of a CTA
 constexpr int kW = kT / 32;
 constexpr int kRowsPerThread = 2;   // rows a thread keeps in registers
 constexpr int kMaxC = 16;           // CTAs of a cluster at most (above 8 where the device allows it)
-constexpr size_t kMaxDyn = 224 * 1024, kMaxDynExact = 206 * 1024;  // the latter leaves room for the rows' partials
+constexpr size_t kMaxDyn = 221 * 1024, kMaxDynExact = 206 * 1024;  // beside the sums' slots; the latter also the rows' values
 constexpr int kMaxGroups = kMaxC * kT * kRowsPerThread / 32;        // groups of 32 rows of a part
 
 struct Args {
@@ -77,7 +79,11 @@ struct Args {
 };
 constexpr unsigned long long kWaitNs = 2000000000ull;  // a sum takes microseconds
 
-// a value hi + lo of two FP32 numbers
+// Sums over the cluster and their quotients alpha and beta, which an iteration takes rounded to FP32.  Added as pairs
+// hi + lo of FP32 numbers (48 bits), they give that FP32 number in all but a few of a thousand cases: where the
+// quotient is not within 2^-34 of the middle between two.  There, and outside of 2^-100 to 2^100 after a scaling by the
+// last refresh's, the sums are taken again as integers and divided exactly.  So alpha and beta are the nearest FP32
+// numbers, as with FP64 sums.
 struct Pair {
     float h, l;
 };
@@ -89,11 +95,133 @@ __device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
     const float h = __fadd_rn(s, l);
     return Pair{h, __fsub_rn(l, __fsub_rn(h, s))};
 }
-// a / b rounded to FP32
-__device__ __forceinline__ float pair_div(Pair a, Pair b) {
+__device__ __forceinline__ Pair pair(double v) {
+    const float h = (float)v;
+    return Pair{h, (float)(v - (double)h)};
+}
+// a power of two near 1 / v
+__device__ __forceinline__ float scale_of(double v) {
+    return __int_as_float((127 + max(-120, min(120, 1023 - ((int)(__double_as_longlong(v) >> 52) & 0x7ff)))) << 23);
+}
+__device__ __forceinline__ bool in_range(float v) { return v > 0x1p-100f && v < 0x1p100f; }  // (false with NaN)
+// a / b rounded to FP32; sure: it is the nearest to the sums' quotient
+__device__ __forceinline__ float pair_div(Pair a, Pair b, bool &sure) {
     const float q = __fdiv_rn(a.h, b.h);
     const float r = __fadd_rn(__fmaf_rn(-q, b.h, a.h), __fmaf_rn(-q, b.l, a.l));
-    return __fadd_rn(q, __fdiv_rn(r, b.h));
+    const float c = __fdiv_rn(r, b.h), d = q * 0x1p-34f;
+    sure = in_range(a.h) && in_range(b.h) && in_range(q) &&
+           __fadd_rn(q, __fadd_rn(c, d)) == __fadd_rn(q, __fsub_rn(c, d));
+    return __fadd_rn(q, c);
+}
+// the sum of get(0 .. n - 1), n <= 512, the same in every lane
+template <int K, class F>
+__device__ __forceinline__ Pair pair_sum(F get) {
+    Pair p[K];
+#pragma unroll
+    for (int i = 0; i < K; i++) p[i] = Pair{get(32 * i + (int)(threadIdx.x & 31)), 0.0f};
+#pragma unroll
+    for (int o = K / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; i++) p[i] = pair_add(p[i], p[i + o]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        p[0] = pair_add(p[0], Pair{__shfl_xor_sync(0xffffffffu, p[0].h, o), __shfl_xor_sync(0xffffffffu, p[0].l, o)});
+    return p[0];
+}
+template <class F>
+__device__ __forceinline__ Pair pair_sum(int n, F get) {
+    if (n <= 32) return pair_sum<1>(get);
+    if (n <= 64) return pair_sum<2>(get);
+    if (n <= 128) return pair_sum<4>(get);
+    if (n <= 256) return pair_sum<8>(get);
+    return pair_sum<16>(get);
+}
+
+// A number (neg ? -1 : 1) m 2^e, the top bit of m set; m = 0: zero, or with e = kNoNumber NaN
+struct Num {
+    unsigned long long m;
+    int e;
+    bool neg;
+};
+constexpr int kNoNumber = INT_MIN, kInfinite = 1 << 20;
+__device__ __forceinline__ Num number(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int ex = (int)(b >> 52 & 0x7ff);
+    unsigned long long m = b & 0xfffffffffffffULL;
+    const bool neg = b >> 63;
+    if (ex == 0x7ff) return m ? Num{0, kNoNumber, false} : Num{1ULL << 63, kInfinite, neg};
+    if (ex > 0) m |= 1ULL << 52;
+    if (m == 0) return Num{0, 0, false};
+    const int up = __clzll((long long)m);
+    return Num{m << up, max(ex, 1) - 1075 - up, neg};
+}
+// a > b of numbers that are not negative (false with NaN)
+__device__ __forceinline__ bool greater(const Num &a, const Num &b) {
+    if (a.m == 0 || a.neg) return false;
+    if (b.m == 0) return b.e != kNoNumber;
+    return a.e != b.e ? a.e > b.e : a.m > b.m;
+}
+// the leading 24 bits as a float in [1, 2)
+__device__ __forceinline__ float leading(const Num &a) { return __int_as_float(0x3f800000 | ((int)(a.m >> 40) & 0x7fffff)); }
+// a / b rounded to FP32: a quotient of the leading bits, corrected by its exact remainder (long division)
+__device__ __noinline__ float quotient(Num a, Num b) {
+    if (a.m == 0 || b.m == 0) return a.m == 0 && a.e != kNoNumber && b.m != 0 ? 0.0f : __int_as_float(0x7fc00000);
+    // a.m 2^up / b.m has 24 bits, or those of a denormal
+    const int up = min(a.m >= b.m ? 23 : 24, a.e - b.e + 149);
+    if (up < 0) return 0.0f;
+    const unsigned long long n = a.m >> 4, d = b.m >> 4;  // 60 bits, so that remainders of some d fit 64
+    int q = __float2int_rn(__fdiv_rn(leading(a), leading(b)) * (float)(1 << up));
+    long long r = (long long)((n << up) - (unsigned long long)q * d);  // |r| < 4 d, exact modulo 2^64
+    const int k = __float2int_rn(__fdiv_rn((float)(int)(r >> 32), (float)(int)(d >> 32)));
+    q += k;
+    r -= (long long)k * (long long)d;
+    if (2 * r > (long long)d) q++;
+    if (2 * r < -(long long)d) q--;
+    const float v = ldexpf((float)q, a.e - b.e - up);
+    return a.neg != b.neg ? -v : v;
+}
+// The sum of v[0 .. n), n <= 512, the same in every lane: as integers of a unit 2^-52 of the largest value's exponent, in
+// which FP32 values down to 2^-29 of it are exact.  eights: the values of eight neighbours are added first, in FP32.
+__device__ __noinline__ Num exact_sum(const float *v, int n, bool eights) {
+    constexpr int kUp = 29;
+    const int lane = threadIdx.x & 31;
+    auto get = [&](int i) {
+        float t = i + lane < n ? v[i + lane] : 0.0f;
+        if (eights) {
+            t += __shfl_xor_sync(0xffffffffu, t, 4);
+            t += __shfl_xor_sync(0xffffffffu, t, 2);
+            t += __shfl_xor_sync(0xffffffffu, t, 1);
+            if (lane & 7) t = 0.0f;
+        }
+        return t;
+    };
+    int top = 1;
+    for (int i = 0; i < n; i += 32) top = max(top, __float_as_int(get(i)) >> 23 & 0xff);
+    top = (int)__reduce_max_sync(0xffffffffu, (unsigned)top);
+    if (top == 255) {  // infinite or NaN
+        float f = 0.0f;
+        for (int i = 0; i < n; i += 32) f += get(i);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+        return number((double)f);
+    }
+    long long s = 0;  // |s| < 16 2^53 in a lane, 2^62 in all
+    for (int i = 0; i < n; i += 32) {
+        const int b = __float_as_int(get(i)), ex = b >> 23 & 0xff;
+        const unsigned long long m = (unsigned long long)((b & 0x7fffff) | (ex ? 0x800000 : 0)) << kUp;
+        const int down = top - max(ex, 1);  // rounded where bits go
+        const unsigned long long w = down > 53 ? 0 : (m + (down > kUp ? 1ULL << (down - 1) : 0)) >> down;
+        s += b < 0 ? -(long long)w : (long long)w;
+    }
+    // three parts whose sums over the lanes fit 32 bits
+    const unsigned p0 = __reduce_add_sync(0xffffffffu, (unsigned)(s & 0x3ffffff)),
+                   p1 = __reduce_add_sync(0xffffffffu, (unsigned)(s >> 26 & 0x3ffffff));
+    const int p2 = __reduce_add_sync(0xffffffffu, (int)(s >> 52));
+    s = ((long long)p2 << 52) + ((long long)p1 << 26) + (long long)p0;
+    if (s == 0) return Num{0, 0, false};
+    const unsigned long long m = s < 0 ? 0ULL - (unsigned long long)s : (unsigned long long)s;
+    const int up = __clzll((long long)m);
+    return Num{m << up, top - 150 - kUp - up, s < 0};
 }
 
 template <int B>
@@ -119,6 +247,16 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t local, int r) {  // th
 // v to a place in a CTA's shared memory, counted by an mbarrier there
 __device__ __forceinline__ void store_async(uint32_t to, float v, uint32_t bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];" ::"r"(to), "f"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void store_async4(uint32_t to, float4 v, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void store_async2(uint32_t to, float v, float w, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(to), "f"(v),
+                 "f"(w), "r"(bar)
                  : "memory");
 }
 // waits for the phase of an mbarrier to complete; false after `limit` nanoseconds (a try may suspend the thread for a time
@@ -225,17 +363,18 @@ __device__ __forceinline__ void exact_row(const float4 *val4, const float *val1,
 template <int B, bool Exact>
 __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     constexpr int BB = B * B, M = kRowsPerThread;
-    constexpr int XR = Exact ? kT * kRowsPerThread : 1, XG = Exact ? kMaxGroups : 1;
-    __shared__ float s_row[2][XR];           // Exact: a value of each row of the slice
-    __shared__ float s_grp[3][XG];           //   the sums of 32 rows: p.q; r.z and r.r
-    __shared__ double s_grpd[2][XG / 2 + 1]; //   the sums of 64 rows at a refresh
+    constexpr int XR = Exact ? kT * kRowsPerThread : 1;
+    __shared__ float s_row[2][XR];                                  // Exact: a value of each row of the slice
+    // the cluster's sums of 32 rows, or of warps: p.q, r.r, and r.z of this iteration and the last by turns
+    __shared__ __align__(16) float s_warp[2][kW];
+    __shared__ __align__(16) float s_grp[4][Exact ? kMaxGroups : kMaxC * kW];
+    __shared__ double s_grpd[2][Exact ? kMaxGroups / 2 + 1 : 1];    // Exact: the sums of 64 rows at a refresh
     extern __shared__ float dyn[];
-    __shared__ float s_warp[2 * kW];
     __shared__ int s_off[M * kW + 1];       // first slot of each 32 rows' (row parts') blocks
-    __shared__ float s_slot[2][2][kMaxC];   // the cluster's partials of the two sums
     __shared__ double s_slotd[2][kMaxC], s_dwarp[2][kW], s_dtot[2], s_um[kMaxC];
     __shared__ __align__(8) uint64_t s_bar[2];                      // the two sums' arrivals
-    __shared__ int s_w0, s_w1, s_win[kMaxC][2], s_bytes, s_abort;
+    __shared__ int s_w0, s_w1, s_win[kMaxC][2], s_bytes, s_abort, s_late, s_stop;
+    __shared__ float s_alpha, s_beta;
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const long long part = a.list ? a.list[blockIdx.x / C] : 0;
@@ -264,7 +403,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     if (tid == 0) {
         s_w0 = (int)n0;
         s_w1 = (int)n1;
-        s_bytes = s_abort = 0;
+        s_bytes = s_abort = s_late = 0;
         for (int i = 0; i < 2; i++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_addr(&s_bar[i])), "r"(1) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -364,7 +503,6 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
         *cl.map_shared_rank(&s_win[rank][1], tid) = w0 + W;
     }
     barrier();  // (also: every CTA's mbarriers and zero window exist before a neighbour writes there)
-    const int bytes2 = s_bytes + 2 * C * 4;  // what arrives here in a second sum
     unsigned to[M];
 #pragma unroll
     for (int m = 0; m < M; m++) {
@@ -385,8 +523,12 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             const uint32_t z_to = cluster_addr(shared_addr(zwin + ((int)n0 + row[m] - s_win[r][0]) * B), r);
             if constexpr (decltype(counted)::value) {
                 const uint32_t bar = cluster_addr(shared_addr(&s_bar[1]), r);
+                if constexpr (B == 2) {
+                    store_async2(z_to, z[0], z[1], bar);
+                } else {
 #pragma unroll
-                for (int c = 0; c < B; c++) store_async(z_to + 4 * c, z[c], bar);
+                    for (int c = 0; c < B; c++) store_async(z_to + 4 * c, z[c], bar);
+                }
             } else {
 #pragma unroll
                 for (int c = 0; c < B; c++)
@@ -394,49 +536,41 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             }
         }
     };
-    // where this CTA's partials go: lanes r and 16 + r push to rank r
     const int half = lane >> 4, hl = lane & 15;
-    const uint32_t slot_to = cluster_addr(shared_addr(&s_slot[0][half][rank]), min(hl, C - 1)),
-                   bar_to = cluster_addr(shared_addr(&s_bar[0]), min(hl, C - 1));
+    // Sums over the cluster: the sums of 32 rows, or of warps, go to all CTAs.  Two sums share their steps, one in each half
+    // of a warp.  Warp 0 (and 1, the second sum) waits for what arrives here, adds it and tells the CTA; without its
+    // __syncwarp the lanes would go on one by one (the beam below: 111 ms).
+    // A wait that gives up: the CTA goes on, with values that mean nothing but stay in bounds, to the end of the iteration,
+    // where it leaves the loop as one.  The others learn of it (s_abort) at the next barrier of the cluster, before they
+    // store into another CTA again, and none has left by then.
     unsigned parity = 0;  // bit i: the phase of s_bar[i] to wait for
-    // A wait that gives up: this thread goes on, with values that mean nothing but stay in bounds, to the iteration's next
-    // __syncthreads_or, where its CTA leaves the loop as one.  The others learn of it (s_abort) at the next barrier of the
-    // cluster, before they store into another CTA again, and none has left by then.
-    bool timeout = false;
+    int turn = 0;         // the last r.z are s_grp[2 + turn]
     const int senders = rank == a.withhold ? 0 : C;
-    // the cluster's sums of v0 (and v1, with two), the same pairs in every thread; set: the slots used.  Two sums share
-    // their steps, one in each half of a warp.
-    auto cluster_sum = [&](auto two, int set, float v0, float v1, Pair &o0, Pair &o1) {
+    auto arrived = [&](int set, int bytes) {
+        if (tid == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(&s_bar[set])), "r"(bytes)
+                         : "memory");
+        if (warp <= set && !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u, a.wait_ns)) s_late = 1;
+        __syncwarp();
+        parity ^= 1u << set;
+    };
+    // the sums of v0 (and v1) over the threads, a warp's in FP32; a CTA's 16 sums as four stores to each CTA (16 of four
+    // bytes: 58 ms for the batch below instead of 49)
+    auto push_warps = [&](auto two, int set, float v0, float v1) {
         constexpr bool two_sums = decltype(two)::value;
         float t;
         if (two_sums) t = (half ? v1 : v0) + __shfl_xor_sync(0xffffffffu, half ? v0 : v1, 16);
         else t = v0 + __shfl_xor_sync(0xffffffffu, v0, 16);
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (hl == 0) s_warp[half * kW + warp] = t;
+        if (hl == 0 && (two_sums || half == 0)) s_warp[half][warp] = t;
         __syncthreads();
-        if (warp == 0) {
-            t = s_warp[two_sums ? lane : hl];
-#pragma unroll
-            for (int o = kW / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (hl < (two_sums ? C : senders) && (two_sums || half == 0)) store_async(slot_to + set * 2 * kMaxC * 4, t, bar_to + set * 8);
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(&s_bar[set])),
-                             "r"(two_sums ? bytes2 : C * 4) : "memory");
-        }
-        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u, a.wait_ns);
-        parity ^= 1u << set;
-        Pair p{hl < C ? s_slot[set][two_sums ? half : 0][hl] : 0.0f, 0.0f};
-#pragma unroll
-        for (int o = kMaxC / 2; o > 0; o >>= 1)
-            p = pair_add(p, Pair{__shfl_xor_sync(0xffffffffu, p.h, o), __shfl_xor_sync(0xffffffffu, p.l, o)});
-        if (two_sums) {
-            const Pair q{__shfl_xor_sync(0xffffffffu, p.h, 16), __shfl_xor_sync(0xffffffffu, p.l, 16)};
-            o0 = half ? q : p;
-            o1 = half ? p : q;
-        } else {
-            o0 = p;
-        }
+        if (warp < (two_sums ? 2 : 1))
+            for (int r = lane >> 2; r < (two_sums ? C : senders); r += 8)
+                store_async4(cluster_addr(shared_addr(&s_grp[two_sums ? (warp ? 1 : 3 - turn) : 0][rank * kW + 4 * (lane & 3)]), r),
+                             *reinterpret_cast<const float4 *>(&s_warp[warp][4 * (lane & 3)]),
+                             cluster_addr(shared_addr(&s_bar[set]), r));
+        arrived(set, two_sums ? s_bytes + 8 * C * kW : 4 * C * kW);
     };
     // Exact: sums over 32 rows of the slice's values s_row[0] (s_row[1]), in the order `first` (p.q: lane bits 2, 1, then 16,
     // 8, 4, as the warps of 4 rows and CTAs of 32 add them) or natural, pushed to every CTA
@@ -460,17 +594,11 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
                 t += __shfl_xor_sync(0xffffffffu, t, 8);
                 t += __shfl_xor_sync(0xffffffffu, t, 4);
             }
-            if (hl < (two_sums ? C : senders) && (two_sums || half == 0))
-                store_async(cluster_addr(shared_addr(&s_grp[two_sums ? 1 + half : 0][g0 + g]), hl), t, bar_to + set * 8);
+            if (hl < (two_sums ? C : senders) && (two_sums || half == 0))  // lane r (and 16 + r) to CTA r
+                store_async(cluster_addr(shared_addr(&s_grp[two_sums ? (half ? 1 : 3 - turn) : 0][g0 + g]), hl), t,
+                            cluster_addr(shared_addr(&s_bar[set]), hl));
         }
-        if (tid == 0)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(&s_bar[set])),
-                         "r"(two_sums ? s_bytes + 8 * groups : 4 * groups) : "memory");
-        timeout |= !wait_phase(shared_addr(&s_bar[set]), (parity >> set) & 1u, a.wait_ns);
-        parity ^= 1u << set;
-    };
-    auto lane_pair = [&](Pair p, int o) {
-        return pair_add(p, Pair{__shfl_xor_sync(0xffffffffu, p.h, o), __shfl_xor_sync(0xffffffffu, p.l, o)});
+        arrived(set, two_sums ? s_bytes + 8 * groups : 4 * groups);
     };
     // FP64 sums (a refresh only), valid in every thread
     auto cluster_sum64 = [&](double v0, double v1, double &t0, double &t1) {
@@ -506,10 +634,6 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
         __syncthreads();
         t0 = s_dtot[0];
         t1 = s_dtot[1];
-    };
-    auto split = [](double v) {
-        const float h = (float)v;
-        return Pair{h, (float)(v - (double)h)};
     };
     // the FP64 true residual of the slice from a.x (published by a barrier before): r, z = Minv r, r.z and |r|^2
     auto residual64 = [&](double &rz, double &rr) {
@@ -611,15 +735,19 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     double rz64, rr_true;
     residual64(rz64, rr_true);
     const double bnorm2 = rr_true;
-    const float stop_rr = (float)(0.0625 * a.tol2 * bnorm2);
-    Pair gam = split(rz64);
+    const double stop_rr = 0.0625 * a.tol2 * bnorm2;
+    float scale = scale_of(rz64);
+    Pair gam = pair(rz64 * (double)scale);
+    bool fresh = true;  // the last r.z is a refresh's
+    auto last_rz = [&]() { return fresh ? number(rz64) : exact_sum(s_grp[2 + turn], Exact ? groups : C * kW, Exact); };
     // the next refresh: after a 10x drop, or, where that would end within the tolerance, at a quarter of the
     // tolerance (a refresh just inside it would return the solution with up to four times the residual; not with
     // Exact, which refreshes where solve_mixed does)
     auto threshold = [&]() {
-        return Exact || 1e-2 * rr_true > a.tol2 * bnorm2 ? fmaxf(stop_rr, (float)(1e-2 * rr_true)) : stop_rr;
+        return Exact || 1e-2 * rr_true > a.tol2 * bnorm2 ? fmax(stop_rr, 1e-2 * rr_true) : stop_rr;
     };
-    float thr = threshold(), beta = 0.0f;
+    double thr = threshold();
+    float scale_rr = scale_of(thr), stop_at = (float)(thr * (double)scale_rr), beta = 0.0f;
     int iters = 0, refreshes = 0, status = 0, since = 0;
     bool done = !(bnorm2 > 0.0) || rr_true <= a.tol2 * bnorm2;
     if (isnan(rr_true)) { status = AMR_ENOCONV; done = true; }
@@ -674,18 +802,23 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
                 for (int c = 0; c < B; c++) dot = fmaf(pwin[(own + row[m]) * B + c], q[m][c], dot);
             }
         }
-        Pair pq, t2[2];
-        if constexpr (Exact) {
-            push_groups(std::false_type(), 0);
-            pq = Pair{0.0f, 0.0f};
-            for (int i = lane; i < groups; i += 32) pq = pair_add(pq, Pair{s_grp[0][i], 0.0f});
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) pq = lane_pair(pq, o);
-        } else {
-            cluster_sum(std::false_type(), 0, dot, 0.0f, pq, pq);
+        if constexpr (Exact) push_groups(std::false_type(), 0);
+        else push_warps(std::false_type(), 0, dot, 0.0f);
+        const int parts = Exact ? groups : C * kW;
+        if (warp == 0) {
+            const Pair pq = pair_sum(parts, [&](int i) { return i < parts ? s_grp[0][i] * scale : 0.0f; });
+            bool sure;
+            float al = pair_div(gam, pq, sure);
+            if (!sure) {  // (the same in all lanes)
+                const Num e = exact_sum(s_grp[0], parts, false);
+                al = e.m == 0 || e.neg ? __int_as_float(0x7fc00000) : quotient(last_rz(), e);
+            }
+            if (lane == 0) s_alpha = al;
+            __syncwarp();
         }
-        const bool broken = !(pq.h > 0.0f);  // ends the solve below, where the CTA knows of waits that gave up
-        const float alpha = broken ? 0.0f : pair_div(gam, pq);
+        __syncthreads();
+        const bool broken = isnan(s_alpha);  // ends the solve below, where the CTA knows of waits that gave up
+        const float alpha = broken ? 0.0f : s_alpha;
         // x += alpha p ; r -= alpha q ; z = Minv r
         float v0 = 0.0f, v1 = 0.0f;
 #pragma unroll
@@ -713,32 +846,45 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
                 s_row[1][i] = v1;
             }
         }
-        if constexpr (Exact) {
-            push_groups(std::true_type(), 1);
-            // CTAs of 256 rows: eight warps' sums by bits 4, 2, 1; then over the CTAs
-            t2[0] = t2[1] = Pair{0.0f, 0.0f};
-            for (int i0 = 0; i0 < groups; i0 += 32)
-#pragma unroll
-                for (int w = 0; w < 2; w++) {
-                    float t = i0 + lane < groups ? s_grp[1 + w][i0 + lane] : 0.0f;
-                    t += __shfl_xor_sync(0xffffffffu, t, 4);
-                    t += __shfl_xor_sync(0xffffffffu, t, 2);
-                    t += __shfl_xor_sync(0xffffffffu, t, 1);
-                    t2[w] = pair_add(t2[w], Pair{t, 0.0f});
+        if constexpr (Exact) push_groups(std::true_type(), 1);
+        else push_warps(std::true_type(), 1, v0, v1);
+        const float *rz = s_grp[3 - turn];
+        if (warp < 2) {
+            const float *v = warp == 0 ? rz : s_grp[1], sc = warp == 0 ? scale : scale_rr;
+            const Pair t = pair_sum(parts, [&](int i) {
+                float x = i < parts ? v[i] : 0.0f;
+                if constexpr (Exact) {  // CTAs of 256 rows: eight warps' sums by bits 4, 2, 1
+                    x += __shfl_xor_sync(0xffffffffu, x, 4);
+                    x += __shfl_xor_sync(0xffffffffu, x, 2);
+                    x += __shfl_xor_sync(0xffffffffu, x, 1);
+                    if (lane & 7) x = 0.0f;
                 }
-#pragma unroll
-            for (int w = 0; w < 2; w++) t2[w] = lane_pair(lane_pair(t2[w], 16), 8);
-        } else {
-            cluster_sum(std::true_type(), 1, v0, v1, t2[0], t2[1]);
+                return x * sc;
+            });
+            if (warp == 0) {
+                bool sure;
+                float be = pair_div(t, gam, sure);
+                if (!sure) be = quotient(exact_sum(rz, parts, Exact), last_rz());
+                gam = t;
+                if (lane == 0) s_beta = be;
+            } else {
+                bool more = t.h > stop_at;  // r.r above the threshold: no refresh yet
+                if (!(in_range(t.h) && fabsf(t.h - stop_at) > 0x1p-20f * stop_at))
+                    more = greater(exact_sum(v, parts, Exact), number(thr));
+                if (lane == 0) s_stop = !more;
+            }
+            __syncwarp();
         }
-        if (__syncthreads_or(timeout)) { status = AMR_ETIMEOUT; break; }
+        turn ^= 1;
+        fresh = false;
+        __syncthreads();
+        if (s_late) { status = AMR_ETIMEOUT; break; }
         if (broken) { status = AMR_ENOCONV; break; }
-        beta = pair_div(t2[0], gam);
-        gam = t2[0];
+        beta = s_beta;
         iters++;
         since++;
         if (Exact && iters >= a.max_iters) { status = AMR_ENOCONV; break; }
-        if (!(t2[1].h > thr) || since >= a.force_every) {
+        if (s_stop || since >= a.force_every) {
             // refresh: fold the FP32 correction into the FP64 solution and recompute the true residual
 #pragma unroll
             for (int m = 0; m < M; m++) {
@@ -755,8 +901,12 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             barrier();
             if (__syncthreads_or(s_abort)) { status = AMR_ETIMEOUT; break; }
             residual64(rz64, rr_true);
-            gam = split(rz64);
+            scale = scale_of(rz64);
+            gam = pair(rz64 * (double)scale);
+            fresh = true;
             thr = threshold();
+            scale_rr = scale_of(thr);
+            stop_at = (float)(thr * (double)scale_rr);
             refreshes++;
             since = 0;
             if (isnan(rr_true)) { status = AMR_ENOCONV; break; }
@@ -798,6 +948,31 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
         a.stat[part] = s;
     }
     if (a.t1 && tid == 0) atomicMax(a.t1, global_ns());
+}
+
+// for tests: a warp per case, the quotient of the sums of a and b, each cases x n, n <= 512; exact: by integers in any case
+__global__ void __launch_bounds__(32) k_sum_quotient(int n, const float *a, const float *b, bool exact, float *out) {
+    __shared__ float s[2][kMaxGroups];
+    const int64_t at = (int64_t)blockIdx.x * n;
+    for (int i = threadIdx.x; i < n; i += 32) {
+        s[0][i] = a[at + i];
+        s[1][i] = b[at + i];
+    }
+    __syncwarp();
+    Pair p[2];
+    float scale = 1.0f;
+#pragma unroll
+    for (int k = 1; k >= 0; k--) {
+        if (k == 1) {
+            const Pair t = pair_sum(n, [&](int i) { return i < n ? s[1][i] : 0.0f; });
+            scale = scale_of((double)t.h);
+        }
+        p[k] = pair_sum(n, [&](int i) { return i < n ? s[k][i] * scale : 0.0f; });
+    }
+    bool sure;
+    float v = pair_div(p[0], p[1], sure);
+    if (!sure || exact) v = quotient(exact_sum(s[0], n, false), exact_sum(s[1], n, false));
+    if (threadIdx.x == 0) out[blockIdx.x] = v;
 }
 
 // the kernels' attributes, once per device and process (a launch that changed them would race with others); the
@@ -1033,6 +1208,23 @@ static void withheld_sum(amr_model *m, bool exact, int rank, unsigned long long 
     amr_d2h(m, st.data(), w.stat, st.size() * sizeof(AmrPartStat));
     status.clear();
     for (const AmrPartStat &s : st) status.push_back(s.status);
+}
+
+int amr_test_sum_quotient(int64_t cases, int32_t n, const float *a, const float *b, int32_t exact, float *out) {
+    if (cases < 1 || cases > INT32_MAX || n < 1 || n > kMaxGroups) return AMR_EINVAL;
+    const size_t bytes = (size_t)cases * n * sizeof(float);
+    float *d = nullptr;
+    if (cudaMalloc(&d, 2 * bytes + cases * sizeof(float)) != cudaSuccess) return AMR_ENOMEM;
+    float *db = d + cases * n, *dout = db + cases * n;
+    cudaError_t e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(db, b, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_sum_quotient<<<(unsigned)cases, 32>>>(n, d, db, exact != 0, dout);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, dout, cases * sizeof(float), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? AMR_OK : AMR_ECUDA;
 }
 
 int amr_test_resident_wait(amr_model *m, int32_t exact, int32_t rank, double limit_ms, int32_t *status, int32_t *ctas) {
