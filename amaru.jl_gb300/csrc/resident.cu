@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
     __shared__ __align__(16) float s_warp[2][kW];
     __shared__ __align__(16) float s_grp[4][Exact ? kMaxGroups : kMaxC * kW];
     __shared__ double s_grpd[2][Exact ? kMaxGroups / 2 + 1 : 1];    // Exact: the sums of 64 rows at a refresh
-    extern __shared__ float dyn[];
+    extern __shared__ __align__(16) float dyn[];  // read as float4
     __shared__ int s_off[M * kW + 1];       // first slot of each 32 rows' (row parts') blocks
     __shared__ double s_slotd[2][kMaxC], s_dwarp[2][kW], s_dtot[2], s_um[kMaxC];
     __shared__ __align__(8) uint64_t s_bar[2];                      // the two sums' arrivals
