@@ -48,10 +48,11 @@ constexpr int kSweepTile = 32;  // pivots of a step of the dense level's inversi
 
 // row lengths of the dense level's FP64 work matrix (whole tiles) and of its inverse
 inline int64_t dense_ld(int64_t nc) { return (nc + kSweepTile - 1) / kSweepTile * kSweepTile; }
-// doubles of the padded matrix, a step's two panels and two diagonal tiles, the panels' digits and their rows' scales
+// doubles of the padded matrix, a step's two panels and two diagonal tiles' factors, the panels' digits and their rows' scales
 constexpr int kDig = 7, kDigRow = kDig * kSweepTile;
+constexpr int kPivot = 2 * kSweepTile * kSweepTile + 2 * kSweepTile;  // doubles of a diagonal tile's inverse and factors
 inline size_t sweep_doubles(int64_t ld) {
-    return (size_t)(ld * ld + 2 * ld * kSweepTile + 2 * kSweepTile * kSweepTile + 2 * ld * kDigRow / 4 + 2 * ld);
+    return (size_t)(ld * ld + 2 * ld * kSweepTile + 2 * kPivot + 2 * ld * kDigRow / 4 + 2 * ld);
 }
 inline int64_t inverse_ld(int64_t nc) { return (nc + 3) / 4 * 4; }
 
@@ -1363,8 +1364,8 @@ __global__ void k_prolong_sa16(int64_t n, const int64_t *prp, const int32_t *pcj
 // The inverse of an SPD matrix of nc rows takes nc^3 / 2 FMAs when only one triangle is formed.  An elimination with one
 // launch per pivot moved the whole augmented matrix through L2 for every pivot: 33.5 ms at nc = 1 428 (23.5 us a pivot),
 // 3.8 ms at nc = 558.  Here 32 pivots are taken at a time:
-//   D = A_kk^-1 (in shared memory), W_i = A_ik D (k_sweep_panel), A_ij -= W_i A_kj for the other tiles of the
-//   lower triangle (k_sweep_update), A_ik = W_i, A_kk = -D;
+//   D = A_kk^-1 and A_kk = L diag(x g^2) L' (in shared memory), U_i = A_ik L^-T / g, V_i = U_i / x (k_sweep_panel),
+//   A_ij -= V_i U_j' = A_ik D A_jk' for the other tiles of the lower triangle (k_sweep_update), A_ik = A_ik D, A_kk = -D;
 // after the last block the triangle holds -A^-1.  A 32 x 32 tile per CTA gives n = 1 332 some 900 tiles a step, and every
 // tile is read and written once per 32 pivots.  The CTA that updates the next diagonal tile inverts it in the same launch,
 // beside the other tiles, so a step costs two launches.  With the update's products on the FP64 pipe (two FMAs a clock
@@ -1414,6 +1415,7 @@ __device__ __forceinline__ double reciprocal(double d) {
 struct SweepTile {
     double S[2][kSw][kSw + 1];  // the tile before and after a pivot, by turns
     double col[2][kSw], fac[2][kSw], inv[2];
+    double L[kSw][kSw + 1], piv[kSw];  // the tile before as L diag(piv) L', L unit lower (the part below the diagonal)
 };
 
 // T.S[0] (lower triangle) swept over its kSw pivots: -S^-1, in T.S[0]; 256 threads.  One barrier a pivot: while the
@@ -1437,10 +1439,14 @@ __device__ void sweep_tile(SweepTile &T) {
         }
     }
     auto column = [&](int to, int q, double v) {  // lane's entry v of pivot q's column
-        const double iv = reciprocal(__shfl_sync(0xffffffffu, v, q));
+        const double d = __shfl_sync(0xffffffffu, v, q), iv = reciprocal(d), f = nz(v) ? v * iv : 0.0;
         T.col[to][lane] = v;
-        T.fac[to][lane] = nz(v) ? v * iv : 0.0;
-        if (lane == 0) T.inv[to] = iv;
+        T.fac[to][lane] = f;
+        T.L[lane][q] = lane > q ? f : 0.0;
+        if (lane == 0) {
+            T.inv[to] = iv;
+            T.piv[q] = d;
+        }
     };
     if (lead) column(0, 0, T.S[0][lane][0]);
     __syncthreads();
@@ -1462,11 +1468,20 @@ __device__ void sweep_tile(SweepTile &T) {
         __syncthreads();
     }
 }
-// D = -S mirrored (the inverse of the diagonal tile, all kSw x kSw entries)
+// the inverse of the diagonal tile (-S mirrored, all kSw x kSw entries), L, and per pivot d = x g^2 with g a power of two and
+// x in [1, 4): 1 / g and 1 / x
 __device__ void store_inverse(const SweepTile &T, double *D) {
     for (int t = threadIdx.x; t < kSw * kSw; t += 256) {
         const int r = t / kSw, c = t % kSw;
         D[t] = -(r >= c ? T.S[0][r][c] : T.S[0][c][r]);
+        D[kSw * kSw + t] = T.L[r][c];
+    }
+    if (threadIdx.x < kSw) {
+        const double d = T.piv[threadIdx.x];
+        const int ex = __double2hiint(d) >> 20 & 0x7ff;
+        const double ig = ex == 0 || ex == 0x7ff ? 1.0 : __hiloint2double((1023 - ((ex - 1023) >> 1)) << 20, 0);
+        D[2 * kSw * kSw + threadIdx.x] = ig;
+        D[2 * kSw * kSw + kSw + threadIdx.x] = 1.0 / (d * ig * ig);
     }
 }
 
@@ -1479,9 +1494,9 @@ __global__ void __launch_bounds__(256) k_sweep_first(const double *C, int64_t ld
     store_inverse(T, D);
 }
 
-// The update's products W_i A_kj are formed on the tensor cores from exact slices (the splitting of Ozaki, Ogita, Oishi and
-// Rump, Numer. Algorithms 59, 2012; on matrix units Mukunoki et al. 2020): each row of W and of A_ik is scaled by a power
-// of two to integers of 55 bits, written as kDig signed digits of 8 bits, which bf16 holds exactly.  A product of two
+// The update's products V_i U_j' are formed on the tensor cores from exact slices (the splitting of Ozaki, Ogita, Oishi and
+// Rump, Numer. Algorithms 59, 2012; on matrix units Mukunoki et al. 2020): each row of V and of U is rounded to integers of 55
+// bits under its largest entry, written as kDig signed digits of 8 bits, which bf16 holds exactly.  A product of two
 // digits has 14 bits, a sum of 32 of them and of the up to seven digit pairs of one weight 22, so the FP32 accumulators
 // are exact; the pairs (s, t), s + t <= kDig + 2, leave out 2^-64 of the rows' largest entries' product, and the weighted
 // sum is rounded once where 32 FP64 FMAs round 32 times.
@@ -1490,7 +1505,7 @@ struct SweepDigits {
     double *ws, *ps;   // ld: 2^(e - 19) for rows of entries below 2^e; 0 for a zero row, NaN for a non-finite one
 };
 inline SweepDigits sweep_digits(double *C, int64_t ld) {
-    uint16_t *d = reinterpret_cast<uint16_t *>(C + ld * ld + 2 * ld * kSw + 2 * kSw * kSw);
+    uint16_t *d = reinterpret_cast<uint16_t *>(C + ld * ld + 2 * ld * kSw + 2 * kPivot);
     double *sc = reinterpret_cast<double *>(d + 2 * ld * kDigRow);
     return {d, d + ld * kDigRow, sc, sc + ld};
 }
@@ -1523,12 +1538,18 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// W_i = A_ik D for 8 rows of a tile row i != k per CTA (four CTAs a tile row), written over A_ik and to Wb, with the old
-// A_ik in Pb, and both as digits; the last CTA writes A_kk = -D.
+// For 8 rows of a tile row i != k per CTA (four CTAs a tile row): A_ik = A_ik D, and the factors of the update's product
+// A_ik D A_jk' = V_i U_j': with A_kk = L diag(x g^2) L', U_i = A_ik L^-T / g by substitution and V_i = U_i / x, to Pb and
+// Wb and as digits; the last CTA writes A_kk = -D.
+//
+// Both factors' rows are of the magnitude of the root of their diagonal entry, however ill-conditioned the tile: the
+// update loses what an elimination pivot by pivot loses.  With A_ik D for V_i and A_ik for U_j the product cancels where
+// the tile is ill-conditioned, and digits relative to a row's largest entry keep little of the others (33 rows, cond
+// 1e10: error 0.04 of the inverse, now as the elimination's).
 __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *C, const double *D, double *Wb,
                                                      double *Pb, SweepDigits dg) {
-    constexpr int R = 8;
-    __shared__ double sA[R][kSw + 1], sD[kSw][kSw + 1];
+    constexpr int R = 8, N = kSw * kSw / 256;
+    __shared__ double sA[R][kSw + 1], sD[kSw][kSw + 1], sL[kSw][kSw + 1];
     if (blockIdx.x == gridDim.x - 1) {
         for (int t = threadIdx.x; t < kSw * kSw; t += 256)
             C[((int64_t)k * kSw + t / kSw) * ld + k * kSw + t % kSw] = -D[t];
@@ -1540,9 +1561,10 @@ __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *
     const int r = threadIdx.x / kSw, q = threadIdx.x % kSw;    // row and column, columns fastest
     const int rt = threadIdx.x % R, qt = threadIdx.x / R;      // rows fastest
     bool fin = true;
-    double d[kSw * kSw / 256];
+    double d[2 * N];
 #pragma unroll
-    for (int u = 0; u < kSw * kSw / 256; u++) d[u] = D[threadIdx.x + 256 * u];
+    for (int u = 0; u < 2 * N; u++) d[u] = D[threadIdx.x + 256 * u];
+    const double ig = D[2 * kSw * kSw + q], ix = D[2 * kSw * kSw + kSw + q];
     double a;
     if (i > k) {  // stored as the tile (i, k)
         a = C[((int64_t)i * kSw + r0 + r) * ld + k * kSw + q];
@@ -1551,31 +1573,42 @@ __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *
         a = C[((int64_t)k * kSw + qt) * ld + i * kSw + r0 + rt];
         sA[rt][qt] = a;
     }
-    fin &= finite(a);
+    fin &= finite(a) && finite(ix);
 #pragma unroll
-    for (int u = 0; u < kSw * kSw / 256; u++) {
+    for (int u = 0; u < N; u++) {
         sD[(threadIdx.x + 256 * u) / kSw][q] = d[u];
-        fin &= finite(d[u]);
+        sL[(threadIdx.x + 256 * u) / kSw][q] = d[N + u];
+        fin &= finite(d[u]) && finite(d[N + u]);
     }
     const int any = __syncthreads_or(nz(a)), all_finite = __syncthreads_and(fin);
     const int64_t row = (int64_t)i * kSw + r0 + r;
-    Pb[row * kSw + q] = sA[r][q];
-    row_digits(sA[r][q], dg.P + row * kDigRow, dg.ps + row);
-    if (!any) {  // W_i is zero as A_ik is
+    if (!any) {  // the factors are zero as A_ik is
+        Pb[row * kSw + q] = 0.0;
         Wb[row * kSw + q] = 0.0;
+        row_digits(0.0, dg.P + row * kDigRow, dg.ps + row);
         row_digits(0.0, dg.W + row * kDigRow, dg.ws + row);
         return;
     }
-    double w = 0.0;
+    double w = 0.0, u = sA[r][q];
     if (all_finite) {
 #pragma unroll 8
-        for (int t = 0; t < kSw; t++) w = fma(sA[r][t], sD[t][q], w);
+        for (int t = 0; t < kSw; t++) {
+            w = fma(sA[r][t], sD[t][q], w);
+            u = fma(-__shfl_sync(0xffffffffu, u, t), sL[q][t], u);  // (L is zero from the diagonal on)
+        }
     } else {
-        for (int t = 0; t < kSw; t++)
+        for (int t = 0; t < kSw; t++) {
             if (nz(sA[r][t]) && nz(sD[t][q])) w = fma(sA[r][t], sD[t][q], w);
+            const double ut = __shfl_sync(0xffffffffu, u, t);
+            if (nz(ut) && nz(sL[q][t])) u = fma(-ut, sL[q][t], u);
+        }
     }
-    Wb[row * kSw + q] = w;
-    row_digits(w, dg.W + row * kDigRow, dg.ws + row);
+    u *= ig;
+    const double v = nz(u) ? u * ix : 0.0;
+    Pb[row * kSw + q] = u;
+    Wb[row * kSw + q] = v;
+    row_digits(u, dg.P + row * kDigRow, dg.ps + row);
+    row_digits(v, dg.W + row * kDigRow, dg.ws + row);
     if (i > k) {
         C[row * ld + k * kSw + q] = w;
     } else {  // the transpose, written along the rows of the tile (k, i)
@@ -1586,7 +1619,7 @@ __global__ void __launch_bounds__(256) k_sweep_panel(int64_t ld, int k, double *
     }
 }
 
-// A_ij -= W_i A_kj for a tile (i, j) of the lower triangle per CTA, i, j != k, m = tile rows - 1; the next diagonal
+// A_ij -= V_i U_j' for a tile (i, j) of the lower triangle per CTA, i, j != k, m = tile rows - 1; the next diagonal
 // tile is CTA 0's, which also inverts it.  A warp has 16 x 8 entries.  The columns of a row are taken in the order that
 // gives each lane 16 consecutive bytes of its row's digits (the same order on both sides: the sum runs over them).
 // Rows with a non-finite entry take the products in FP64, zero factors left out.
@@ -1712,7 +1745,7 @@ void sweep_steps(cudaStream_t s, double *C, int64_t ld) {
     const SweepDigits dg = sweep_digits(C, ld);
     k_sweep_first<<<1, 256, 0, s>>>(C, ld, Db);
     for (int k = 0; k < nt; k++) {
-        double *Dk = Db + (k & 1) * kSw * kSw, *Dn = Db + ((k + 1) & 1) * kSw * kSw;
+        double *Dk = Db + (k & 1) * kPivot, *Dn = Db + ((k + 1) & 1) * kPivot;
         k_sweep_panel<<<(unsigned)(4 * (nt - 1) + 1), 256, 0, s>>>(ld, k, C, Dk, Wb, Pb, dg);
         const int64_t tiles = (int64_t)(nt - 1) * nt / 2;
         if (tiles > 0) k_sweep_update<<<(unsigned)tiles, 256, 0, s>>>(ld, k, nt - 1, C, Wb, Pb, dg, Dn);
@@ -1726,6 +1759,21 @@ __global__ void k_dense_extract(int64_t nc, const double *C, int64_t ld, V *Cinv
     if (t >= nc * ldc) return;
     const int64_t r = t / ldc, c = t % ldc;
     Cinv[t] = c >= nc ? V(0) : (V)(-(r >= c ? C[r * ld + c] : C[c * ld + r]));
+}
+// the expanded lower triangle of a BSR matrix of n block rows, padded to whole tiles (2 launches and a memset); its
+// swept triangle to the inverse (1 launch)
+template <int NM, class V>
+void dense_expand(cudaStream_t s, int64_t n, const int64_t *rp, const int32_t *cj, const int64_t *diag, const V *A,
+                  int64_t nbs, double *C, int64_t nc) {
+    const int64_t ld = dense_ld(nc);
+    (void)diag;
+    AMR_CUDA(cudaMemsetAsync(C, 0, ld * ld * sizeof(double), s));
+    k_dense_expand<NM, V><<<(unsigned)n, 256, 0, s>>>(n, rp, cj, A, nbs, C, ld);
+    k_dense_pad<<<1, kSw, 0, s>>>(nc, ld, C);
+}
+template <class V>
+void dense_extract(cudaStream_t s, int64_t nc, const double *C, V *Cinv, int64_t ldc) {
+    k_dense_extract<V><<<nblk(nc * ldc, 256), 256, 0, s>>>(nc, C, dense_ld(nc), Cinv, ldc);
 }
 // x = Cinv b in FP32, warp per row, 16-byte loads of the matrix (rows padded to ldc, a multiple of 4), zero entries
 // skipped as below: bound by the latency of a row's loads, 8.2 us at 1 344 rows (10 us a word at a time).
@@ -2116,9 +2164,7 @@ struct Cycle {
         AmgLevel &D = g->L[nl - 1];
         const int64_t nc = g->nc, ld = dense_ld(nc), ldc = inverse_ld(nc);
         const int nt = (int)(ld / kSw);  // tile rows
-        AMR_CUDA(cudaMemsetAsync(g->Cd, 0, ld * ld * sizeof(double), s));
-        k_dense_expand<NM, V><<<(unsigned)D.n, 256, 0, s>>>(D.n, D.rp, D.cj, vals<V>(D).A, D.nbs, g->Cd, ld);
-        k_dense_pad<<<1, kSw, 0, s>>>(nc, ld, g->Cd);
+        dense_expand<NM, V>(s, D.n, D.rp, D.cj, D.diag, vals<V>(D).A, D.nbs, g->Cd, nc);
         AMR_COUNT(2);
         // the sweep steps as one CUDA graph, captured once per hierarchy (its buffers are fixed)
         if (!g->gj_exec) {
@@ -2137,7 +2183,7 @@ struct Cycle {
         }
         AMR_CUDA(cudaGraphLaunch(g->gj_exec, s));
         AMR_COUNT(1 + nt + (nt > 1 ? nt : 0));
-        k_dense_extract<V><<<nblk(nc * ldc, 256), 256, 0, s>>>(nc, g->Cd, ld, coarse_inverse(g), ldc);
+        dense_extract<V>(s, nc, g->Cd, coarse_inverse(g), ldc);
         AMR_COUNT(1);
         AMR_CUDA(cudaGetLastError());
     }
@@ -2195,6 +2241,33 @@ void amr_amg_prepare64(amr_model *m) {
         else Cycle<2, 3, double>::numeric(m, m->amg);
         m->amg->numeric64_valid = true;
     }
+}
+
+int amr_test_dense_inverse(int32_t n, const double *A, double *X) {
+    if (n < 1 || n > kDenseMax) return AMR_EINVAL;
+    const int64_t ld = dense_ld(n), nn = (int64_t)n * n;
+    std::vector<int64_t> rp(n + 1), diag(n);
+    std::vector<int32_t> cj(nn);
+    for (int i = 0; i <= n; i++) rp[i] = (int64_t)i * n;
+    for (int i = 0; i < n; i++) diag[i] = (int64_t)i * n + i;
+    for (int64_t k = 0; k < nn; k++) cj[k] = (int32_t)(k % n);
+    char *d = nullptr;
+    const size_t work = sweep_doubles(ld) * 8;
+    if (cudaMalloc(&d, work + 16 * nn + 4 * nn + 16 * (n + 1)) != cudaSuccess) return AMR_ENOMEM;
+    double *C = (double *)d, *dA = C + sweep_doubles(ld), *dX = dA + nn;
+    int64_t *drp = (int64_t *)(dX + nn), *ddiag = drp + n + 1;
+    int32_t *dcj = (int32_t *)(ddiag + n);
+    cudaMemcpy(dA, A, 8 * nn, cudaMemcpyHostToDevice);
+    cudaMemcpy(drp, rp.data(), 8 * (n + 1), cudaMemcpyHostToDevice);
+    cudaMemcpy(ddiag, diag.data(), 8 * n, cudaMemcpyHostToDevice);
+    cudaMemcpy(dcj, cj.data(), 4 * nn, cudaMemcpyHostToDevice);
+    dense_expand<1, double>(0, n, drp, dcj, ddiag, dA, nn, C, n);
+    sweep_steps(0, C, ld);
+    dense_extract<double>(0, n, C, dX, n);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(X, dX, 8 * nn, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? AMR_OK : AMR_ECUDA;
 }
 
 // z = V-cycle(r), fine-level node-major FP32 vectors, on the handle's stream

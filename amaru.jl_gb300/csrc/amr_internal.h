@@ -314,6 +314,8 @@ void amr_amg_vcycle64(amr_model *m, const double *r, double *z);
 void amr_amg_invalidate(amr_model *m);
 double amr_amg_time_residual(amr_model *m, int reps, bool fp64, double *bytes);
 void amr_amg_free(amr_model *m);
+// for tests: the inverse of an SPD matrix of n rows as the dense coarsest level forms it
+extern "C" int amr_test_dense_inverse(int32_t n, const double *A, double *X);
 // recovery.cu: nodal_patch_recovery (structure once per model, values per call)
 void amr_recovery_prepare(amr_model *m);
 const std::vector<int32_t> &amr_recovery_codes(amr_model *m);
