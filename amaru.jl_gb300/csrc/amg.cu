@@ -1401,17 +1401,6 @@ __global__ void k_dense_pad(int64_t nc, int64_t ld, double *C) {
     if (r < ld) C[r * ld + r] = 1.0;
 }
 
-// 1 / d from the FP32 reciprocal and two Newton steps (24, 48, 53 bits): a shorter chain on the FP64 pipe than the
-// division, which is taken outside the float range
-__device__ __forceinline__ double reciprocal(double d) {
-    const float f = (float)d;
-    const float a = fabsf(f);
-    if (!(a > 1e-30f && a < 1e30f)) return 1.0 / d;
-    double x = (double)__frcp_rn(f);
-    x = fma(x, fma(-d, x, 1.0), x);
-    return fma(x, fma(-d, x, 1.0), x);
-}
-
 struct SweepTile {
     double S[2][kSw][kSw + 1];  // the tile before and after a pivot, by turns
     double col[2][kSw], fac[2][kSw], inv[2];
@@ -1439,7 +1428,7 @@ __device__ void sweep_tile(SweepTile &T) {
         }
     }
     auto column = [&](int to, int q, double v) {  // lane's entry v of pivot q's column
-        const double d = __shfl_sync(0xffffffffu, v, q), iv = reciprocal(d), f = nz(v) ? v * iv : 0.0;
+        const double d = __shfl_sync(0xffffffffu, v, q), iv = 1.0 / d, f = nz(v) ? v * iv : 0.0;
         T.col[to][lane] = v;
         T.fac[to][lane] = f;
         T.L[lane][q] = lane > q ? f : 0.0;
