@@ -237,6 +237,12 @@ void amr_export_csc(amr_model *m, int64_t *nnz, int64_t *colptr, int64_t *rowval
 // K64 = Ks + s1 M + s2 (alpha M + beta Ks) (Ks may be null: K = 0), then K32, Minv
 void amr_dyn_combine(amr_model *m, const double *Ks, double s1, double s2, double alpha, double beta);
 void amr_update_elements(amr_model *m, const double *dU_nm, double *dFin_nm);  // node-major device vectors
+void amr_ensure_geometry(amr_model *m);                 // the 3-D geometry caches, once per model
+// elements per CTA of the internal-force kernel that the tuner times, the untuned one first; for tests: with their
+// shared memory (6 at most)
+std::vector<int> amr_internal_candidates(int dim, int nen, int nip, bool cached);
+extern "C" int amr_test_internal_candidates(int32_t dim, int32_t nen, int32_t nip, int32_t cached, int32_t *epb,
+                                            int64_t *smem);
 void amr_apply_dofs(amr_model *m);                      // masks after amr_set_dofs
 void amr_loads(amr_model *m, const amr_load *loads, int nloads, double t, double *F_nm);  // F_nm += (device)
 int amr_check_status(amr_model *m);                     // reads d_status, resets, returns code

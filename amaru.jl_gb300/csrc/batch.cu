@@ -1654,9 +1654,10 @@ void amr_autotune_model(amr_model *m, amr_tuning *out) {
     t.ngroups = (int32_t)std::min<size_t>(m->groups.size(), AMR_MAX_TUNED_GROUPS);
     t.stiffness_seconds = 0.0;
     t.internal_seconds = 0.0;
+    amr_ensure_geometry(m);  // of all groups, before they are taken out of the list
     std::vector<AmrGroup> all = m->groups;
     try {
-        for (size_t gi = 0; gi < m->groups.size(); gi++) {
+        for (size_t gi = 0; gi < all.size(); gi++) {
             // time this group's kernels alone: the other groups are taken out of the list meanwhile
             AmrGroup g = all[gi];
             const int np = pairs_of(g.nen), ndim = amr::shape_ndim(g.shape);
@@ -1675,9 +1676,7 @@ void amr_autotune_model(amr_model *m, amr_tuning *out) {
             t.stiffness_seconds += best * 1e-3;
             double besti = 1e300;
             int best_int = g.epb_int;
-            for (int e : {1, 2, 4, 8, 16}) {
-                const size_t smem = sizeof(double) * (size_t)e * (2 * g.nen * ndim + g.nip * g.nen * ndim);
-                if (smem > 200 * 1024) continue;
+            for (int e : amr_internal_candidates(ndim, g.nen, g.nip, m->geo_valid && g.geo_g)) {
                 g.epb_int = e;
                 m->groups.assign(1, g);
                 const double ms = time_ms(m, [&] { amr_update_elements(m, dU, dF); }, 3);

@@ -1536,21 +1536,30 @@ void launch_stiff_ref(amr_model *m, const AmrGroup &g) {
     AMR_CUDA(cudaGetLastError());
 }
 
+// elements per CTA of the internal-force kernel, with the 3-D geometry cache and without, and its shared memory
+int internal_epb(int nen, int nip, bool cached) {
+    (void)nen;
+    return cached ? std::max(1, kIntThreads / nip) : nip >= 16 ? 4 : 16;
+}
+size_t internal_smem(int dim, int nen, int nip, bool cached, int epb) {
+    return sizeof(double) * (size_t)epb * (cached ? nen * 3 + nip * 7 : 2 * nen * dim + nip * nen * dim);
+}
+
 template <int DIM, int NEN>
 void launch_internal(amr_model *m, const AmrGroup &g, const double *dU) {
     GroupArgs ga{g.tab, g.nip, g.first, g.count, m->geo_valid ? g.geo_g : nullptr, m->geo_valid ? g.geo_w : nullptr};
     if constexpr (DIM == 3)
         if (ga.geo_g) {
-            const int epb = g.epb_int > 0 ? g.epb_int : std::max(1, kIntThreads / g.nip);
-            const size_t smem = sizeof(double) * (size_t)epb * (NEN * 3 + g.nip * 7);  // 24 KB at most: TET4, 64 elements
+            const int epb = g.epb_int > 0 ? g.epb_int : internal_epb(NEN, g.nip, true);
+            const size_t smem = internal_smem(3, NEN, g.nip, true, epb);
             internal_cached_kernel<NEN><<<nblk(g.count, epb), kIntThreads, smem, m->stream>>>(
                 margs(m), ga, epb, dU, m->stbk, m->st, m->Fel, m->d_status);
             AMR_COUNT(1);
             AMR_CUDA(cudaGetLastError());
             return;
         }
-    int epb = g.epb_int > 0 ? g.epb_int : ((g.nip >= 16) ? 4 : 16);
-    size_t smem = sizeof(double) * (size_t)epb * (2 * NEN * DIM + g.nip * NEN * DIM);
+    int epb = g.epb_int > 0 ? g.epb_int : internal_epb(NEN, g.nip, false);
+    size_t smem = internal_smem(DIM, NEN, g.nip, false, epb);
     int threads = std::max(epb * g.nip, epb * NEN * DIM);
     threads = ((threads + 31) / 32) * 32;
     if (threads > 256) threads = 256;
@@ -1590,6 +1599,22 @@ int amr_check_status(amr_model *m) {
         amr_h2d(m, m->d_status, reset, sizeof reset);
     }
     return code;
+}
+
+std::vector<int> amr_internal_candidates(int dim, int nen, int nip, bool cached) {
+    std::vector<int> c{internal_epb(nen, nip, cached)};
+    for (int e : {1, 2, 4, 8, 16})
+        if (e != c[0] && internal_smem(dim, nen, nip, cached, e) <= (cached ? 48 : 200) * 1024) c.push_back(e);
+    return c;
+}
+
+int amr_test_internal_candidates(int32_t dim, int32_t nen, int32_t nip, int32_t cached, int32_t *epb, int64_t *smem) {
+    const std::vector<int> c = amr_internal_candidates(dim, nen, nip, cached != 0);
+    for (size_t i = 0; i < c.size(); i++) {
+        epb[i] = c[i];
+        smem[i] = (int64_t)internal_smem(dim, nen, nip, cached != 0, c[i]);
+    }
+    return (int)c.size();
 }
 
 // Builds the 3-D groups' geometry caches once per model (the coordinates never change).  If an element is
