@@ -1700,8 +1700,9 @@ void amr_autotune_model(amr_model *m, amr_tuning *out) {
     m->assembly_mode = saved_mode;
     amr_check_status(m);  // a trial update with dU = 0 reports nothing the caller asked for
     AMR_CUDA(cudaMemcpyAsync(m->st, st_save, nst * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    // batched solve: resident CTAs per SM, on a capped run of the assembled K with a unit load
-    if (m->batch && m->K_valid) {
+    // batched solve: resident CTAs per SM of the kernel that streams the matrices (the parts that a cluster's shared
+    // memory does not hold), on a capped run of the assembled K with a unit load
+    if (m->batch && m->batch->nstream > 0 && m->K_valid) {
         AmrBatch *b = m->batch;
         double *x = dU, *rhs = dF, *reac = nullptr;
         amr_alloc(&reac, n);
