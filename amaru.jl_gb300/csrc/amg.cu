@@ -790,25 +790,26 @@ __global__ void __launch_bounds__(128) k_sa_ap(int64_t nq, const int32_t *qrow, 
     for (int u = 0; u < BF * NM; u++) o[u] = acc[u];
 }
 
-// coarse operator P' (A P), kGalLanes lanes per coarse block (I, J): sum over the fine rows i that P reaches I from
+// coarse operator P' (A P), LANES lanes per coarse block (I, J): sum over the fine rows i that P reaches I from
 // (block s) of P_s' Q_iJ (if row i of A P has column J), the lanes' sums added in a fixed order.  Bound by the latency of
-// the search in row i: a thread per block walked some 200 rows one after another
-// (TET10 24 x 5 x 10: 461 us, now 84; HEX20 100 x 40 x 40: the second level's operator 1.53 ms, now 0.24; the first level's, enough blocks for every thread,
-// 4.1 and 4.35).
-constexpr int kGalLanes = 8;
-template <int BF, int NM, class V>
+// the search in row i: a thread per block walked some 200 rows one after another.  With 1 / 4 / 8 lanes: HEX20
+// 100 x 40 x 40, first level, 825 000 blocks, 4.10 / 3.94 / 4.36 ms, second, 3 700 blocks, 1.50 / 0.44 / 0.24; HEX20
+// 60 x 24 x 24, 178 000 blocks, 1.17 / 0.89 / 0.92; 50 x 20 x 20, 88 000 blocks, 0.76 / 0.51 / 0.50; TET10 24 x 5 x 10,
+// 8 200 blocks, 0.48 / 0.15 / 0.09; QUAD8 300 x 300, 343 000 blocks, 150 / 128 / 140 us.
+constexpr int64_t kGalMany = 100000;  // blocks from which four lanes are faster than eight
+template <int BF, int NM, class V, int LANES>
 __global__ void k_sa_galerkin(int64_t ncb, const int32_t *crow, const int32_t *ccj, const int64_t *ptp,
                               const int32_t *pti, const int32_t *pts, const V *P, const int64_t *qrp,
                               const int32_t *qcj, const V *Q, V *Ac, int64_t nbsc) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, cb = t / kGalLanes;
-    const int lane = (int)(t % kGalLanes);
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, cb = t / LANES;
+    const int lane = (int)(t % LANES);
     if (cb >= ncb) return;  // (uniform over a block's lanes)
-    const unsigned mask = ((1u << kGalLanes) - 1) << ((threadIdx.x & 31) / kGalLanes * kGalLanes);
+    const unsigned mask = ((1ull << LANES) - 1) << ((threadIdx.x & 31) / LANES * LANES);
     const int32_t I = crow[cb], J = ccj[cb];
     V acc[NM * NM];
 #pragma unroll
     for (int u = 0; u < NM * NM; u++) acc[u] = V(0);
-    for (int64_t e = ptp[I] + lane; e < ptp[I + 1]; e += kGalLanes) {
+    for (int64_t e = ptp[I] + lane; e < ptp[I + 1]; e += LANES) {
         const int64_t i = pti[e];
         int64_t lo = qrp[i], hi = qrp[i + 1];  // J in the sorted columns of row i of A P
         while (lo < hi) {
@@ -830,12 +831,12 @@ __global__ void k_sa_galerkin(int64_t ncb, const int32_t *crow, const int32_t *c
         }
     }
 #pragma unroll
-    for (int o = kGalLanes / 2; o > 0; o >>= 1)
+    for (int o = LANES / 2; o > 0; o >>= 1)
 #pragma unroll
         for (int u = 0; u < NM * NM; u++) acc[u] += __shfl_xor_sync(mask, acc[u], o);
 #pragma unroll
     for (int u = 0; u < NM * NM; u++)
-        if (u % kGalLanes == lane) Ac[(int64_t)u * nbsc + cb] = acc[u];
+        if (u % LANES == lane) Ac[(int64_t)u * nbsc + cb] = acc[u];
 }
 
 // The FP32 cycle's prolongator rounded to FP16 (saturated at the FP16 range): P16 by rows, P16T by columns
@@ -2114,8 +2115,13 @@ struct Cycle {
         }
         k_sa_ap<BF, NM, V><<<grid(F.nq), 128, 0, s>>>(F.nq, F.qrow, F.qcj, F.rp, F.cj, A, nbs, F.prp, F.pcj,
                                                             fv.P, fv.Q, F.p_steps);
-        k_sa_galerkin<BF, NM, V><<<grid(C.nblocks * kGalLanes), 128, 0, s>>>(C.nblocks, F.crow, C.cj, F.ptp, F.pti, F.pts,
-                                                                       fv.P, F.qrp, F.qcj, fv.Q, cv.A, C.nbs);
+        auto product = [&](auto lanes) {
+            constexpr int LANES = decltype(lanes)::value;
+            k_sa_galerkin<BF, NM, V, LANES><<<grid(C.nblocks * LANES), 128, 0, s>>>(
+                C.nblocks, F.crow, C.cj, F.ptp, F.pti, F.pts, fv.P, F.qrp, F.qcj, fv.Q, cv.A, C.nbs);
+        };
+        if (C.nblocks < kGalMany) product(std::integral_constant<int, 8>());
+        else product(std::integral_constant<int, 4>());
         AMR_COUNT(3);
     }
     static void numeric(amr_model *m, AmrAmg *g) {
