@@ -48,7 +48,8 @@ constexpr int kSweepTile = 32;  // pivots of a step of the dense level's inversi
 
 // row lengths of the dense level's FP64 work matrix (whole tiles) and of its inverse
 inline int64_t dense_ld(int64_t nc) { return (nc + kSweepTile - 1) / kSweepTile * kSweepTile; }
-// doubles of the padded matrix, a step's two panels and two diagonal tiles' factors, the panels' digits and their rows' scales
+// doubles of the padded matrix, a step's two panels and two diagonal tiles' factors, the panels' digits and their rows'
+// scales
 constexpr int kDig = 7, kDigRow = kDig * kSweepTile;
 constexpr int kPivot = 2 * kSweepTile * kSweepTile + 2 * kSweepTile;  // doubles of a diagonal tile's inverse and factors
 inline size_t sweep_doubles(int64_t ld) {
@@ -1458,8 +1459,8 @@ __device__ void sweep_tile(SweepTile &T) {
         __syncthreads();
     }
 }
-// the inverse of the diagonal tile (-S mirrored, all kSw x kSw entries), L, and per pivot d = x g^2 with g a power of two and
-// x in [1, 4): 1 / g and 1 / x
+// the inverse of the diagonal tile (-S mirrored, all kSw x kSw entries), L, and per pivot d = x g^2 with g a power of two
+// and x in [1, 4): 1 / g and 1 / x
 __device__ void store_inverse(const SweepTile &T, double *D) {
     for (int t = threadIdx.x; t < kSw * kSw; t += 256) {
         const int r = t / kSw, c = t % kSw;
@@ -1485,8 +1486,8 @@ __global__ void __launch_bounds__(256) k_sweep_first(const double *C, int64_t ld
 }
 
 // The update's products V_i U_j' are formed on the tensor cores from exact slices (the splitting of Ozaki, Ogita, Oishi and
-// Rump, Numer. Algorithms 59, 2012; on matrix units Mukunoki et al. 2020): each row of V and of U is rounded to integers of 55
-// bits under its largest entry, written as kDig signed digits of 8 bits, which bf16 holds exactly.  A product of two
+// Rump, Numer. Algorithms 59, 2012; on matrix units Mukunoki et al. 2020): each row of V and of U is rounded to integers
+// of 55 bits under its largest entry, written as kDig signed digits of 8 bits, which bf16 holds exactly.  A product of two
 // digits has 14 bits, a sum of 32 of them and of the up to seven digit pairs of one weight 22, so the FP32 accumulators
 // are exact; the pairs (s, t), s + t <= kDig + 2, leave out 2^-64 of the rows' largest entries' product, and the weighted
 // sum is rounded once where 32 FP64 FMAs round 32 times.
@@ -1645,8 +1646,8 @@ __global__ void __launch_bounds__(256, 2) k_sweep_update(int64_t ld, int k, int 
         if (work) {
             const uint4 *a0 = reinterpret_cast<const uint4 *>(dg.W + ((int64_t)i * kSw + r) * kDigRow) + lane % 4;
             const uint4 *a1 = a0 + 8 * (kDigRow / 8);
-            const uint4 *b0 = reinterpret_cast<const uint4 *>(dg.P + ((int64_t)j * kSw + (warp >> 1) * 8 + lane / 4) * kDigRow) +
-                              lane % 4;
+            const int64_t bp = (int64_t)j * kSw + (warp >> 1) * 8 + lane / 4;
+            const uint4 *b0 = reinterpret_cast<const uint4 *>(dg.P + bp * kDigRow) + lane % 4;
             uint4 x[kDig], y[kDig];
 #pragma unroll
             for (int s = 0; s < kDig; s++) {

@@ -294,13 +294,12 @@ extern "C" int amr_test_sum_quotient(int64_t cases, int32_t n, const float *a, c
 extern "C" int amr_test_resident_wait(amr_model *m, int32_t exact, int32_t rank, double limit_ms, int32_t *status,
                                       int32_t *ctas);
 // solves the parts list[0..nparts) (null: part 0) on `stream`: part p's slice bounds at slices[first[p]] (null: 0), the
-// slices' row orders in perm (per node of the model); x
-// (in: prescribed values, initial guess), b, reac node-major FP64; rows64: 2 x nnodes of scratch (exact shapes); stat per part; t0 / t1 (may be null) the
-// %globaltimer span
+// slices' row orders in perm (per node of the model); x (in: prescribed values, initial guess), b, reac node-major FP64;
+// rows64: 2 x nnodes of scratch (exact shapes); stat per part; t0 / t1 (may be null) the %globaltimer span
 void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
-                         const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active, const double *b, double *x, double *reac,
-                         double *rows64, AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1,
-                         double tol2, int max_iters, int force_every, cudaStream_t stream);
+                         const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active,
+                         const double *b, double *x, double *reac, double *rows64, AmrPartStat *stat,
+                         unsigned long long *t0, unsigned long long *t1, double tol2, int max_iters, int force_every, cudaStream_t stream);
 // vector helpers (solver.cu)
 double amr_norm_inf(amr_model *m, const double *v, const uint8_t *mask_or_null);
 void amr_eq_to_nm(amr_model *m, const double *d_eq, double *d_nm);  // scatter eq_id-ordered -> node-major (0 elsewhere)

@@ -1195,9 +1195,9 @@ void launch_pcg(amr_model *m, const PcgArgs &a, int ctas_per_sm) {
         const size_t lane = b->side.empty() ? 0 : g % (b->side.size() + 1);  // 0: the handle's stream
         cudaStream_t st = lane == 0 ? m->stream : b->side[lane - 1];
         if (lane > 0 && g == lane) AMR_CUDA(cudaStreamWaitEvent(st, b->fork, 0));
-        amr_resident_launch(m, q.shape, q.count, b->slices, b->first, b->perm, b->order + q.first, a.active, a.b, a.x, a.reac, nullptr, a.stat,
-                            a.step ? &a.step->t0 : nullptr, a.step ? &a.step->t1 : nullptr, a.tol2, a.max_iters,
-                            a.force_every, st);
+        amr_resident_launch(m, q.shape, q.count, b->slices, b->first, b->perm, b->order + q.first, a.active, a.b, a.x,
+                            a.reac, nullptr, a.stat, a.step ? &a.step->t0 : nullptr, a.step ? &a.step->t1 : nullptr,
+                            a.tol2, a.max_iters, a.force_every, st);
     }
     if (b->nstream > 0) {
         AMR_CUDA(cudaMemsetAsync(b->counter, 0, 2 * sizeof(unsigned long long), m->stream));

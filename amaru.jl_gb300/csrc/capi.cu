@@ -770,7 +770,9 @@ int amr_solve(amr_model *m, double *U, double *F, const amr_solve_opts *opts, am
             stats->rel_residual = r.rel_residual;
             stats->seconds = r.seconds;
         }
-        if (r.status) throw AmrError(r.status, std::string(amr_solve_failure(r.status)) + " (relative residual " + std::to_string(r.rel_residual) + ")");
+        if (r.status)
+            throw AmrError(r.status, std::string(amr_solve_failure(r.status)) + " (relative residual " +
+                                         std::to_string(r.rel_residual) + ")");
         double umax = amr_norm_inf(m, x, m->free_mask);
         if (std::isnan(umax) || std::isinf(umax)) throw AmrError(AMR_ENAN, "solve_system!: NaN values in the solution");
         if (umax > 1e8) throw AmrError(AMR_ESINGULAR, "solve_system!: Possible syngular matrix");

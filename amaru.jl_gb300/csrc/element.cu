@@ -791,7 +791,8 @@ __device__ __forceinline__ double ref_value(int q, int d, const double *g, const
 constexpr int kRefChunk = 8;
 template <int DIM, int NEN>
 __host__ __device__ constexpr int ref_doubles(int nip) {  // shared memory of the CTA, in doubles
-    return NEN * DIM + nip * (2 * NEN * DIM + 36 + 2 * DIM * DIM + 1 + NEN) + (nip < kRefChunk ? nip : kRefChunk) * 6 * NEN * DIM;
+    return NEN * DIM + nip * (2 * NEN * DIM + 36 + 2 * DIM * DIM + 1 + NEN) +
+           (nip < kRefChunk ? nip : kRefChunk) * 6 * NEN * DIM;
 }
 
 template <int DIM, int NEN>

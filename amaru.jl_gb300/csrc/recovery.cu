@@ -580,7 +580,8 @@ __global__ void __launch_bounds__(8 * kGramTasks) k_patch_gram(FitArgs A) {
     double dmin = DBL_MAX, dmax = 0.0;
 #pragma unroll
     for (int j = 0; j < NT; j++) {
-        double d = j < nt ? m[mono_find<DIM>(2 * mono_exp<DIM>(j, 0), 2 * mono_exp<DIM>(j, 1), 2 * mono_exp<DIM>(j, 2))] : 1.0;
+        double d = 1.0;
+        if (j < nt) d = m[mono_find<DIM>(2 * mono_exp<DIM>(j, 0), 2 * mono_exp<DIM>(j, 1), 2 * mono_exp<DIM>(j, 2))];
 #pragma unroll
         for (int q = 0; q < NT; q++)
             if (q < j) d -= R[packed(q, j)] * R[packed(q, j)];
@@ -597,7 +598,8 @@ __global__ void __launch_bounds__(8 * kGramTasks) k_patch_gram(FitArgs A) {
             if (i > j) {
                 double v = 0.0;
                 if (i < nt) {
-                    v = m[mono_find<DIM>(mono_exp<DIM>(i, 0) + mono_exp<DIM>(j, 0), mono_exp<DIM>(i, 1) + mono_exp<DIM>(j, 1),
+                    v = m[mono_find<DIM>(mono_exp<DIM>(i, 0) + mono_exp<DIM>(j, 0),
+                                         mono_exp<DIM>(i, 1) + mono_exp<DIM>(j, 1),
                                          mono_exp<DIM>(i, 2) + mono_exp<DIM>(j, 2))];
 #pragma unroll
                     for (int q = 0; q < NT; q++)
@@ -1025,7 +1027,8 @@ void build(amr_model *m) {
             const double nnod = (double)(t_node_ptr.back() - t_node_ptr[t_node_ptr.size() - 2]);
             // per element of the patch the translated monomials and moments (or nt FMA per IP and field), per node and
             // field nt - 1 FMA
-            flops += ecount * mono_ops + (moments ? ecount * (m->ndim == 3 ? 25.0 : 20.0) : 2.0 * mcount * nt) * mask_nf[mk] +
+            const double field_ops = moments ? ecount * (m->ndim == 3 ? 25.0 : 20.0) : 2.0 * mcount * nt;
+            flops += ecount * mono_ops + field_ops * mask_nf[mk] +
                      2.0 * nnod * (nt - 1) * mask_nf[mk];
         }
     }

@@ -49,7 +49,7 @@ constexpr int kT = 512;             // threads of a CTA
 constexpr int kW = kT / 32;
 constexpr int kRowsPerThread = 2;   // rows a thread keeps in registers
 constexpr int kMaxC = 16;           // CTAs of a cluster at most (above 8 where the device allows it)
-constexpr size_t kMaxDyn = 221 * 1024, kMaxDynExact = 206 * 1024;  // beside the sums' slots; the latter also the rows' values
+constexpr size_t kMaxDyn = 221 * 1024, kMaxDynExact = 206 * 1024;  // beside the sums' slots (Exact: and the rows' values)
 constexpr int kMaxGroups = kMaxC * kT * kRowsPerThread / 32;        // groups of 32 rows of a part
 
 struct Args {
@@ -313,7 +313,7 @@ __device__ __forceinline__ double tree_sum(int n, F get) {
     }
     return nw == 1 ? w[0] : ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
 }
-// One row's product (or this thread's eighth-th of it): the thread's share of the eight sums of k_spmv32v's lanes, which take
+// One row's product (or this thread's part of it): the thread's share of the eight sums of k_spmv32v's lanes, which take
 // four blocks each in turn, then the lanes' tree
 template <int B, int S>
 __device__ __forceinline__ void exact_row(const float4 *val4, const float *val1, const uint16_t *cols, int kcap, int e,
@@ -467,7 +467,8 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
             const int e = slot0[m] + 32 * t;
             cols[e] = in ? (uint16_t)(a.cj[k] - w0) : (uint16_t)own;
 #pragma unroll
-            for (int q = 0; q < BB / 4; q++) val4[q * a.kcap + e] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            for (int q = 0; q < BB / 4; q++)
+                val4[q * a.kcap + e] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             if (BB % 4) val1[e] = v[BB - 1];
         }
     }
@@ -565,15 +566,17 @@ __global__ void __launch_bounds__(kT, 1) k_resident_pcg(Args a) {
         for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         if (hl == 0 && (two_sums || half == 0)) s_warp[half][warp] = t;
         __syncthreads();
-        if (warp < (two_sums ? 2 : 1))
+        if (warp < (two_sums ? 2 : 1)) {
+            const int q = 4 * (lane & 3);
+            const uint32_t slot = shared_addr(&s_grp[two_sums ? (warp ? 1 : 3 - turn) : 0][rank * kW + q]);
+            const float4 sums = *reinterpret_cast<const float4 *>(&s_warp[warp][q]);
             for (int r = lane >> 2; r < (two_sums ? C : senders); r += 8)
-                store_async4(cluster_addr(shared_addr(&s_grp[two_sums ? (warp ? 1 : 3 - turn) : 0][rank * kW + 4 * (lane & 3)]), r),
-                             *reinterpret_cast<const float4 *>(&s_warp[warp][4 * (lane & 3)]),
-                             cluster_addr(shared_addr(&s_bar[set]), r));
+                store_async4(cluster_addr(slot, r), sums, cluster_addr(shared_addr(&s_bar[set]), r));
+        }
         arrived(set, two_sums ? s_bytes + 8 * C * kW : 4 * C * kW);
     };
-    // Exact: sums over 32 rows of the slice's values s_row[0] (s_row[1]), in the order `first` (p.q: lane bits 2, 1, then 16,
-    // 8, 4, as the warps of 4 rows and CTAs of 32 add them) or natural, pushed to every CTA
+    // Exact: sums over 32 rows of the slice's values s_row[0] (s_row[1]), pushed to every CTA; of p.q by the lane bits 2, 1,
+    // then 16, 8, 4, as the warps of 4 rows and CTAs of 32 add them, the others in natural order
     const int64_t P0 = bound[0];
     const int groups = (int)((bound[C] - P0 + 31) / 32), g0 = (int)((n0 - P0) / 32);
     auto push_groups = [&](auto two, int set) {
@@ -1163,9 +1166,9 @@ static Args args_of(const amr_model *m, const AmrResidentShape &shape, const int
 }
 
 void amr_resident_launch(amr_model *m, const AmrResidentShape &shape, int64_t nparts, const int64_t *slices,
-                         const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active, const double *b, double *x, double *reac,
-                         double *rows64, AmrPartStat *stat, unsigned long long *t0, unsigned long long *t1,
-                         double tol2, int max_iters, int force_every, cudaStream_t stream) {
+                         const int64_t *first, const uint16_t *perm, const int64_t *list, const uint8_t *active,
+                         const double *b, double *x, double *reac, double *rows64, AmrPartStat *stat,
+                         unsigned long long *t0, unsigned long long *t1, double tol2, int max_iters, int force_every, cudaStream_t stream) {
     if (nparts <= 0) return;
     Args a = args_of(m, shape, slices, perm, b, x, reac, rows64, stat);
     a.first = first; a.list = list; a.active = active; a.t0 = t0; a.t1 = t1;

@@ -792,8 +792,8 @@ static bool solve_resident(amr_model *m, AmrSolveWork *w, double *x, const doubl
     const int every = o.refine_every > 0 ? o.refine_every : 32;
     cudaStream_t s = m->stream;
     AMR_CUDA(cudaEventRecord(m->ev0, s));
-    amr_resident_launch(m, w->shape, 1, w->slices, nullptr, w->perm, nullptr, nullptr, b, x, reac, w->rows64, w->stat, nullptr,
-                        nullptr, o.rtol * o.rtol, o.max_iters, 16 * every, s);
+    amr_resident_launch(m, w->shape, 1, w->slices, nullptr, w->perm, nullptr, nullptr, b, x, reac, w->rows64, w->stat,
+                        nullptr, nullptr, o.rtol * o.rtol, o.max_iters, 16 * every, s);
     AMR_CUDA(cudaEventRecord(m->ev1, s));
     AMR_CUDA(cudaMemcpyAsync(w->h_stat, w->stat, sizeof(AmrPartStat), cudaMemcpyDeviceToHost, s));
     AMR_CUDA(cudaStreamSynchronize(s));
