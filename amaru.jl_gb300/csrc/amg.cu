@@ -1372,7 +1372,7 @@ __global__ void k_prolong_sa16(int64_t n, const int64_t *prp, const int32_t *pcj
 // tile is read and written once per 32 pivots.  The CTA that updates the next diagonal tile inverts it in the same launch,
 // beside the other tiles, so a step costs two launches.  With the update's products on the FP64 pipe (two FMAs a clock
 // per SM) that pipe bound a step: 61 of 68 us at nc = 1 428, 3.9 ms in all, 0.96 at nc = 558.  From exact slices on the
-// tensor cores it takes 2.25 and 0.74 ms, and the 32 pivots of the next diagonal tile, 28 us a step, bound it.
+// tensor cores it takes 2.45 and 0.81 ms, and the 32 pivots of the next diagonal tile, 28 us a step, bound it.
 //
 // A product with a zero factor is left out, and a tile pair without a nonzero is skipped: the level is block diagonal
 // over the parts of a batch, so a part's non-finite values stay in its own rows and columns, and the zero tiles

@@ -276,10 +276,12 @@ struct AmrResidentShape {
     std::vector<uint16_t> perm;                // per node, slice by slice: its rows by descending length, stable
 };
 // Shared memory a CTA's slice should stay within when a cluster of fewer CTAs would also do, for a model alone: fewer
-// CTAs mean shorter sums, smaller slices a shorter product.  An elastoplastic stage of 1 613 QUAD8 nodes (14 000
-// iterations) took 51.0 ms with 100 KB, 54.5 ms with 48 KB and 57.9 ms with all 206 KB; a stage of 525 HEX8 nodes 3.0 ms
-// with 24 to 100 KB and 3.2 ms with 206 KB.
-constexpr size_t kAmrSliceSingle = 100 * 1024;
+// CTAs mean shorter sums, smaller slices a shorter product.  An iteration with 24 / 48 / 100 / 206 KB, us: HEX8 20 x 4 x 4
+// 4.76 / 4.77 / 4.77 / 5.51, 20 x 7 x 6 5.8 / 5.8 / 5.8 / 6.4; TET4 9 x 6 x 5 4.6 / 4.6 / 4.6 / 5.5; QUAD8 12 x 9
+// 3.23 / 3.24 / 3.66 / 4.37, 61 x 7 3.29 / 3.29 / 3.45 / 3.95, 33 x 31 3.85 / 3.85 / 3.85 / 4.33; QUAD4 40 x 33
+// 3.30 / 3.31 / 3.45 / 5.07; TRI6 14 x 9 3.11 / 3.11 / 3.91 / 5.24; TET10 4 x 3 x 3, HEX20 4 x 2 x 2 and QUAD8 50 x 50 the
+// same with each.  12 KB gives what 24 KB gives.
+constexpr size_t kAmrSliceSingle = 48 * 1024;
 AmrResidentShape amr_resident_shape(const amr_model *m, int64_t P0, int64_t P1, size_t prefer, bool exact);
 size_t amr_resident_bytes(const amr_model *m, const AmrResidentShape &s);  // of a slice of these sizes
 size_t amr_resident_max_bytes();

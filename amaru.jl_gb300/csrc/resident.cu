@@ -29,7 +29,7 @@
 //   * nothing in an iteration takes the FP64 pipe (two lanes a clock per SM; FP64 trees and quotients took as long as the
 //     rest of an iteration): the partials, FP32 as in solver.cu, are added as pairs of FP32 numbers, and in the few cases
 //     where 48 bits do not settle alpha's or beta's rounding again as integers (in all cases: batch below 63 ms).
-// Measured, three launches per iteration over all SMs before: 26 us an iteration, now 3.5 us with Exact
+// Measured, three launches per iteration over all SMs before: 26 us an iteration, now 3.2 us with Exact
 // (1 613 QUAD8 nodes, 8 CTAs); a batch of 64 QUAD8 models of 10 to 60 cells a side 230 ms, now 49 ms.
 #include <algorithm>
 #include <climits>

@@ -44,7 +44,7 @@ def test_every_cta_has_rows(cell, ndim):
     for n in sizes:
         mesh = A.Mesh(A.Block([[0.0] * ndim, [1.0] * ndim], cellshape=cell, **dict(zip(("nx", "ny", "nz"), n))))
         rp, cj = _pattern(mesh)
-        for prefer in (24 << 10, 100 << 10, 206 << 10):
+        for prefer in (24 << 10, 48 << 10, 100 << 10, 206 << 10):
             ctas, bounds, nbytes = _shape(ndim, rp, cj, prefer, 1)
             if ctas == 0:
                 continue
