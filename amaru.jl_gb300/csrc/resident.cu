@@ -260,9 +260,10 @@ __device__ __forceinline__ void store_async2(uint32_t to, float v, float w, uint
                  : "memory");
 }
 // waits for the phase of an mbarrier to complete; false after `limit` nanoseconds (a try may suspend the thread for a time
-// that the device sets, so tries alone would not bound it)
+// that the device sets, so tries alone would not bound it).  A pause between two looks at the clock counts for 20 ms at
+// most: while another process has the GPU, nobody here could have sent anything.
 __device__ __forceinline__ bool wait_phase(uint32_t bar, unsigned parity, unsigned long long limit) {
-    unsigned long long start = 0;
+    unsigned long long last = 0, waited = 0;
     for (int i = 0; i < (1 << 28); i++) {
         uint32_t done;
         asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
@@ -273,8 +274,9 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, unsigned parity, unsign
         if (done) return true;
         if (i % 16 == 15) {
             const unsigned long long now = global_ns();
-            if (!start) start = now;
-            else if (now - start > limit) break;
+            if (last) waited += min(now - last, 20000000ull);
+            if (waited > limit) break;
+            last = now;
         }
     }
     return false;
