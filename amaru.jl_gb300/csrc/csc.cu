@@ -5,6 +5,9 @@
 // walk over the node's block row, whose pattern is symmetric, so that the blocks of the column are the transposed
 // positions.  On the host the same walk, the scatter and a sort per column took 9 ms for 1.27 million entries (29 x 13 x
 // 13 HEX8); the count now takes 0.04 ms and the export 0.25 ms, of which the read-back of 20 MB is most.
+// Few entries are still walked on the host, where the launches and their arrays cost more: both calls that a mount takes
+// (the count, then all) 43 us instead of 107 for 576 entries, 85 instead of 117 for 7 200; 117 and 119 for 11 700, 136
+// and 118 for 15 800.
 #include "amr_internal.h"
 
 #include <algorithm>
@@ -13,6 +16,7 @@ namespace {
 
 constexpr size_t kCscChunk = size_t(1) << 21;  // entries of a chunk, 32 bytes each: 64 MB at most
 constexpr size_t kCscMin = size_t(1) << 15;    // below this a failed allocation is an error
+constexpr int64_t kCscHost = 12000;            // entries of the blocks up to which the host makes the columns
 
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -118,6 +122,41 @@ void columns(amr_model *m, const CscScratch &w, int64_t c0, int64_t c1, const ui
     AMR_CUDA(cudaGetLastError());
 }
 
+// the same on the host: entries by walking the rows, then each column sorted by its rows
+void host_csc(amr_model *m, int64_t *nnz_out, int64_t *colptr, int64_t *rowval, double *nzval, const uint16_t *d_keep,
+              const double *d_vals) {
+    const int B = m->B;
+    std::vector<uint16_t> keep(m->nblocks);
+    std::vector<double> vals;
+    amr_d2h(m, keep.data(), d_keep, m->nblocks * sizeof(uint16_t));
+    if (colptr && nzval) {
+        vals.resize((size_t)m->bstride * m->BB);
+        amr_d2h(m, vals.data(), d_vals, vals.size() * sizeof(double));
+    }
+    const std::vector<int64_t> &eq = m->h_eq_id;
+    auto walk = [&](auto entry) {
+        for (int64_t n = 0; n < m->nnodes; n++)
+            for (int64_t k = m->h_brow_ptr[n]; k < m->h_brow_ptr[n + 1]; k++)
+                for (int q = 0; q < m->BB; q++) {
+                    const int64_t r = eq[3 * n + q / B], c = eq[3 * (int64_t)m->h_bcol[k] + q % B];
+                    if (r >= 0 && c >= 0 && (keep[k] >> q & 1)) entry(r, c, (size_t)q * m->bstride + k);
+                }
+    };
+    std::vector<int64_t> at(m->ndofs + 1, 0);
+    walk([&](int64_t, int64_t c, size_t) { at[c + 1]++; });
+    for (int64_t i = 0; i < m->ndofs; i++) at[i + 1] += at[i];
+    *nnz_out = at[m->ndofs];
+    if (!colptr) return;
+    std::copy(at.begin(), at.end(), colptr);
+    std::vector<std::pair<int64_t, size_t>> e(*nnz_out);  // row, place of the value
+    walk([&](int64_t r, int64_t c, size_t v) { e[at[c]++] = {r, v}; });
+    for (int64_t c = 0; c < m->ndofs; c++) std::sort(e.begin() + colptr[c], e.begin() + colptr[c + 1]);
+    for (int64_t i = 0; i < *nnz_out; i++) {
+        rowval[i] = e[i].first;
+        if (nzval) nzval[i] = vals[e[i].second];
+    }
+}
+
 }  // namespace
 
 void amr_export_csc(amr_model *m, int64_t *nnz_out, int64_t *colptr, int64_t *rowval, double *nzval, const uint16_t *keep,
@@ -126,6 +165,10 @@ void amr_export_csc(amr_model *m, int64_t *nnz_out, int64_t *colptr, int64_t *ro
     *nnz_out = 0;
     if (nd == 0) {
         if (colptr) colptr[0] = 0;
+        return;
+    }
+    if (m->nblocks * m->BB <= kCscHost) {
+        host_csc(m, nnz_out, colptr, rowval, nzval, keep, vals);
         return;
     }
     CscScratch w;
