@@ -10,14 +10,17 @@
 // appearance).  Contribution lists give every node its task slots in patch order,
 // the order of the reference's V_vals[node] += V[i].
 //
+// The normal matrices depend on the mesh alone, so they are part of the structure (device):
+//   k_elem_geometry  lanes of a warp per element: sums over its IPs of the monomials that the normal matrices need
+//   k_patch_gram  eight lanes per task: the elements' sums translated to the patch centre, the normal matrix
+//                 and its Cholesky factor
+//
 // Values (per call, device):
 //   k_ip_fields   thread per IP: ip_state_vals of the IP's material
 //                 (linear-elastic.jl:140-164, von-mises.jl:159-168,330-341,
 //                 drucker-prager.jl:152-163 over tensors.jl:162-215)
-//   k_elem_moments  lanes of a warp per element: sums over its IPs of the monomials that the normal matrices need, and
-//                 the moments of the fields with the regression terms, about the element's centre
-//   k_patch_gram  eight lanes per task: the elements' sums translated to the patch centre, the normal matrix
-//                 and its Cholesky factor
+//   k_elem_moments  lanes of a warp per element: the moments of the fields with the regression terms, about the element's
+//                 centre
 //   k_patch_fit   warp per task: the least-squares polynomial of reg_terms
 //                 (fe-model.jl:488-501) through the task's IP values, evaluated at
 //                 its nodes.  The regression runs in patch-centred coordinates
@@ -42,6 +45,7 @@
 #include <climits>
 #include <cmath>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "amr_internal.h"
@@ -421,15 +425,11 @@ __device__ __forceinline__ double unordered(long long k) {
     return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
 }
 
-// W lanes per element, W >= its number of IPs.  The FP64 pipe (2 operations per SM and cycle) bounds all of the fit, so
-// the sums over IPs, which every patch of an element took again, are taken once per element about its centre and
-// translated: at 27 points and 16 fields a patch of eight elements needs 41 000 operations from the points and 15 000 from
-// the moments.  41 x 17 x 17 HEX20: the one kernel per patch took 1.16 ms at 81 % of the pipe; a whole
-// recovery took 1.73 ms and takes 1.01 (20 x 20 x 20: the fit alone 0.78 and 0.30 ms).
+// W lanes per element, W >= its number of IPs: the sums of the monomials about the element's centre.
 constexpr int kElemWarps = 4;
 constexpr int kMonoPad = 25;
-template <int DIM, bool MOM, int W>
-__global__ void __launch_bounds__(32 * kElemWarps) k_elem_moments(FitArgs A) {
+template <int DIM, int W>
+__global__ void __launch_bounds__(32 * kElemWarps) k_elem_geometry(FitArgs A) {
     constexpr int ROWS = W < AMR_MAXIP ? W : AMR_MAXIP;
     __shared__ double s_mono[32 / W * kElemWarps][ROWS * kMonoPad];
     const int slot = threadIdx.x / W, sub = threadIdx.x % W;
@@ -484,8 +484,45 @@ __global__ void __launch_bounds__(32 * kElemWarps) k_elem_moments(FitArgs A) {
             geo[kElemLow + d] = lo[d];
             geo[kElemHigh + d] = hi[d];
         }
-    if (!MOM) return;
-    const int P = kTerms<DIM> * A.nf;
+}
+
+// The fields' moments with the regression terms, about the element's centre.  The FP64 pipe (2 operations per SM and
+// cycle) bounds all of the fit, so the sums over IPs, which every patch of an element took again, are taken once per
+// element and translated: at 27 points and 16 fields a patch of eight elements needs 41 000 operations from the points and
+// 15 000 from the moments.  41 x 17 x 17 HEX20: with one kernel per patch, 1.16 ms at 81 % of the pipe, a whole
+// recovery took 1.73 ms; now 0.89 (20 x 20 x 20: the fit alone 0.78 ms, now 0.24).
+template <int DIM, int W>
+__global__ void __launch_bounds__(32 * kElemWarps) k_elem_moments(FitArgs A) {
+    constexpr int ROWS = W < AMR_MAXIP ? W : AMR_MAXIP, NT = kTerms<DIM>, PAD = 7;
+    __shared__ double s_mono[32 / W * kElemWarps][ROWS * PAD];
+    const int slot = threadIdx.x / W, sub = threadIdx.x % W;
+    const int64_t e = (int64_t)blockIdx.x * (32 / W * kElemWarps) + slot;
+    const bool any = e < A.nelems;
+    double *mono = s_mono[slot];
+    const int64_t g0 = any ? A.ip_ptr[e] : 0;
+    const int nip = any ? min((int)(A.ip_ptr[e + 1] - g0), ROWS) : 0;
+    if (sub < nip) {
+        const double *ce = A.geo + e * kElemRec + kElemCentre;
+        double x[3];
+#pragma unroll
+        for (int d = 0; d < DIM; d++) x[d] = A.ipx[3 * (g0 + sub) + d] - ce[d];
+        double pw[3][3];
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            pw[d][0] = 1.0;
+            pw[d][1] = x[d];
+            pw[d][2] = x[d] * x[d];
+        }
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            double v = pw[0][mono_exp<DIM>(i, 0)] * pw[1][mono_exp<DIM>(i, 1)];
+            if (DIM == 3) v *= pw[2][mono_exp<DIM>(i, 2)];
+            mono[sub * PAD + i] = v;
+        }
+    }
+    __syncwarp();
+    if (!any) return;
+    const int P = NT * A.nf;
     const double *v = A.ipv + g0 * A.nf;
     double *out = A.mom + e * P;
     constexpr int U = 4;  // pairs (term, field) of a lane at a time
@@ -501,7 +538,7 @@ __global__ void __launch_bounds__(32 * kElemWarps) k_elem_moments(FitArgs A) {
         }
         for (int i = 0; i < nip; i++)
 #pragma unroll
-            for (int u = 0; u < U; u++) acc[u] = fma(mono[i * kMonoPad + q[u]], v[i * A.nf + k[u]], acc[u]);
+            for (int u = 0; u < U; u++) acc[u] = fma(mono[i * PAD + q[u]], v[i * A.nf + k[u]], acc[u]);
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (p0 + W * u < P) out[p0 + W * u] = acc[u];
@@ -510,7 +547,8 @@ __global__ void __launch_bounds__(32 * kElemWarps) k_elem_moments(FitArgs A) {
 
 // Eight lanes per task sum the elements' translated monomials; then a thread per task factors the normal matrix, whose
 // chain of square roots and divisions costs a warp as much as all moments when each warp does its own (7 pivots, 32
-// lanes alike).
+// lanes alike).  Once per model, as the mesh alone gives it: at each recovery this and the element sums cost small ones
+// two launches, 145 us instead of 111 for 288 HEX8 (136 with one kernel per patch).
 constexpr int kGramTasks = 16;
 template <int DIM>
 __global__ void __launch_bounds__(8 * kGramTasks) k_patch_gram(FitArgs A) {
@@ -850,8 +888,8 @@ struct AmrRecovery {
     int nf = 0, nmask = 0, m_max = 1, e_max = 1;
     std::vector<int32_t> codes;      // output field codes, reference order
     int64_t ntasks = 0, nslots = 0, ncontrib = 0;
-    double fit_flops = 0.0;          // FP64 operations of one fit (its three kernels)
-    int64_t n_svd = 0;               // tasks on the SVD path (known after a launch)
+    double fit_flops = 0.0;          // FP64 operations of one fit (moments, coefficients, nodal values)
+    int64_t n_svd = 0;               // tasks on the SVD path
     // device
     double *ipx = nullptr, *ipv = nullptr, *vst = nullptr;
     double *geo = nullptr, *mom = nullptr, *t_rec = nullptr;  // element and task records; mom only where it is used
@@ -987,15 +1025,8 @@ void build(amr_model *m) {
     std::vector<int32_t> t_elem, t_node, t_mask, t_center, t_m;
     std::vector<int64_t> stamp(nn, -1);
     const bool moments = by_elements(m);
-    // FP64 operations: the elements' sums of monomials and moments; translating and adding one element's monomials
-    const int nm = m->ndim == 3 ? kMono<3> : kMono<2>;
-    double flops = (double)m->nip_total * (nm + (moments ? 2.0 * (m->ndim == 3 ? kTerms<3> : kTerms<2>) * R->nf : 0.0));
-    double mono_ops = nm;
-    for (int i = 0; i < nm; i++)
-        for (int d = 0; d < m->ndim; d++) {
-            const int a = m->ndim == 3 ? mono_exp<3>(i, d) : mono_exp<2>(i, d);
-            mono_ops += a * (a + 1);  // a (a + 1) / 2 FMA
-        }
+    // FP64 operations of a fit, the elements' moments first
+    double flops = moments ? 2.0 * m->nip_total * (m->ndim == 3 ? kTerms<3> : kTerms<2>) * R->nf : 0.0;
     for (int64_t n = 0; n < nn; n++) {
         if (!src[n]) continue;
         const int32_t *pb = src[n] == 1 ? &ip_list[ip_cnt[n]] : &bp_list[bp_cnt[n]];
@@ -1025,11 +1056,10 @@ void build(amr_model *m) {
             const int nt = m->ndim == 3 ? (mcount >= 7 ? 7 : mcount >= 4 ? 4 : 1)
                                         : (mcount >= 6 ? 6 : mcount >= 4 ? 4 : mcount >= 3 ? 3 : 1);
             const double nnod = (double)(t_node_ptr.back() - t_node_ptr[t_node_ptr.size() - 2]);
-            // per element of the patch the translated monomials and moments (or nt FMA per IP and field), per node and
-            // field nt - 1 FMA
+            // per element of the patch and field the translated moments (or nt FMA per IP and field), per node and field
+            // nt - 1 FMA
             const double field_ops = moments ? ecount * (m->ndim == 3 ? 25.0 : 20.0) : 2.0 * mcount * nt;
-            flops += ecount * mono_ops + field_ops * mask_nf[mk] +
-                     2.0 * nnod * (nt - 1) * mask_nf[mk];
+            flops += field_ops * mask_nf[mk] + 2.0 * nnod * (nt - 1) * mask_nf[mk];
         }
     }
     R->fit_flops = flops;
@@ -1121,29 +1151,48 @@ void launch_tasks(amr_model *m, K kernel, const FitArgs &A, size_t smem) {
     AMR_CUDA(cudaGetLastError());
 }
 
-template <int DIM, bool MOM, int W>
-void launch_elements(amr_model *m, const FitArgs &A) {
-    const int64_t per = 32 / W * kElemWarps;
-    k_elem_moments<DIM, MOM, W><<<(unsigned)((m->nelems + per - 1) / per), 32 * kElemWarps, 0, m->stream>>>(A);
+// f with the lanes per element as a constant, its argument the CTAs
+template <class F>
+void over_elements(const amr_model *m, F f) {
+    int nip = 1;
+    for (const AmrGroup &g : m->groups) nip = std::max(nip, (int)g.nip);
+    auto go = [&](auto w) {
+        constexpr int64_t per = 32 / decltype(w)::value * kElemWarps;
+        f(w, (unsigned)((m->nelems + per - 1) / per));
+    };
+    if (nip <= 4) go(std::integral_constant<int, 4>());
+    else if (nip <= 8) go(std::integral_constant<int, 8>());
+    else go(std::integral_constant<int, 32>());
+}
+
+// the normal matrices of all tasks, and which of them take the SVD
+template <int DIM>
+void launch_geometry(amr_model *m) {
+    const FitArgs A = fit_args(m);
+    over_elements(m, [&](auto w, unsigned grid) {
+        k_elem_geometry<DIM, decltype(w)::value><<<grid, 32 * kElemWarps, 0, m->stream>>>(A);
+    });
+    k_patch_gram<DIM><<<(unsigned)((A.ntasks + kGramTasks - 1) / kGramTasks), 8 * kGramTasks, 0, m->stream>>>(A);
+    AMR_COUNT(2);
+    AMR_CUDA(cudaGetLastError());
 }
 
 template <int DIM, bool MOM>
 void launch_fit_dim(amr_model *m, const FitArgs &A, size_t smem) {
-    int nip = 1;
-    for (const AmrGroup &g : m->groups) nip = std::max(nip, (int)g.nip);
-    if (nip <= 4) launch_elements<DIM, MOM, 4>(m, A);
-    else if (nip <= 8) launch_elements<DIM, MOM, 8>(m, A);
-    else launch_elements<DIM, MOM, 32>(m, A);
-    k_patch_gram<DIM><<<(unsigned)((A.ntasks + kGramTasks - 1) / kGramTasks), 8 * kGramTasks, 0, m->stream>>>(A);
-    AMR_COUNT(2);
-    AMR_CUDA(cudaGetLastError());
+    if (MOM) {
+        over_elements(m, [&](auto w, unsigned grid) {
+            k_elem_moments<DIM, decltype(w)::value><<<grid, 32 * kElemWarps, 0, m->stream>>>(A);
+        });
+        AMR_COUNT(1);
+        AMR_CUDA(cudaGetLastError());
+    }
     launch_tasks(m, k_patch_fit<DIM, MOM>, A, MOM ? kFitWarps * kFitDoubles * sizeof(double) : smem);
 }
 
 // the fit and SVD launches over all tasks
 void launch_fit(amr_model *m, bool svd) {
     AmrRecovery *R = m->rec;
-    if (!R->ntasks) return;
+    if (!R->ntasks || (svd && !R->n_svd)) return;
     const size_t smem = (size_t)fit_warp_doubles(R->m_max, R->e_max) * sizeof(double) * kFitWarps;
     const FitArgs A = fit_args(m);
     if (m->ndim == 3) {
@@ -1163,6 +1212,14 @@ void amr_recovery_prepare(amr_model *m) {
     if (!m->rec) {
         try {
             build(m);
+            AmrRecovery *R = m->rec;
+            if (R->ntasks) {
+                if (m->ndim == 3) launch_geometry<3>(m);
+                else launch_geometry<2>(m);
+                std::vector<int32_t> flag(R->ntasks);
+                amr_d2h(m, flag.data(), R->t_flag, flag.size() * sizeof(int32_t));
+                R->n_svd = std::count(flag.begin(), flag.end(), 1);
+            }
         } catch (...) {
             amr_recovery_free(m);
             throw;
@@ -1211,12 +1268,7 @@ double amr_recovery_time_fit(amr_model *m, int reps, double *flops, int64_t *n_s
     float ms = 0.0f;
     AMR_CUDA(cudaEventElapsedTime(&ms, m->ev0, m->ev1));
     if (flops) *flops = R->fit_flops;
-    if (n_svd) {
-        std::vector<int32_t> fl(R->ntasks);
-        if (R->ntasks)
-            amr_d2h(m, fl.data(), R->t_flag, R->ntasks * sizeof(int32_t));
-        *n_svd = std::count(fl.begin(), fl.end(), 1);
-    }
+    if (n_svd) *n_svd = R->n_svd;
     return ms * 1e-3 / std::max(1, reps);
 }
 

@@ -430,7 +430,7 @@ def recovery_leg(model, with_cpu, reps=5):
            "device_s": float(np.mean(ts)), "value": nn / float(np.mean(ts)), "unit": "nodes/s",
            "e2e": {"value": nn / float(np.mean(te)), "unit": "nodes/s", "s": float(np.mean(te)),
                    "d2h_bytes": int(V.size * 8)},
-           "patch_fit": {"kernel": "k_elem_moments<3>, k_patch_gram<3>, k_patch_fit<3> (moments per element, Cholesky per patch, nodal values)",
+           "patch_fit": {"kernel": "k_elem_moments<3>, k_patch_fit<3> (moments per element, coefficients and nodal values per patch)",
                          "avg_launch_s": fit_t, "flops_per_launch": flops,
                          "achieved": flops / fit_t / 1e12, "unit": "TFLOP/s (FP64)",
                          "peak": fp64_peak_tflops(), "peak_source": "measured FP64 FMA peak (amr_measure_peak)",
