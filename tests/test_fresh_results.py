@@ -44,4 +44,3 @@ def test_matrix_and_states_into_new_memory():
     assert _median(fresh) <= 8 * kept + 2e-3
     kept = _median(lambda: lib.amr_get_state(h, L.ptr(st)))
     assert _median(lambda: model.state()) <= 8 * kept + 2e-3
-    assert _median(lambda: model.dev.K_csc()) <= 8e-3  # with scipy's own conversion, 1.5 ms here
